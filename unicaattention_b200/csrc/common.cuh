@@ -21,6 +21,7 @@ constexpr int HEAD_DIM = 128;
 constexpr int KEY_TILE = 64;     // keys per tile: the K scale block and the softmax tile of the numerics contract
 constexpr int QUERY_TILE = 128;  // query rows per tile: the Q scale block, and M of one tcgen05.mma
 constexpr float LOG2_255 = 7.99435343685886f;
+constexpr float V8_BIAS = 128.0f;  // V8 is stored as code + 128, an unsigned byte (see flush32 in attention_int8.cu)
 
 // Where token `token` of head `head_index` (= batch * heads + head) starts in a [batch, heads, tokens, 128] tensor with
 // a contiguous last dimension and any other strides; strides in elements.  Field for field the reference's struct
@@ -267,6 +268,69 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, int parity, volatile in
     }
 }
 
+// The wait of the accurate attention kernel's roles: up to LINE_PROBES probes in ONE statement, so that to the compiler a wait
+// is straight-line code.  As a C++ loop between threads that hold up to 232 registers it cut the tile loops into basic blocks:
+// the flush loop alone then took 722 cycles per key tile against 480 for its arithmetic.  What is left outside is the cold path
+// that looks at the abort word and the clock.  SLEEP_NS > 0: for a wait nobody is in a hurry for, which then costs the computing
+// warps of its scheduler next to no issue slots.
+constexpr int LINE_PROBES = 64;
+template <unsigned SLEEP_NS>
+__device__ __forceinline__ bool mbar_probe_line(uint64_t* bar, int parity) {
+    uint32_t done;
+    if constexpr (SLEEP_NS > 0) {
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p, q;\n\t"
+            ".reg .u32 left;\n\t"
+            "mov.u32 left, %3;\n"
+            "UNICA_NAP_AGAIN:\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "@p bra UNICA_NAP_DONE;\n\t"
+            "nanosleep.u32 %4;\n\t"
+            "sub.u32 left, left, 1;\n\t"
+            "setp.ne.u32 q, left, 0;\n\t"
+            "@q bra UNICA_NAP_AGAIN;\n"
+            "UNICA_NAP_DONE:\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity), "n"(LINE_PROBES), "n"(SLEEP_NS)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p, q;\n\t"
+            ".reg .u32 left;\n\t"
+            "mov.u32 left, %3;\n"
+            "UNICA_LINE_AGAIN:\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "@p bra UNICA_LINE_DONE;\n\t"
+            "sub.u32 left, left, 1;\n\t"
+            "setp.ne.u32 q, left, 0;\n\t"
+            "@q bra UNICA_LINE_AGAIN;\n"
+            "UNICA_LINE_DONE:\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity), "n"(LINE_PROBES)
+            : "memory");
+    }
+    return done != 0;
+}
+template <unsigned SLEEP_NS = 0>
+__device__ __forceinline__ bool mbar_wait_line(uint64_t* bar, int parity, int* abort_flag, int* status, int code) {
+    if (mbar_probe_line<SLEEP_NS>(bar, parity)) return true;
+    const long long start = clock64();
+    while (*static_cast<volatile int*>(abort_flag) == 0) {
+        if (mbar_probe_line<SLEEP_NS>(bar, parity)) return true;
+        if (clock64() - start > WAIT_LIMIT_CYCLES) {
+            *static_cast<volatile int*>(abort_flag) = 1;
+            if (status) atomicCAS(status, 0, code);
+        }
+    }
+    return false;
+}
+
 // Two barriers at once: both probes are in flight together, so a lone thread pays one probe latency (some 250 cycles)
 // instead of two.  parity_b < 0: there is no second barrier.
 template <unsigned SLEEP_NS = WAIT_SLEEP_NS>
@@ -352,41 +416,6 @@ __device__ __forceinline__ bool mbar_wait2(uint64_t* bar_a, int parity_a, uint64
     }
 }
 
-// A word in shared memory that one thread of the block advances and others wait for.  Looking at a word costs a waiting
-// warp an ordinary shared-memory load (some 30 cycles), a tenth of an mbarrier probe, so where the event is first seen by
-// a thread that has to watch it anyway (the completion of tcgen05.mma by the thread that issued them), that thread passes
-// it on through such a word.  Release / acquire at block scope; bounded like every other wait here.
-#ifndef UNICA_FLAG_SLEEP_NS
-#define UNICA_FLAG_SLEEP_NS 0
-#endif
-__device__ __forceinline__ void flag_publish(int* flag, int value) {
-    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(flag)), "r"(value) : "memory");
-}
-__device__ __forceinline__ bool flag_wait(const int* flag, int at_least, volatile int* abort_flag, int* status, int code) {
-    long long start = 0;
-    for (int looks = 1;; ++looks) {
-        int value;
-        asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(value) : "r"(smem_u32(flag)) : "memory");
-        if (value >= at_least) return true;
-#if UNICA_FLAG_SLEEP_NS > 0
-        __nanosleep(UNICA_FLAG_SLEEP_NS);  // back-to-back looks crowd the queue the computing warps' exponentials go through
-#endif
-        if (looks % 256 == 0) {
-            if (*abort_flag) return false;
-            const long long now = clock64();
-            if (start == 0) start = now;
-            if (now - start > WAIT_LIMIT_CYCLES) {
-                *abort_flag = 1;
-                if (status) atomicCAS(status, 0, code);
-                return false;
-            }
-        }
-    }
-}
-__device__ __forceinline__ bool flag_wait_warp(const int* flag, int at_least, volatile int* abort_flag, int* status, int code) {
-    return __all_sync(0xffffffffu, flag_wait(flag, at_least, abort_flag, status, code));
-}
-
 // The same for a whole warp: every lane waits, and all get the same answer.  The vote also reconverges the warp, which
 // the .sync.aligned tensor-memory instructions that usually follow require: a tcgen05.ld executed by part of a warp
 // never completes.
@@ -404,6 +433,14 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes,
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+
+// shared -> global, counted in this thread's bulk groups (same alignment rules); the shared bytes must have been made
+// visible with fence_proxy_async() first, and stay as they are until bulk_store_read_wait()
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_read_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // generic-proxy writes to shared memory made visible to the async proxy (tcgen05.mma operand reads)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -607,6 +644,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t k_ste
 __host__ __device__ constexpr uint32_t idesc_i8(bool a_signed, int m, int n) {
     return (2u << 4) | (uint32_t(a_signed) << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
+
+// The same with A and B u8.
+__host__ __device__ constexpr uint32_t idesc_u8(int m, int n) { return (2u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24); }
 
 // Instruction descriptor of kind::tf32: D f32; A and B tf32 (32-bit words whose low 13 bits the tensor core ignores);
 // both K-major; M x N.  The operand images have the byte geometry of the 8-bit ones: 16 bytes (four values) per row and

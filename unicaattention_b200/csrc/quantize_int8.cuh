@@ -44,10 +44,11 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
         : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
     return d;
 }
-__device__ __forceinline__ float2 quotient_code2(float2 x, float2 inv2, float2 minus_scale2) {
+// (or the integer plus `bias`, a small integer: exact).
+__device__ __forceinline__ float2 quotient_code2(float2 x, float2 inv2, float2 minus_scale2, float bias = 0.0f) {
     const float2 q0 = mul2(x, inv2);
     const float2 q1 = fma2(fma2(q0, minus_scale2, x), inv2, q0);
-    return add2(q1, make_float2(MAGIC, MAGIC));
+    return add2(q1, make_float2(MAGIC + bias, MAGIC + bias));
 }
 __device__ __forceinline__ bool needs_division(float scale) { return (__float_as_uint(scale) & 0x7fffffu) == 0x7fffffu; }
 __device__ __forceinline__ float code_by_division(float x, float scale) { return rintf(__fdiv_rn(x, scale)) + MAGIC; }
@@ -140,7 +141,7 @@ __device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__
 // the channel's min and max over the head (low, high: [heads][128]); true: one scale per key over its channels, and
 // v_token [heads][tiles][2][64] gets log2 s and 1 / s of the tile's keys (zeros past n_tokens).  skip: [heads][n_tokens],
 // 1 = the key is written as zeros (outlier keys), or null.
-// v8: [heads][tiles][4 chunks of 16 keys][128 channels][16] bytes: the K-major B operand of P.V.  v_scale [heads][128].
+// v8: [heads][tiles][4 chunks of 16 keys][128 channels][16] bytes, code + V8_BIAS: the K-major B operand of P.V.  v_scale [heads][128].
 template <bool PER_TOKEN, int NT = THREADS, bool STAGED = false>
 __device__ __forceinline__ void v_int8_emit(const __nv_bfloat16 (*tile)[HEAD_DIM], bool half, const float* key_scale, const float* key_inv,
                                             const float* low, const float* high, int head, int t, int tiles, int8_t* __restrict__ v8,
@@ -235,11 +236,11 @@ __device__ __forceinline__ void v_int8_emit(const __nv_bfloat16 (*tile)[HEAD_DIM
                 scale2 = make_float2(s, s), inv2 = make_float2(inv, inv), minus_scale2 = make_float2(-s, -s);
                 divide = needs_division(s);
             }
-            code[j] = quotient_code2(x, inv2, minus_scale2);
-            if (divide) code[j] = make_float2(code_by_division(x.x, scale2.x), code_by_division(x.y, scale2.y));
+            code[j] = quotient_code2(x, inv2, minus_scale2, V8_BIAS);
+            if (divide) code[j] = make_float2(code_by_division(x.x, scale2.x) + V8_BIAS, code_by_division(x.y, scale2.y) + V8_BIAS);
             if (!STAGED && !PER_TOKEN) {  // low and high come from the caller: a value outside them must not wrap around
-                code[j].x = fminf(fmaxf(code[j].x, MAGIC - 127.0f), MAGIC + 127.0f);
-                code[j].y = fminf(fmaxf(code[j].y, MAGIC - 127.0f), MAGIC + 127.0f);
+                code[j].x = fminf(fmaxf(code[j].x, MAGIC + V8_BIAS - 127.0f), MAGIC + V8_BIAS + 127.0f);
+                code[j].y = fminf(fmaxf(code[j].y, MAGIC + V8_BIAS - 127.0f), MAGIC + V8_BIAS + 127.0f);
             }
         }
         uint32_t first[2], second[2];
