@@ -280,6 +280,36 @@ int unica_b200_selftest_mma_nvf4(const void* a_image, const void* b_image, const
  * (0: one accumulator).  Allocates scratch and synchronises the stream: a measurement tool. */
 int unica_b200_peak(int kind, int n, int count, int blocks, double* cycles_per_instruction, void* stream);
 
+/* A whole call in one entry point: statistics, quantization and attention, with the operands in a workspace of the caller's
+ * (256-byte aligned, unica_b200_attention_workspace() bytes, free again when the queued work has run).  Results are bit for
+ * bit those of the single steps in the order of unica/__init__.py:288-356.  kernel: UNICA_B200_ACCURATE (v_mode,
+ * n_outliers for UNICA_B200_V_OUTLIERS, which is limited to 8192 keys here) or UNICA_B200_FAST (smooth_q: 0 or a multiple of
+ * 256).  rope: a (cos, sin) table as the _rope entry points take it, or NULL.  peer_out, n_peers: as in the _peers entry
+ * points.  launches: how many kernels were queued. */
+#define UNICA_B200_ACCURATE 0
+#define UNICA_B200_FAST 1
+typedef struct {
+    const void *q, *k, *v;
+    void *out, *workspace;
+    size_t workspace_bytes;
+    const void* rope;
+    long long rope_batch_stride;
+    void* const* peer_out;
+    int* status;
+    void* stream;
+    unica_token_layout q_layout, k_layout, v_layout, out_layout;
+    int heads, n_queries, n_keys, kernel, v_mode, n_outliers, smooth_q, n_peers;
+    float scale_log2;
+} unica_b200_call;
+int unica_b200_attention_workspace(const unica_b200_call* call, size_t* bytes);
+int unica_b200_attention_call(const unica_b200_call* call, int* launches);
+
+/* V in INT8 per channel without each head's n_outliers (1..8) keys of largest max |v| (ties: the lower key), which are written
+ * as zeros: what quantize_v(outliers=..) makes of n_tokens <= 8192 (unica/__init__.py:384-399, 420-432), in one launch.
+ * keys [heads][n_outliers] (-1: the head has fewer keys), rows float [heads][n_outliers][128]: V over the scale. */
+int unica_b200_quantize_v_int8_outliers(const void* v, unica_token_layout layout, int heads, int n_tokens, int n_outliers, int8_t* v8,
+                                        float* v_scale, int* keys, float* rows, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,63 @@
+"""A whole call through the one entry point (and, up to 8192 tokens, the one-launch quantizers) against the single steps, bit
+for bit: kernel_inputs() and the kernel on its operands, at sizes around the statistics' 256-token blocks, the 64-key tiles and
+the line between the short and the long quantizers."""
+
+import pytest
+import torch
+
+from gpu_common import qkv
+
+pytestmark = pytest.mark.gpu
+PRESETS = ["per_channel", "per_token", "outliers", "fast"]
+
+
+def rope(tokens, batch=1):
+    angle = torch.rand((batch, tokens, 1, 64), generator=torch.Generator().manual_seed(7)) * 6
+    cos, sin = angle.cos(), angle.sin()
+    return torch.stack([torch.stack([cos, -sin], -1), torch.stack([sin, cos], -1)], -2).cuda()
+
+
+@pytest.mark.parametrize("preset", PRESETS)
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 3, 300, 77), (1, 2, 1000, 1000), (1, 2, 129, 5), (1, 2, 2050, 8192), (1, 1, 8192, 8193), (1, 2, 8300, 700)])
+def test_one_entry_point_equals_the_steps(shape, preset):
+    import unicaattention_b200 as unica
+
+    q, k, v = (x.cuda() for x in qkv(*shape, seed=shape[3], channel_scale=True))
+    settings = unica.PRESETS[preset]
+    inputs = unica.kernel_inputs(q, k, v, **settings)
+    if preset == "outliers" and shape[3] >= 8:
+        v8, scale, keys, rows = inputs[4], inputs[5], *inputs[6]
+        order = unica.v_outliers(v, 8).sort(-1).values  # found by torch
+        assert torch.equal(keys.long().sort(-1).values, order)
+    steps = unica.attention(q, k, v, inputs=inputs, **settings)
+    assert torch.equal(unica.attention(q, k, v, **settings), steps)
+    half = [x.transpose(1, 2).contiguous().transpose(1, 2).half() for x in (q, k, v)]
+    steps = unica.attention(*(x.half().bfloat16() for x in (q, k, v)), **settings).half()
+    assert torch.equal(unica.attention(*half, **settings), steps)
+    unica.check_status()
+
+
+@pytest.mark.parametrize("preset", PRESETS)
+@pytest.mark.parametrize("tokens", [65, 513, 4100, 8200])
+def test_with_rope(tokens, preset):
+    import unicaattention_b200 as unica
+
+    q, k, v = (x.cuda() for x in qkv(2, 2, tokens, tokens, seed=tokens))
+    table, settings = rope(tokens), unica.PRESETS[preset]
+    steps = unica.attention(q, k, v, inputs=unica.kernel_inputs(q, k, v, rope=table, **settings), rope=table, **settings)
+    assert torch.equal(unica.attention(q, k, v, rope=table, **settings), steps)
+    unica.check_status()
+
+
+@pytest.mark.parametrize("tokens", [1, 255, 257, 2048, 8192])
+def test_short_operands_equal_the_separate_passes(tokens):
+    """quantize_k and quantize_v_channel of short heads, whose means are summed as rope_stats sums them."""
+    import unicaattention_b200 as unica
+
+    _, k, v = (x.cuda() for x in qkv(1, 3, 1, tokens, seed=tokens, channel_scale=True))
+    k8, scale, mean = unica.quantize_k(k)
+    assert torch.equal(mean, unica.rope_stats(k)[0])
+    want8, want_scale = unica.quantize_int8(k, mean, 64)
+    assert torch.equal(k8, want8) and torch.equal(scale, want_scale)
+    assert all(torch.equal(a, b) for a, b in zip(unica.quantize_v_channel(v), unica.quantize_v(v)))
+    unica.check_status()

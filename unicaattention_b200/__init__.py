@@ -83,8 +83,10 @@ def token_layout(x: torch.Tensor) -> TokenLayout:
 def readable(x: torch.Tensor) -> torch.Tensor:
     """x itself if the kernels can read it in place (contiguous last dimension, 16-byte aligned tokens), else a
     contiguous copy (unica/__init__.py:103-108)."""
-    in_place = (x.stride(-1) == 1 and x.data_ptr() % 16 == 0
-                and all(x.stride(i) % 8 == 0 or x.shape[i] == 1 for i in range(3)))
+    batch, head, token, channel = x.stride()
+    if channel == 1 and not (batch | head | token) % 8 and not x.data_ptr() % 16:
+        return x
+    in_place = channel == 1 and x.data_ptr() % 16 == 0 and all(x.stride(i) % 8 == 0 or x.shape[i] == 1 for i in range(3))
     return x if in_place else x.contiguous()
 
 
@@ -93,6 +95,8 @@ def on_their_device(function):
 
     @functools.wraps(function)
     def run(q, *args, **kwargs):
+        if q.is_cuda and q.device.index == torch.cuda.current_device():  # already so: the usual case, and entering it again costs 3 us
+            return function(q, *args, **kwargs)
         with torch.cuda.device(q.device):
             return function(q, *args, **kwargs)
 
@@ -115,10 +119,11 @@ _status_words: dict = {}
 
 def status_word(device: torch.device) -> torch.Tensor:
     """The int32 word the attention kernels leave non-zero when one of their bounded waits gave up; one per device."""
-    device = torch.device(device)
-    if device not in _status_words:
-        _status_words[device] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _status_words[device]
+    word = _status_words.get(device)
+    if word is None:
+        device = torch.device(device)
+        word = _status_words.setdefault(device, torch.zeros(1, dtype=torch.int32, device=device))
+    return word
 
 
 def check_status(device=None) -> None:
@@ -342,6 +347,12 @@ def quantize_v(v: torch.Tensor, layout: int = 2, per_token: bool = False, outlie
     low = high = tokens = skip = None
     if per_token:
         tokens = torch.empty(batch, heads, tiles, 2, V8_PAD_KEYS, device=v.device)
+    elif outliers and n <= lib.CALL_TOKENS:  # everything in one launch
+        keys = torch.empty(batch, heads, outliers, dtype=torch.int32, device=v.device)
+        rows = torch.empty(batch, heads, outliers, HEAD_DIM, device=v.device)
+        lib.call("unica_b200_quantize_v_int8_outliers", lib.ptr(v), token_layout(v), batch * heads, n, outliers, lib.ptr(v8), lib.ptr(scale),
+                 lib.ptr(keys), lib.ptr(rows), lib.stream())
+        return v8, scale, keys, rows
     elif outliers:
         keys = v_outliers(v, outliers)
         skip = torch.zeros(batch, heads, n, dtype=torch.uint8, device=v.device).scatter_(-1, keys, 1)
@@ -429,7 +440,7 @@ def _settings(kernel: str, tile: dict) -> dict:
         raise ValueError(f"unknown kernel {kernel!r}, expected one of {KERNELS}")
     if unknown := tile.keys() - TILE.keys():
         raise ValueError(f"unknown tile settings {sorted(unknown)}, expected some of {sorted(TILE)}")
-    settings = TILE | tile
+    settings = TILE | tile if tile else TILE
     if settings["KEYS_PER_TILE"] != KEYS_PER_TILE:
         raise ValueError(f"KEYS_PER_TILE is fixed at {KEYS_PER_TILE}: it is part of the numerics")
     return settings
@@ -479,6 +490,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         return out
     if inputs is None:
         try:
+            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out)):
+                return out
             inputs = kernel_inputs(q, k, v, kernel, rope, **tile)
         except torch.cuda.OutOfMemoryError:
             # The planner's picture of free memory was out of date (something took memory since it asked): forget it and
@@ -501,8 +514,48 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
              lib.ptr(v_scale), lib.ptr(v_token if v_mode == lib.V_TOKEN else None), v_mode, lib.ptr(keys), lib.ptr(rows),
              0 if keys is None else keys.shape[-1], lib.ptr(out), peers, len(peer_out), token_layout(out), batch * heads, n_queries,
              n_keys, HEAD_DIM**-0.5 * LOG2E, lib.ptr(status_word(q.device)), lib.stream())
-    del settings
     return out
+
+
+_WORKSPACE_BYTES: dict = {}  # (heads, queries, keys, kernel, V mode, outliers, SMOOTH_Q, rope?) -> bytes
+
+
+def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int) -> bool:
+    """The whole call through one entry point of the library: quantization and kernel with their operands in one workspace.
+    Bit for bit kernel_inputs() and the kernel, without their dozen allocations and trips through ctypes.  False: not
+    for this call (the outlier keys of a long V are found by torch)."""
+    batch, heads, n_queries, _ = q.shape
+    n_keys = k.shape[2]
+    fast, smooth, outliers = kernel == "attention_fp4", settings["SMOOTH_Q"], 0
+    v_mode = lib.V_CHANNEL
+    if fast:
+        if smooth % 256:
+            raise ValueError(f"SMOOTH_Q must be a multiple of 256, got {smooth}")
+    elif settings["V_TOKEN"]:
+        v_mode = lib.V_TOKEN
+    elif settings["V_OUTLIERS"]:
+        v_mode, outliers = lib.V_OUTLIERS, settings["V_OUTLIERS"]
+        if n_keys > lib.CALL_TOKENS or not 0 < outliers <= MAX_OUTLIERS:
+            return False
+    table, table_stride = (0, 0) if rope is None else rope_args(rope, q)
+    if rope is not None:
+        table = table.value
+    half = int(q.dtype == torch.float16)
+    layouts = (*q.stride()[:3], heads, half, *k.stride()[:3], heads, half, *v.stride()[:3], heads, half, *out.stride()[:3], heads, half)
+    sizes = (batch * heads, n_queries, n_keys, int(fast), v_mode, outliers, smooth if fast else 0)
+    where = (table, table_stride, 0 if peers is None else ctypes.addressof(peers), status_word(q.device).data_ptr(),
+             torch.cuda.current_stream().cuda_stream)
+    scale = HEAD_DIM**-0.5 * LOG2E
+    key = (*sizes, rope is None)
+    size = _WORKSPACE_BYTES.get(key)
+    if size is None:
+        if len(_WORKSPACE_BYTES) > 4096:
+            _WORKSPACE_BYTES.clear()
+        size = _WORKSPACE_BYTES[key] = lib.attention_workspace(lib.pack_call(0, 0, 0, 0, 0, 0, *where, *layouts, *sizes, 0, scale))
+    workspace = torch.empty(size, dtype=torch.uint8, device=q.device)
+    lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
+                                     n_peers, scale))
+    return True
 
 
 # ----------------------------------------------------------------------------------------------------------------------
@@ -525,10 +578,16 @@ def free_vram(device: torch.device, fresh: bool = False) -> int:
     return cached[0]
 
 
+_TENTH: dict = {}  # device -> a tenth of its memory
+
+
 def vram_reserve(device: torch.device) -> int:
     if VRAM_RESERVE is not None:
         return VRAM_RESERVE
-    return max(2**30, torch.cuda.get_device_properties(device).total_memory // 10)
+    tenth = _TENTH.get(device)
+    if tenth is None:
+        tenth = _TENTH[device] = torch.cuda.get_device_properties(device).total_memory // 10
+    return max(2**30, tenth)
 
 
 def heads_per_call(q: torch.Tensor, k: torch.Tensor, kernel: str, tile: dict) -> int:

@@ -121,7 +121,7 @@ __device__ __forceinline__ uint32_t e2m1x8(const float2 (&v)[4]) {
 __global__ void __launch_bounds__(F4_THREADS, 1)
     attention_fp4_kernel(const uint8_t* __restrict__ q4, const uint32_t* __restrict__ sfq, const uint8_t* __restrict__ k4,
                          const uint32_t* __restrict__ sfk, const uint8_t* __restrict__ v4, const uint32_t* __restrict__ sfv,
-                         const float* __restrict__ qk_outer, const float* __restrict__ v_outer, const float* __restrict__ bias,
+                         const float* __restrict__ qk_outer, const float* __restrict__ k_outer, const float* __restrict__ v_outer, const float* __restrict__ bias,
                          int q_blocks, int smooth_q, __nv_bfloat16* __restrict__ out, TokenLayout out_layout, const __grid_constant__ PeerOutputs peers, int n_queries,
                          int n_keys, float scale_log2, uint32_t* __restrict__ p_words, int* status) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(F4_THREADS, 1)
         const int g = warp / 4, row = (warp % 4) * 32 + lane;
         const int q_row = (F4_TILES * blockIdx.x + g) * QUERY_TILE + row;
         const uint32_t my = tmem + (uint32_t((warp % 4) * 32) << 16) + g * 256;
-        const float c = qk_outer[head] * scale_log2;
+        const float c = (k_outer ? fmaxf(qk_outer[head] * k_outer[head], 1e-30f) : qk_outer[head]) * scale_log2;
         const float2 c2 = make_float2(c, c);
         const bool smoothed = bias != nullptr;
         float m = -INFINITY;
@@ -435,8 +435,8 @@ extern "C" int unica_b200_trace_read_fp4(long long* host_out) {
 }
 #endif
 
-static int attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4, const void* sfv,
-                         const float* qk_outer, const float* v_outer, const float* bias, int q_blocks, int smooth_q, void* out,
+int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4, const void* sfv,
+                         const float* qk_outer, const float* k_outer, const float* v_outer, const float* bias, int q_blocks, int smooth_q, void* out,
                          void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads, int n_queries, int n_keys,
                          float scale_log2, uint32_t* p_words, int* status, void* stream) {
     if (!q4 || !sfq || !k4 || !sfk || !v4 || !sfv || !qk_outer || !v_outer || !out) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: null pointer");
@@ -454,7 +454,7 @@ static int attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, 
         return unica_check_launch("attention_fp4 (shared memory size)");
     attention_fp4_kernel<<<grid, F4_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(
         q4, static_cast<const uint32_t*>(sfq), k4, static_cast<const uint32_t*>(sfk), v4, static_cast<const uint32_t*>(sfv), qk_outer,
-        v_outer, bias, q_blocks, smooth_q > 0 ? smooth_q : 1, static_cast<__nv_bfloat16*>(out), to_layout(out_layout), peers, n_queries,
+        k_outer, v_outer, bias, q_blocks, smooth_q > 0 ? smooth_q : 1, static_cast<__nv_bfloat16*>(out), to_layout(out_layout), peers, n_queries,
         n_keys, scale_log2, p_words, status);
     return unica_check_launch("attention_fp4");
 }
@@ -463,7 +463,7 @@ extern "C" int unica_b200_attention_fp4(const uint8_t* q4, const void* sfq, cons
                                         const void* sfv, const float* qk_outer, const float* v_outer, const float* bias,
                                         int q_blocks, int smooth_q, void* out, unica_token_layout out_layout, int heads,
                                         int n_queries, int n_keys, float scale_log2, int* status, void* stream) {
-    return attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, v_outer, bias, q_blocks, smooth_q, out, nullptr, 0, out_layout, heads,
+    return unica_attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, nullptr, v_outer, bias, q_blocks, smooth_q, out, nullptr, 0, out_layout, heads,
                          n_queries, n_keys, scale_log2, nullptr, status, stream);
 }
 
@@ -472,7 +472,7 @@ extern "C" int unica_b200_attention_fp4_peers(const uint8_t* q4, const void* sfq
                                               const float* bias, int q_blocks, int smooth_q, void* out, void* const* peer_out,
                                               int n_peers, unica_token_layout out_layout, int heads, int n_queries, int n_keys,
                                               float scale_log2, int* status, void* stream) {
-    return attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, v_outer, bias, q_blocks, smooth_q, out, peer_out, n_peers, out_layout, heads,
+    return unica_attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, nullptr, v_outer, bias, q_blocks, smooth_q, out, peer_out, n_peers, out_layout, heads,
                          n_queries, n_keys, scale_log2, nullptr, status, stream);
 }
 
@@ -482,6 +482,6 @@ extern "C" int unica_b200_attention_fp4_codes(const uint8_t* q4, const void* sfq
                                               int heads, int n_queries, int n_keys, float scale_log2, uint32_t* p_words, int* status,
                                               void* stream) {
     if (!p_words) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4_codes: null pointer");
-    return attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, v_outer, bias, q_blocks, smooth_q, out, nullptr, 0, out_layout, heads,
+    return unica_attention_fp4(q4, sfq, k4, sfk, v4, sfv, qk_outer, nullptr, v_outer, bias, q_blocks, smooth_q, out, nullptr, 0, out_layout, heads,
                          n_queries, n_keys, scale_log2, p_words, status, stream);
 }

@@ -781,7 +781,7 @@ __global__ void __launch_bounds__(128) selftest_mma_i8_kernel(const uint8_t* __r
 
 using namespace unica;
 
-static int attention_int8(const int8_t* q8, const float* q_scale, const int8_t* k8, const float* k_scale, const int8_t* v8,
+int unica_attention_int8(const int8_t* q8, const float* q_scale, const int8_t* k8, const float* k_scale, const int8_t* v8,
                           const float* v_scale, const float* v_token, int v_mode, const int* outlier_keys, const float* outlier_rows,
                           int n_outliers, void* out, void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads,
                           int n_queries, int n_keys, float scale_log2, int* status, void* stream) {
@@ -839,7 +839,7 @@ extern "C" int unica_b200_attention_int8(const int8_t* q8, const float* q_scale,
                                          const int* outlier_keys, const float* outlier_rows, int n_outliers, void* out,
                                          unica_token_layout out_layout, int heads, int n_queries, int n_keys, float scale_log2,
                                          int* status, void* stream) {
-    return attention_int8(q8, q_scale, k8, k_scale, v8, v_scale, v_token, v_mode, outlier_keys, outlier_rows, n_outliers, out, nullptr, 0,
+    return unica_attention_int8(q8, q_scale, k8, k_scale, v8, v_scale, v_token, v_mode, outlier_keys, outlier_rows, n_outliers, out, nullptr, 0,
                           out_layout, heads, n_queries, n_keys, scale_log2, status, stream);
 }
 
@@ -848,7 +848,7 @@ extern "C" int unica_b200_attention_int8_peers(const int8_t* q8, const float* q_
                                                const int* outlier_keys, const float* outlier_rows, int n_outliers, void* out,
                                                void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads,
                                                int n_queries, int n_keys, float scale_log2, int* status, void* stream) {
-    return attention_int8(q8, q_scale, k8, k_scale, v8, v_scale, v_token, v_mode, outlier_keys, outlier_rows, n_outliers, out, peer_out,
+    return unica_attention_int8(q8, q_scale, k8, k_scale, v8, v_scale, v_token, v_mode, outlier_keys, outlier_rows, n_outliers, out, peer_out,
                           n_peers, out_layout, heads, n_queries, n_keys, scale_log2, status, stream);
 }
 

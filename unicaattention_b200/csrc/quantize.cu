@@ -107,8 +107,9 @@ __global__ void __launch_bounds__(THREADS) quantize_v_int8_kernel(const __nv_bfl
                                                                    float* __restrict__ v_token) {
     __shared__ VTileSmem sm;
     const int head = blockIdx.y;
-    v_int8_tile<PER_TOKEN>(v, in, low ? low + head * HEAD_DIM : nullptr, high ? high + head * HEAD_DIM : nullptr, skip, head, blockIdx.x,
-                           gridDim.x, n_tokens, v8, v_scale, v_token, sm);
+    v_int8_tile<PER_TOKEN>(v, in, low ? low + head * HEAD_DIM : nullptr, high ? high + head * HEAD_DIM : nullptr,
+                           [&](int token) { return skip && skip[size_t(head) * n_tokens + token]; }, head, blockIdx.x, gridDim.x, n_tokens, v8, v_scale,
+                           v_token, sm);
 }
 
 }  // namespace unica

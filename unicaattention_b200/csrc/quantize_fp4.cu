@@ -9,50 +9,10 @@
 // contraction index in the low nibble), and the scale bytes in the order the attention kernel copies them into tensor
 // memory.  Keys inside a 64-key tile are stored in the reference's slot order (bench/emulate.py:116-119): the 16-key
 // scale blocks of P and V are defined on that order, so it is part of the numerics.
-#include <cuda_fp8.h>
-
 #include "capi.h"
+#include "quantize_fp4.cuh"
 
 namespace unica {
-
-constexpr int FP4_THREADS = 256;
-constexpr int V4_ROWS = 144;      // 128 channels + 16 rows of ones: their column of P.V is the running denominator
-constexpr int V4_SF_WORDS = 256;  // scale words of a tile: two blocks of [32 lanes][4], the second for rows 128..143
-
-__host__ __device__ __forceinline__ int slot_key(int k) { return 32 * (k / 32) + 8 * (k % 8 / 2) + 2 * (k % 32 / 8) + k % 2; }
-
-__device__ __forceinline__ uint32_t to_e4m3(float x) { return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3); }
-__device__ __forceinline__ float from_e4m3(uint32_t byte) {
-    return __half2float(__half(__nv_cvt_fp8_to_halfraw(static_cast<__nv_fp8_storage_t>(byte), __NV_E4M3)));
-}
-
-// 8 floats -> 8 e2m1 codes, element i in nibble i.
-__device__ __forceinline__ uint32_t pack_e2m1x8(const float* v) {
-    uint32_t word;
-    asm("{\n\t"
-        ".reg .b8 b0, b1, b2, b3;\n\t"
-        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
-        "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-        "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-        "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-        "mov.b32 %0, {b0, b1, b2, b3};\n\t"
-        "}"
-        : "=r"(word)
-        : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
-    return word;
-}
-
-// One block of 16 values: scale byte and 16 codes (two words).
-__device__ __forceinline__ void quantize_block16(float (&v)[16], float outer, uint32_t& byte, uint2& codes) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    byte = to_e4m3(__fdiv_rn(amax * (1.0f / 6.0f), outer));
-    const float scale = from_e4m3(byte) * outer;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = scale > 0.0f ? __fdiv_rn(v[i], scale) : 0.0f;
-    codes = make_uint2(pack_e2m1x8(v), pack_e2m1x8(v + 8));
-}
 
 // outer[head] = max(max |x - mean| * (1/2688), 1e-30) from the per-channel (and per mean group) min and max of x:
 // the extreme elements go through the same float subtraction as every element, so this is the head's exact maximum
@@ -75,11 +35,7 @@ __global__ void __launch_bounds__(HEAD_DIM) nvfp4_outer_rows_kernel(const float*
     if (c == 0) outer[head] = fmaxf(fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])) * (1.0f / 2688.0f), 1e-30f);
 }
 
-// Q or K minus its mean in NVFP4 along the channels, one block per tile of ROWS tokens (128: Q, 64: K).
-// SLOTS: row r of a tile holds token tile * 64 + slot_key(r) (K); else token tile * ROWS + r (Q).
-// mean: [heads][groups][128], one group per mean_tokens tokens, or null.
-// codes: [heads][tiles][4 chunks of 32 channels][ROWS][16] bytes; sf: Q [heads][tiles][2 halves of 64 channels][128][4]
-// bytes, K [heads][tiles][32 lanes][4 words][4] bytes (see the store below).
+// One block per tile.  mean: [heads][groups][128], one group per mean_tokens tokens, or null.  Grid (tiles, heads).
 template <int ROWS, bool SLOTS>
 __global__ void __launch_bounds__(FP4_THREADS) quantize_rows_fp4_kernel(const __nv_bfloat16* __restrict__ x, TokenLayout in,
                                                                          const float* __restrict__ mean, int mean_tokens, int groups,
@@ -87,98 +43,20 @@ __global__ void __launch_bounds__(FP4_THREADS) quantize_rows_fp4_kernel(const __
                                                                          uint8_t* __restrict__ codes, uint8_t* __restrict__ sf,
                                                                          RopeTable rope) {
     const int head = blockIdx.y, tile = blockIdx.x;
-    const float head_outer = outer[head];
-    uint8_t* tile_codes = codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM / 2);
-    uint8_t* tile_sf = sf + (size_t(head) * gridDim.x + tile) * (ROWS * 8);
-#pragma unroll
-    for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
-        const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;  // block of 16 channels
-        const int token = SLOTS ? tile * ROWS + slot_key(row) : tile * ROWS + row;
-        float v[16];
-        if (token < n_tokens) {
-            const __nv_bfloat16* src = x + in.offset(head, token) + block * 16;
-            const uint4 raw[2] = {load_bf16x8(src, in.half), load_bf16x8(src + 8, in.half)};
-            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw);
-            const float* mu = mean ? mean + (size_t(head) * groups + token / mean_tokens) * HEAD_DIM + block * 16 : nullptr;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 f = __bfloat1622float2(pairs[i]);
-                v[2 * i] = f.x, v[2 * i + 1] = f.y;
-            }
-            if (rope.table) {  // rotate first: the mean is the rotated x's
-                const __half* f = rope.row(in, head, token);
-                rope8(*reinterpret_cast<float(*)[8]>(v), f, block * 16);
-                rope8(*reinterpret_cast<float(*)[8]>(v + 8), f, block * 16 + 8);
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] -= mu ? mu[i] : 0.0f;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-        }
-        uint32_t byte;
-        uint2 packed;
-        quantize_block16(v, head_outer, byte, packed);
-        *reinterpret_cast<uint2*>(tile_codes + ((block / 2) * ROWS + row) * 16 + (block % 2) * 8) = packed;
-        // the word of (K step = block / 4, row): Q [2][128] by row; K [32 lanes][4]: word 2 step + row / 32 of lane row % 32,
-        // the 16 bytes tcgen05.cp hands to one tensor-memory lane
-        const int word = ROWS == 64 ? (row % 32) * 4 + 2 * (block / 4) + row / 32 : (block / 4) * ROWS + row;
-        tile_sf[word * 4 + block % 4] = uint8_t(byte);
-    }
+    rows_fp4_tile<ROWS, SLOTS>(x, in, [&](int token) { return mean ? mean + (size_t(head) * groups + token / mean_tokens) * HEAD_DIM : nullptr; }, outer[head],
+                               head, tile, n_tokens, codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM / 2),
+                               sf + (size_t(head) * gridDim.x + tile) * (ROWS * 8), rope);
 }
 
-// V in NVFP4 along the keys, per channel, one block per tile of 64 keys (slot order).  low/high: the channel's min and
-// max over the head ([heads][128]); v_outer [heads][128] is written by tile 0.
-// codes: [heads][tiles][2 chunks of 32 slots][144 rows][16] bytes, rows 128..143 all ones (code 0x2);
-// sf: [heads][tiles][2 blocks][32 lanes][4 words] of 4 bytes: block 0 word c / 32 of lane c % 32 = channel c's four
-// bytes, block 1 word 0 of lanes 0..15 = ones (0x38) for rows 128..143, zeros elsewhere.
+// One block per tile of 64 keys.  low/high: [heads][128]; v_outer [heads][128].  Grid (tiles, heads).
 __global__ void __launch_bounds__(FP4_THREADS) quantize_v_fp4_kernel(const __nv_bfloat16* __restrict__ v, TokenLayout in,
                                                                       const float* __restrict__ low, const float* __restrict__ high,
                                                                       int n_tokens, uint8_t* __restrict__ codes, uint8_t* __restrict__ sf,
                                                                       float* __restrict__ v_outer) {
-    __shared__ float tile[KEY_TILE][HEAD_DIM + 1];  // by slot
+    __shared__ V4Tile tile;
     const int head = blockIdx.y, t = blockIdx.x;
-    for (int item = threadIdx.x; item < KEY_TILE * 16; item += FP4_THREADS) {
-        const int slot = item / 16, chunk = item % 16, key = t * KEY_TILE + slot_key(slot);
-        float f[8];
-        if (key < n_tokens) {
-            const uint4 raw = load_bf16x8(v + in.offset(head, key) + chunk * 8, in.half);
-            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 p = __bfloat1622float2(pairs[i]);
-                f[2 * i] = p.x, f[2 * i + 1] = p.y;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) tile[slot][chunk * 8 + i] = f[i];
-    }
-    __syncthreads();
-    uint8_t* tile_codes = codes + (size_t(head) * gridDim.x + t) * (V4_ROWS * 32);
-    uint8_t* tile_sf = sf + (size_t(head) * gridDim.x + t) * (V4_SF_WORDS * 4);
-    for (int item = threadIdx.x; item < HEAD_DIM * 4; item += FP4_THREADS) {
-        const int c = item % HEAD_DIM, block = item / HEAD_DIM;  // block of 16 slots
-        const int ci = head * HEAD_DIM + c;
-        const float outer = fmaxf(fmaxf(high[ci], -low[ci]) * (1.0f / 2688.0f), 1e-30f);
-        if (t == 0 && block == 0) v_outer[ci] = outer;
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = tile[block * 16 + i][c];
-        uint32_t byte;
-        uint2 packed;
-        quantize_block16(x, outer, byte, packed);
-        *reinterpret_cast<uint2*>(tile_codes + ((block / 2) * V4_ROWS + c) * 16 + (block % 2) * 8) = packed;
-        tile_sf[((c % 32) * 4 + c / 32) * 4 + block] = uint8_t(byte);  // word c / 32 of lane c % 32
-    }
-    for (int item = threadIdx.x; item < 2 * 16 * 4; item += FP4_THREADS) {  // the rows of ones: 2 chunks x 16 rows x 4 words
-        const int chunk = item / 64, row = 128 + item / 4 % 16, word = item % 4;
-        reinterpret_cast<uint32_t*>(tile_codes + (chunk * V4_ROWS + row) * 16)[word] = 0x22222222u;
-    }
-    if (threadIdx.x < 128)  // second block: rows 128..143 (ones) are word 0 of lanes 0..15, the rest zeros
-        reinterpret_cast<uint32_t*>(tile_sf)[128 + threadIdx.x] = threadIdx.x % 4 == 0 && threadIdx.x / 4 < 16 ? 0x38383838u : 0u;
+    v_fp4_tile(v, in, low + head * HEAD_DIM, high + head * HEAD_DIM, head, t, n_tokens, codes + (size_t(head) * gridDim.x + t) * (V4_ROWS * 32),
+               sf + (size_t(head) * gridDim.x + t) * (V4_SF_WORDS * 4), v_outer + head * HEAD_DIM, tile);
 }
 
 // The part of the scores that Q smoothing took out, added back exactly (bench/emulate.py:308-309; the reference's

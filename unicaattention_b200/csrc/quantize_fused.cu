@@ -20,6 +20,7 @@
 // here too: a head's tiles are dealt to `per_group` blocks, and `per_group` follows from the device and the token count
 // alone, not from how many heads the call holds, so a head's operands do not depend on what it is quantized with.
 #include "capi.h"
+#include "quantize_call.h"
 #include "quantize_int8.cuh"
 
 namespace unica {
@@ -340,6 +341,14 @@ static int quantize_fused(bool is_v, const void* x, unica_token_layout layout, i
     if (scratch_bytes < UNICA_B200_FUSED_SCRATCH_BYTES || reinterpret_cast<uintptr_t>(scratch) % 16)
         return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize (one launch): scratch must be 16-byte aligned and hold UNICA_B200_FUSED_SCRATCH_BYTES");
     if (int e = unica_check_device()) return e;
+    if (n_tokens <= CALL_TOKENS) {  // short: a cluster of eight blocks per head (see quantize_call.h)
+        CallQuantize call = {};
+        call.heads = heads, call.v_mode = UNICA_B200_V_CHANNEL;
+        CallOperand& op = is_v ? call.v : call.k;
+        op.x = static_cast<const __nv_bfloat16*>(x), op.in = to_layout(layout), op.n_tokens = n_tokens, op.tiles = tiles;
+        op.codes = reinterpret_cast<uint8_t*>(codes), op.scales = scales, op.mean = stat;
+        return quantize_call_int8(call, static_cast<cudaStream_t>(stream));
+    }
     const bool half = layout.dtype == UNICA_B200_FLOAT16;
     const void* kernel = is_v ? (half ? reinterpret_cast<const void*>(quantize_head_int8_kernel<true, true>) : reinterpret_cast<const void*>(quantize_head_int8_kernel<true, false>))
                               : (half ? reinterpret_cast<const void*>(quantize_head_int8_kernel<false, true>) : reinterpret_cast<const void*>(quantize_head_int8_kernel<false, false>));
@@ -387,4 +396,16 @@ extern "C" int unica_b200_quantize_q_int8_stream(const void* q, unica_token_layo
     kernel<<<grid, STREAM_THREADS, RING_BYTES, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(q), to_layout(layout), heads,
                                                                                       n_tokens, tiles, codes, scales);
     return unica_check_launch("quantize_q_int8_stream");
+}
+
+extern "C" int unica_b200_quantize_v_int8_outliers(const void* v, unica_token_layout layout, int heads, int n_tokens, int n_outliers, int8_t* v8,
+                                                   float* v_scale, int* keys, float* rows, void* stream) {
+    if (!v || !v8 || !v_scale || !keys || !rows) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_v_int8_outliers: null pointer");
+    if (heads <= 0 || n_tokens <= 0 || n_tokens > CALL_TOKENS || n_outliers < 1 || n_outliers > 8)
+        return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_v_int8_outliers: heads must be positive, n_tokens in 1..8192, n_outliers in 1..8");
+    CallQuantize call = {};
+    call.heads = heads, call.v_mode = UNICA_B200_V_OUTLIERS, call.n_outliers = n_outliers, call.outlier_keys = keys, call.outlier_rows = rows;
+    call.v.x = static_cast<const __nv_bfloat16*>(v), call.v.in = to_layout(layout), call.v.n_tokens = n_tokens;
+    call.v.tiles = (n_tokens + KEY_TILE - 1) / KEY_TILE, call.v.codes = reinterpret_cast<uint8_t*>(v8), call.v.scales = v_scale;
+    return quantize_call_int8(call, static_cast<cudaStream_t>(stream));
 }

@@ -150,11 +150,11 @@ struct VTileSmem {
     __align__(16) __nv_bfloat16 tile[KEY_TILE][HEAD_DIM];
     float key_scale[KEY_TILE], key_inv[KEY_TILE];
 };
-// low, high: this head's [128] (global or shared memory); tiles: key tiles per head; v_scale [heads][128] or null (the
-// caller writes it); sm: free again after a __syncthreads().
-template <bool PER_TOKEN>
+// low, high: this head's [128] (global or shared memory); skip(token): the key is written as zeros; tiles: key tiles per head;
+// v_scale [heads][128] or null (the caller writes it); sm: free again after a __syncthreads().
+template <bool PER_TOKEN, typename Skip>
 __device__ __forceinline__ void v_int8_tile(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, const float* low, const float* high,
-                                            const uint8_t* __restrict__ skip, int head, int t, int tiles, int n_tokens,
+                                            Skip skip, int head, int t, int tiles, int n_tokens,
                                             int8_t* __restrict__ v8, float* __restrict__ v_scale, float* __restrict__ v_token,
                                             VTileSmem& sm) {
     // The tile goes through shared memory as bf16, keys x channels, and comes out transposed: a thread then owns one
@@ -169,7 +169,7 @@ __device__ __forceinline__ void v_int8_tile(const __nv_bfloat16* __restrict__ v,
         const int key = it * (THREADS / 16) + threadIdx.x / 16;
         const bool valid = token0 + key < n_tokens;
         uint4 raw = make_uint4(0, 0, 0, 0);
-        if (valid && !(skip && skip[size_t(head) * n_tokens + token0 + key]))
+        if (valid && !skip(token0 + key))
             raw = load_bf16x8(v + in.offset(head, token0 + key) + chunk * 8, in.half);
         *reinterpret_cast<uint4*>(&tile[key][chunk * 8]) = raw;
         if (PER_TOKEN) {  // one scale per key over its channels: the 16 threads of a key share their maxima

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import struct
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -59,7 +60,15 @@ SIGNATURES = {
     "unica_b200_quantize_int8_rope": [_P, TokenLayout, _P, _P, _LL, _I, _I, _I, _I, _P, _P, _P],
     "unica_b200_quantize_fp4_rows_rope": [_P, TokenLayout, _P, _I, _P, _LL, _P, _I, _I, _I, _I, _P, _P, _P],
     "unica_b200_smooth_bias_rope": [_P, TokenLayout, _P, _P, _P, _LL, _I, _I, _I, _F, _P, _P, _P],
+    "unica_b200_quantize_v_int8_outliers": [_P, TokenLayout, _I, _I, _I, _P, _P, _P, _P, _P],
+    "unica_b200_attention_workspace": [_P, _P],
+    "unica_b200_attention_call": [_P, _P],
 }
+# struct unica_b200_call as bytes, in the header's order (packing forty numbers at once costs a microsecond, filling a
+# ctypes structure several): q, k, v, out, workspace, its size, rope, its batch stride, peer_out, status, stream; the four
+# layouts; heads, n_queries, n_keys, kernel, v_mode, n_outliers, smooth_q, n_peers; scale_log2
+pack_call = struct.Struct("@PPPPPNPqPPP" + "qqqii" * 4 + "iiiiiiiif4x").pack
+CALL_TOKENS = 8192  # keys up to which a call with V_OUTLIERS fits one entry point
 
 
 @functools.cache
@@ -98,8 +107,26 @@ def stream() -> ctypes.c_void_p:
 
 # kernels an entry point launches when it succeeds (the statistics passes: partial sums, then their reduction)
 KERNELS_PER_CALL = {"unica_b200_channel_stats": 2, "unica_b200_channel_stats_rope": 2, "unica_b200_channel_stats_masked": 2,
-                    "unica_b200_channel_stats_static": 2, "unica_b200_version": 0}
+                    "unica_b200_channel_stats_static": 2, "unica_b200_version": 0, "unica_b200_attention_workspace": 0}
 launches = 0  # kernels of this library launched by this process so far (benchmarks report differences of it)
+
+
+def attention_workspace(call_bytes: bytes) -> int:
+    """Bytes of workspace the call wants."""
+    size = ctypes.c_size_t()
+    call("unica_b200_attention_workspace", call_bytes, ctypes.byref(size))
+    return size.value
+
+
+def attention_call(call_bytes: bytes) -> None:
+    """unica_b200_attention_call on a packed call."""
+    global launches
+    queued = ctypes.c_int()
+    code = library().unica_b200_attention_call(call_bytes, ctypes.byref(queued))
+    launches += queued.value
+    if code:
+        message = f"attention: {last_error()}"
+        raise ValueError(message) if code == ERR_ARGUMENT else RuntimeError(message)
 
 
 def call(name: str, *args) -> None:
