@@ -153,7 +153,7 @@ int unica_b200_attention_int8(const int8_t* q8, const float* q_scale, const int8
 /* ---- fast mode (NVFP4) ------------------------------------------------------------------------------------------
  * Operand layouts, per head (two e2m1 codes per byte, the lower contraction index in the low nibble; one e4m3 scale
  * byte per 16 elements along the contraction; keys of a 64-key tile in the reference's slot order, bench/emulate.py:116-119):
- *   Q4  [q_tiles (even)][4 chunks of 32 channels][128 rows][16]  8 KB/tile   SFQ [q_tiles][2 halves of 64 channels][128][4]
+ *   Q4  [q_tiles (even)][4 chunks of 32 channels][128 rows][16]  8 KB/tile   SFQ [q_tiles][2 halves of 64 channels][32 lanes][4 words][4]
  *   K4  [k_tiles][4][64 slots][16]                               4 KB/tile   SFK [k_tiles][32 lanes][4 words][4]
  *   V4  [k_tiles][2 chunks of 32 slots][144 rows][16]            4.5 KB      SFV [k_tiles][2 blocks][32 lanes][4 words][4]
  *       rows 0..127 channels, rows 128..143 ones (their column of P.V is the softmax denominator)

@@ -16,6 +16,8 @@
 //   acc(g) = P^(g) . V8(g)     kind::i8 u8 x u8 -> s32, 128 x 128, 2 instructions of K = 32, two accumulators (g even / odd);
 //                              V8 is stored plus 128, see flush32
 //
+// (The copies are in the scores warp because a warp of their own, meeting it once per tile, measured 7 % slower.)
+//
 // Key tiles are counted across items (g), and every ring runs on from one item to the next: while the flush warps normalise
 // and store an item, the copies, scores and exponentials of the next one are under way.  With one block per item a block's
 // start (5500 cycles to the first P.V) and end (11700) were exposed, a fifth of a call of 4128 tokens.
@@ -43,6 +45,7 @@
 #include <atomic>
 #include <climits>
 
+#include "attention_common.cuh"
 #include "capi.h"
 
 namespace unica {
@@ -52,13 +55,6 @@ constexpr int SCORES_WARP = 0, PV_WARP = 1, FLUSH_WARP = 4, SOFTMAX_WARP = 8, AT
 // registers per thread after setmaxnreg; the block is launched with ATT_THREADS x LAUNCH_REGISTERS = 65536
 constexpr int LAUNCH_REGISTERS = 128, SOFTMAX_REGISTERS = 120, FLUSH_REGISTERS = 232, SERVICE_REGISTERS = 40;
 static_assert(128 * (2 * SOFTMAX_REGISTERS + FLUSH_REGISTERS + SERVICE_REGISTERS) <= ATT_THREADS * LAUNCH_REGISTERS, "the split must fit the launch");
-template <int REGISTERS>
-__device__ __forceinline__ void set_registers() {  // every warp of a warpgroup executes it
-    if constexpr (REGISTERS > LAUNCH_REGISTERS)
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGISTERS));
-    else
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGISTERS));
-}
 constexpr int K_RING = 6;   // K8 tiles in shared memory: tile g + K_RING - S_RING is fetched when S(g) is issued (see scores_warp)
 constexpr int V_RING = 8;   // V8 tiles (and the keys' scales, per token): tile g is fetched when S(g) is issued
 constexpr int S_RING = 4;   // score buffers in tensor memory
@@ -66,23 +62,12 @@ constexpr int P_RING = 4;   // P^ images in shared memory
 constexpr int ST_RING = 8;  // (tile maximum, row sum) records on their way from the softmax to the flush threads
 // The record of tile g is overwritten by the softmax of tile g + ST_RING, which waits for the flush of tile g + ST_RING - P_RING.
 static_assert(ST_RING > P_RING, "a record must have been read before it is overwritten");
-// Tile g's slot in a ring of N, and the phase parity of the slot's barrier for it.
-template <int N>
-__device__ __forceinline__ int slot(int g) {
-    static_assert((N & (N - 1)) == 0, "rings are powers of two: slots and parities are bits of the tile count");
-    return g & (N - 1);
-}
-template <int N>
-__device__ __forceinline__ int round_parity(int g) {
-    return (g / N) & 1;
-}
 constexpr int Q_BYTES = QUERY_TILE * HEAD_DIM;  // 16384
 constexpr int K_BYTES = KEY_TILE * HEAD_DIM;    // 8192
 constexpr int V_BYTES = KEY_TILE * HEAD_DIM;    // 8192
 constexpr int TOK_BYTES = 2 * KEY_TILE * 4;     // 512
 constexpr int P_BYTES = QUERY_TILE * KEY_TILE;  // 8192
 constexpr int SCALE_BYTES = HEAD_DIM * 4;       // 512
-constexpr int STAGED_PITCH = HEAD_DIM * 2 + 16;  // bytes from one staged output row to the next: rows of a quarter-warp on different banks
 constexpr int TMEM_COLUMNS = 512;
 constexpr int COL_S = 0, COL_ACC = 256;
 constexpr int OUTLIER_BATCH = 16;  // outlier keys whose rows are in shared memory at a time (the epilogue of the outliers mode)
@@ -137,14 +122,6 @@ __device__ __forceinline__ void flush32(const float2 (&y)[16], float2* o, float2
     for (int i = 0; i < 16; ++i) o[i] = fma2(beta2, y[i], o[i]);
 }
 
-// What a block's items are: tiles of 128 query rows, head by head.
-struct Items {
-    int tiles, allocated, count;  // query tiles per head: with queries in them, and in Q8 (an even number); items of the call
-    __device__ __forceinline__ int mine() const { return (count - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x); }  // of this block
-    __device__ __forceinline__ int head(int item) const { return item / tiles; }
-    __device__ __forceinline__ int tile(int item) const { return item % tiles; }
-};
-
 struct AttArgs {
     const int8_t *q8, *k8, *v8;
     const float *q_scale, *k_scale, *v_scale, *v_token;
@@ -162,9 +139,6 @@ struct AttArgs {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // the service warps; what they issue, one elected lane issues (see elect_one() in common.cuh)
-
-// A descriptor `units` of 16 bytes further on in shared memory (its address is in the low word).
-__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t units) { return (desc & 0xffffffff00000000ull) | (uint32_t(desc) + units); }
 
 // The tensor-core work of a tile in one statement, executed by a whole converged warp and issued by one elected lane: election
 // and instructions under one predicate, with no branch around them.  `if (elect_one()) { .. }` inside a loop of the warp took
@@ -203,30 +177,6 @@ __device__ __forceinline__ void issue_pv(uint32_t d, uint64_t p_desc, uint64_t v
         "l"(p_desc), "l"(v_desc), "l"(desc_at(p_desc, P_STEP)), "l"(desc_at(v_desc, V_STEP)), "r"(IDESC_PV), "r"(smem_u32(full))
         : "memory");
     static_assert(KEY_TILE == 64 && HEAD_DIM == 128, "two instructions of K = 32 for P.V, four for the scores");
-}
-__device__ __forceinline__ void commit_elected(uint64_t* bar) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred e;\n\t"
-        ".reg .b32 r;\n\t"
-        "elect.sync r|e, 0xffffffff;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
-        "}" ::"r"(smem_u32(bar))
-        : "memory");
-}
-
-// A copy to shared memory whose arrival its barrier counts, issued by one elected lane of a converged warp.
-__device__ __forceinline__ void copy_elected(void* dst, const void* src, int bytes, uint64_t* full) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred e;\n\t"
-        ".reg .b32 r;\n\t"
-        "elect.sync r|e, 0xffffffff;\n\t"
-        "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
-        "@e cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t"
-        "}" ::"r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(full))
-        : "memory");
 }
 
 // S(g), as soon as K8(g) has landed and the softmax of tile g - S_RING has handed the scores buffer back; and all copies, none
@@ -645,33 +595,10 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
                 make_uint4(output_pair(v[0].x * s0.x * inv, v[0].y * s0.y * inv, a.out_layout.half), output_pair(v[1].x * s0.z * inv, v[1].y * s0.w * inv, a.out_layout.half),
                            output_pair(v[2].x * s1.x * inv, v[2].y * s1.y * inv, a.out_layout.half), output_pair(v[3].x * s1.z * inv, v[3].y * s1.w * inv, a.out_layout.half));
         }
-        const int first_row = q_tile * QUERY_TILE + warp * 32;
-        const bool stored = ok && first_row + lane < a.n_queries;
-        fence_proxy_async();
-        if (stored) bulk_store(a.out + a.out_layout.offset(head, first_row + lane), staged_row, HEAD_DIM * 2);
-        bulk_store_commit();
-        __syncwarp();
-        if (a.peers.count > 0 && ok) {  // plain stores to other GPUs, two whole rows per instruction
-            for (int pair = 0; pair < 16; ++pair) {
-                const int r = 2 * pair + lane / 16;
-                const uint4 value = *reinterpret_cast<const uint4*>(staged + r * STAGED_PITCH + (lane % 16) * 16);
-                if (first_row + r < a.n_queries)
-                    for (int peer = 0; peer < a.peers.count; ++peer)
-                        *reinterpret_cast<uint4*>(a.peers.out[peer] + a.out_layout.offset(head, first_row + r) + (lane % 16) * 8) = value;
-            }
-            __syncwarp();
-        }
+        send_staged_rows(staged, lane, q_tile * QUERY_TILE + warp * 32, a.n_queries, head, a.out, a.out_layout, a.peers, ok);
         if (lane == 0) mbar_arrive(&sm.q_free[slot<2>(i)]);  // Q8 and V's scales have been used
     }
     bulk_store_read_wait();
-}
-
-// The block's shared memory as one role sees it: an address the compiler cannot relate to the other roles' (it otherwise
-// computes the addresses common to several roles before they part, and holds them in registers the computing loops need).
-__device__ __forceinline__ AttSmem& own_view(AttSmem& sm) {
-    uint32_t base = smem_u32(&sm);
-    asm volatile("" : "+r"(base));
-    return *static_cast<AttSmem*>(__cvta_shared_to_generic(base));
 }
 
 template <bool V_TOKEN, bool OUTLIERS>
@@ -700,13 +627,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_int8_kernel(const __
     const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
 
     if (warp >= FLUSH_WARP && warp < SOFTMAX_WARP) {
-        set_registers<FLUSH_REGISTERS>();
+        set_registers<FLUSH_REGISTERS, LAUNCH_REGISTERS>();
         flush_warps<V_TOKEN, OUTLIERS>(own_view(sm), a, k_tiles, tmem, warp - FLUSH_WARP, row);
     } else if (warp >= SOFTMAX_WARP) {
-        set_registers<SOFTMAX_REGISTERS>();
+        set_registers<SOFTMAX_REGISTERS, LAUNCH_REGISTERS>();
         softmax_warps<V_TOKEN>(own_view(sm), a, k_tiles, tmem, warp - SOFTMAX_WARP, row);
     } else {
-        set_registers<SERVICE_REGISTERS>();
+        set_registers<SERVICE_REGISTERS, LAUNCH_REGISTERS>();
         if (warp == SCORES_WARP) {
             scores_warp<V_TOKEN>(own_view(sm), a, k_tiles, tmem);
         } else if (warp == PV_WARP) {

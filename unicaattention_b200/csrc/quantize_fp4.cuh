@@ -50,8 +50,8 @@ __device__ __forceinline__ void quantize_block16(float (&v)[16], float outer, ui
 // Q or K minus its mean in NVFP4 along the channels: one tile of ROWS tokens (128: Q, 64: K) by a block of FP4_THREADS.
 // SLOTS: row r of a tile holds token tile * 64 + slot_key(r) (K); else token tile * ROWS + r (Q).
 // mean_of(token): the 128 means that go with the token, or null.
-// codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][128][4] bytes, K [32 lanes]
-// [4 words][4] bytes (see the store below).
+// codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][32 lanes][4 words]
+// [4] bytes, K [32 lanes][4 words][4] bytes (see the store below).
 template <int ROWS, bool SLOTS, typename MeanOf>
 __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, float head_outer, int head,
                                               int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
@@ -86,9 +86,9 @@ __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ 
         uint2 packed;
         quantize_block16(v, head_outer, byte, packed);
         *reinterpret_cast<uint2*>(tile_codes + ((block / 2) * ROWS + row) * 16 + (block % 2) * 8) = packed;
-        // the word of (K step = block / 4, row): Q [2][128] by row; K [32 lanes][4]: word 2 step + row / 32 of lane row % 32,
-        // the 16 bytes tcgen05.cp hands to one tensor-memory lane
-        const int word = ROWS == 64 ? (row % 32) * 4 + 2 * (block / 4) + row / 32 : (block / 4) * ROWS + row;
+        // the word of (K step = block / 4, row): Q [2][32 lanes][4]: word row / 32 of lane row % 32; K [32 lanes][4]: word 2 step +
+        // row / 32 of lane row % 32: the 16 bytes tcgen05.cp hands to one tensor-memory lane
+        const int word = ROWS == 64 ? (row % 32) * 4 + 2 * (block / 4) + row / 32 : (block / 4) * ROWS + (row % 32) * 4 + row / 32;
         tile_sf[word * 4 + block % 4] = uint8_t(byte);
     }
 }

@@ -23,8 +23,9 @@ SLOT_KEY = tuple(32 * (k // 32) + 8 * (k % 8 // 2) + 2 * (k % 32 // 8) + k % 2 f
 
 
 class FP4Rows(NamedTuple):
-    """Q or K in NVFP4: codes uint8 [batch, heads, tiles, 4, rows, 16]; scale bytes uint8, Q [batch, heads, tiles, 2, 128, 4],
-    K [batch, heads, tiles, 32, 4, 4] (lane, word 2 step + row / 32, byte: the order tcgen05.cp takes)."""
+    """Q or K in NVFP4: codes uint8 [batch, heads, tiles, 4, rows, 16]; scale bytes uint8, Q [batch, heads, tiles, 2, 32, 4, 4]
+    (step, lane, word row / 32, byte), K [batch, heads, tiles, 32, 4, 4] (lane, word 2 step + row / 32, byte): the order
+    tcgen05.cp takes."""
 
     codes: torch.Tensor
     sf: torch.Tensor
@@ -72,7 +73,7 @@ def quantize_fp4_rows(x: torch.Tensor, mean: torch.Tensor | None, pad_to: int = 
     need = math.ceil(n / rows)
     tiles = need if tiles is None else tiles
     codes = torch.empty(batch, heads, tiles, 4, rows, 16, dtype=torch.uint8, device=x.device)
-    sf = torch.empty((batch, heads, tiles, 32, 4, 4) if rows == 64 else (batch, heads, tiles, 2, rows, 4), dtype=torch.uint8, device=x.device)
+    sf = torch.empty((batch, heads, tiles, 32, 4, 4) if rows == 64 else (batch, heads, tiles, 2, 32, 4, 4), dtype=torch.uint8, device=x.device)
     lib.call("unica_b200_quantize_fp4_rows" + ("_rope" if rope is not None else ""), lib.ptr(x), _layout(x), lib.ptr(mean_arg), per,
              *unica.rope_args(rope, x), lib.ptr(outer), batch * heads, n, rows, tiles, lib.ptr(codes), lib.ptr(sf), lib.stream())
     return FP4Rows(codes, sf), outer
@@ -136,7 +137,7 @@ def decode_fp4_rows(x4: FP4Rows, n: int, slots: bool = False) -> tuple[torch.Ten
     if rows == 64:  # K: [tiles, lane, (step, row / 32), byte] -> [tiles, row = 32 (row / 32) + lane, (step, byte)]
         s = sf.view(batch, heads, tiles, 32, 2, 2, 4).permute(0, 1, 2, 5, 3, 4, 6).reshape(batch, heads, tiles * rows, 8)
     else:
-        s = sf.permute(0, 1, 2, 4, 3, 5).reshape(batch, heads, tiles * rows, 8)
+        s = sf.permute(0, 1, 2, 5, 4, 3, 6).reshape(batch, heads, tiles * rows, 8)  # row = 32 word + lane
     if slots:  # row r of a tile holds key slot_key(r): put the keys back in order
         key_of = torch.tensor(SLOT_KEY, device=codes.device)
         order = (torch.arange(tiles, device=codes.device)[:, None] * rows + key_of).flatten()
