@@ -43,65 +43,108 @@ struct CallStats {
 __device__ __forceinline__ int share(int count, int rank) { return count * rank / CALL_CLUSTER; }
 
 // Sum, min and max per channel of 256-token block `b` into part[3][128]: channel_stats_kernel's arithmetic.
-template <typename Skip>
+template <bool SUMS, bool RANGE, typename Skip>
 __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const RopeTable& rope, Skip skip, int head, int b,
                                             int n_tokens, CallStats& sm, float (&part)[3][HEAD_DIM]) {
     const int chunk = threadIdx.x % 16, lane = threadIdx.x / 16;
-    float sum[8], low[8], high[8];
+    float2 sum[4], low[4], high[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sum[i] = 0.0f, low[i] = INFINITY, high[i] = -INFINITY;
-    const int end = min((b + 1) * CALL_BLOCK, n_tokens);
-#pragma unroll 8
-    for (int token = b * CALL_BLOCK + lane; token < end; token += CALL_LANES) {
-        float v[8];
-        load8(v, x + in.offset(head, token) + chunk * 8, in.half);
-        if (skip(token)) continue;
-        if (rope.table) rope8(v, rope.row(in, head, token), chunk * 8);
+    for (int i = 0; i < 4; ++i) sum[i] = make_float2(0.0f, 0.0f), low[i] = make_float2(INFINITY, INFINITY), high[i] = make_float2(-INFINITY, -INFINITY);
+    const int first = b * CALL_BLOCK + lane;
+    const __nv_bfloat16* src = x + in.offset(head, 0) + chunk * 8;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            sum[i] += v[i];
-            low[i] = fminf(low[i], v[i]);
-            high[i] = fmaxf(high[i], v[i]);
+    for (int part8 = 0; part8 < CALL_BLOCK / CALL_LANES; part8 += 8) {  // eight loads in flight
+        uint4 raw[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int token = first + (part8 + j) * CALL_LANES;
+            raw[j] = token < n_tokens ? load_bf16x8(src + token * in.token, in.half) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int token = first + (part8 + j) * CALL_LANES;
+            if (token >= n_tokens || skip(token)) continue;
+            float2 v[4];
+            unpack8(raw[j], v);
+            if (rope.table) rope8(*reinterpret_cast<float(*)[8]>(v), rope.row(in, head, token), chunk * 8);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (SUMS) sum[i] = add2(sum[i], v[i]);
+                if (RANGE) {
+                    low[i] = make_float2(fminf(low[i].x, v[i].x), fminf(low[i].y, v[i].y));
+                    high[i] = make_float2(fmaxf(high[i].x, v[i].x), fmaxf(high[i].y, v[i].y));
+                }
+            }
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        sm.lanes[0][lane][chunk * 8 + i] = sum[i];
-        sm.lanes[1][lane][chunk * 8 + i] = low[i];
-        sm.lanes[2][lane][chunk * 8 + i] = high[i];
+    for (int i = 0; i < 4; ++i) {
+        if (SUMS) *reinterpret_cast<float2*>(&sm.lanes[0][lane][chunk * 8 + 2 * i]) = sum[i];
+        if (RANGE) {
+            *reinterpret_cast<float2*>(&sm.lanes[1][lane][chunk * 8 + 2 * i]) = low[i];
+            *reinterpret_cast<float2*>(&sm.lanes[2][lane][chunk * 8 + 2 * i]) = high[i];
+        }
     }
     __syncthreads();
     if (threadIdx.x < HEAD_DIM) {
         float s = 0.0f, lo = INFINITY, hi = -INFINITY;
+#pragma unroll
         for (int l = 0; l < CALL_LANES; ++l) {
-            s += sm.lanes[0][l][threadIdx.x];
-            lo = fminf(lo, sm.lanes[1][l][threadIdx.x]);
-            hi = fmaxf(hi, sm.lanes[2][l][threadIdx.x]);
+            if (SUMS) s += sm.lanes[0][l][threadIdx.x];
+            if (RANGE) lo = fminf(lo, sm.lanes[1][l][threadIdx.x]), hi = fmaxf(hi, sm.lanes[2][l][threadIdx.x]);
         }
-        part[0][threadIdx.x] = s, part[1][threadIdx.x] = lo, part[2][threadIdx.x] = hi;
+        if (SUMS) part[0][threadIdx.x] = s;
+        if (RANGE) part[1][threadIdx.x] = lo, part[2][threadIdx.x] = hi;
     }
     __syncthreads();
 }
 
-// The head's mean, min and max into sm of every block of the cluster.  Every thread of the cluster calls it.
-template <typename Skip>
+// The head's mean (SUMS), min and max (RANGE) into sm of every block of the cluster.  Every thread of the cluster calls it.
+template <bool SUMS, bool RANGE, typename Skip>
 __device__ __forceinline__ void head_stats(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const RopeTable& rope, Skip skip, int head,
                                            int n_tokens, int rank, CallStats& sm) {
     const int blocks = (n_tokens + CALL_BLOCK - 1) / CALL_BLOCK, b0 = share(blocks, rank), b1 = share(blocks, rank + 1);
-    for (int b = b0; b < b1; ++b) block_stats(x, in, rope, skip, head, b, n_tokens, sm, sm.part[b - b0]);
+    for (int b = b0; b < b1; ++b) block_stats<SUMS, RANGE>(x, in, rope, skip, head, b, n_tokens, sm, sm.part[b - b0]);
     cg::this_cluster().sync();
     if (threadIdx.x < HEAD_DIM) {
+        // all blocks' partial results asked for before the first is added up: a trip to another SM takes some hundred cycles
         float s = 0.0f, lo = INFINITY, hi = -INFINITY;
-        for (int r = 0; r < CALL_CLUSTER; ++r) {
-            const CallStats* theirs = cg::this_cluster().map_shared_rank(&sm, r);
-            const int parts = share(blocks, r + 1) - share(blocks, r);
-            for (int i = 0; i < parts; ++i) {
-                s += theirs->part[i][0][threadIdx.x];
-                lo = fminf(lo, theirs->part[i][1][threadIdx.x]);
-                hi = fmaxf(hi, theirs->part[i][2][threadIdx.x]);
+        float theirs_s[CALL_CLUSTER], theirs_lo[CALL_CLUSTER], theirs_hi[CALL_CLUSTER];
+        const int most = (blocks + CALL_CLUSTER - 1) / CALL_CLUSTER;
+        if (most == 1) {
+#pragma unroll
+            for (int r = 0; r < CALL_CLUSTER; ++r) {
+                const CallStats* theirs = cg::this_cluster().map_shared_rank(&sm, r);
+                if (SUMS) theirs_s[r] = theirs->part[0][0][threadIdx.x];
+                if (RANGE) theirs_lo[r] = theirs->part[0][1][threadIdx.x], theirs_hi[r] = theirs->part[0][2][threadIdx.x];
+            }
+#pragma unroll
+            for (int r = 0; r < CALL_CLUSTER; ++r)
+                if (share(blocks, r + 1) > share(blocks, r)) {  // the others hold nothing
+                    if (SUMS) s += theirs_s[r];
+                    if (RANGE) lo = fminf(lo, theirs_lo[r]), hi = fmaxf(hi, theirs_hi[r]);
+                }
+        } else {
+#pragma unroll
+            for (int r = 0; r < CALL_CLUSTER; ++r) {
+                const CallStats* theirs = cg::this_cluster().map_shared_rank(&sm, r);
+                const int parts = share(blocks, r + 1) - share(blocks, r);
+                float part_s[CALL_PARTS], part_lo[CALL_PARTS], part_hi[CALL_PARTS];
+#pragma unroll
+                for (int i = 0; i < CALL_PARTS; ++i) {
+                    if (SUMS) part_s[i] = theirs->part[i][0][threadIdx.x];
+                    if (RANGE) part_lo[i] = theirs->part[i][1][threadIdx.x], part_hi[i] = theirs->part[i][2][threadIdx.x];
+                }
+#pragma unroll
+                for (int i = 0; i < CALL_PARTS; ++i)
+                    if (i < parts) {
+                        if (SUMS) s += part_s[i];
+                        if (RANGE) lo = fminf(lo, part_lo[i]), hi = fmaxf(hi, part_hi[i]);
+                    }
             }
         }
-        sm.mean[threadIdx.x] = s / float(n_tokens), sm.low[threadIdx.x] = lo, sm.high[threadIdx.x] = hi;
+        if (SUMS) sm.mean[threadIdx.x] = s / float(n_tokens);
+        if (RANGE) sm.low[threadIdx.x] = lo, sm.high[threadIdx.x] = hi;
     }
     __syncthreads();
 }
@@ -178,31 +221,37 @@ struct SkipKeys {
     }
 };
 
-// V_MODE: UNICA_B200_V_*.  Clusters: heads of K, heads of V, then eight tiles of Q each.
-template <int V_MODE>
-__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
+// V_MODE: UNICA_B200_V_*; HALF, ROPE: the input is float16, Q and K are rotated (template parameters so that the other calls
+// carry none of it).  Clusters: heads of K, heads of V, then eight tiles of Q each.
+template <int V_MODE, bool HALF, bool ROPE>
+__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
     __shared__ CallStats sm;
     __shared__ CallOutliers outliers;
+    const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0}, none{nullptr, 0};
     const int rank = int(blockIdx.x) % CALL_CLUSTER, clusters_k = call.k.x ? call.heads : 0, clusters_v = call.v.x ? call.heads : 0;
     int cluster = int(blockIdx.x) / CALL_CLUSTER;
     if (cluster < clusters_k) {
         const CallOperand& op = call.k;
+        TokenLayout in = op.in;
+        in.half = HALF;
         const int head = cluster;
-        head_stats(op.x, op.in, call.rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, false>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
         for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_int8_tile<KEY_TILE>(op.x, op.in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
-                                     static_cast<float*>(op.scales) + tile, call.rope, sm.scratch);
+            rows_int8_tile<KEY_TILE>(op.x, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
+                                     static_cast<float*>(op.scales) + tile, rope, sm.scratch);
             __syncthreads();
         }
     } else if ((cluster -= clusters_k) < clusters_v) {
         const CallOperand& op = call.v;
+        TokenLayout in = op.in;
+        in.half = HALF;
         const int head = cluster;
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
             for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
-                v_int8_tile<decltype(per_token)::value>(op.x, op.in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes),
+                v_int8_tile<decltype(per_token)::value>(op.x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes),
                                                         scale, call.v_token, sm.v_tile);
                 __syncthreads();
             }
@@ -210,9 +259,9 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         if constexpr (V_MODE == UNICA_B200_V_TOKEN) {
             tiles(std::true_type{}, NoSkip{});
         } else if constexpr (V_MODE == UNICA_B200_V_OUTLIERS) {
-            find_outliers(op.x, op.in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
+            find_outliers(op.x, in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
             const SkipKeys skip{outliers.keys, call.n_outliers};
-            head_stats(op.x, op.in, RopeTable{nullptr, 0}, skip, head, op.n_tokens, rank, sm);
+            head_stats<false, true>(op.x, in, none, skip, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, skip);
             if (rank == 0) {  // the outliers' rows over the channel scales
                 for (int i = threadIdx.x; i < call.n_outliers * HEAD_DIM; i += CALL_THREADS) {
@@ -220,24 +269,31 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
                     const float s = fmaxf(fmaxf(sm.high[c], -sm.low[c]) * (1.0f / 127.0f), 1e-12f);
                     float x = 0.0f;
                     if (key >= 0) {
-                        const __nv_bfloat16* src = op.x + op.in.offset(head, key) + c;
-                        x = op.in.half ? __bfloat162float(__float2bfloat16_rn(__half2float(*reinterpret_cast<const __half*>(src)))) : __bfloat162float(*src);
+                        const __nv_bfloat16* src = op.x + in.offset(head, key) + c;
+                        x = HALF ? __bfloat162float(__float2bfloat16_rn(__half2float(*reinterpret_cast<const __half*>(src)))) : __bfloat162float(*src);
                     }
                     call.outlier_rows[(size_t(head) * call.n_outliers) * HEAD_DIM + i] = __fdiv_rn(x, s);
                     if (c == 0) call.outlier_keys[size_t(head) * call.n_outliers + o] = key;
                 }
             }
         } else {
-            head_stats(op.x, op.in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
+            head_stats<false, true>(op.x, in, none, NoSkip{}, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, NoSkip{});
         }
     } else {
         cluster -= clusters_v;
         const CallOperand& op = call.q;
+        TokenLayout in = op.in;
+        in.half = HALF;
         const int tile = cluster * CALL_CLUSTER + rank, head = tile / op.tiles, t = tile % op.tiles;
-        if (head < call.heads)
-            rows_int8_tile<QUERY_TILE>(op.x, op.in, nullptr, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM),
-                                       static_cast<float*>(op.scales) + tile, call.rope, sm.scratch);
+        if (head < call.heads) {
+            int8_t* codes = reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM);
+            float* scale = static_cast<float*>(op.scales) + tile;
+            if constexpr (ROPE)
+                rows_int8_tile<QUERY_TILE>(op.x, in, nullptr, head, t, op.n_tokens, codes, scale, rope, sm.scratch);
+            else
+                rows_int8_tile_raw<QUERY_TILE>(op.x, in, head, t, op.n_tokens, codes, scale, sm.scratch);
+        }
     }
     cg::this_cluster().sync();  // nobody leaves while another block may still read its shared memory
 }
@@ -246,47 +302,55 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
 __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (1.0f / 2688.0f), 1e-30f); }
 
 // Clusters: heads of K, of V, of Q.
-__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+template <bool HALF, bool ROPE>
+__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
     extern __shared__ __align__(16) uint8_t tile_smem[];  // V4Tile
+    const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0};
     const int rank = int(blockIdx.x) % CALL_CLUSTER;
     const int kind = int(blockIdx.x) / CALL_CLUSTER / call.heads, head = int(blockIdx.x) / CALL_CLUSTER % call.heads;
     if (kind == 0) {
         const CallOperand& op = call.k;
-        head_stats(op.x, op.in, call.rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        TokenLayout in = op.in;
+        in.half = HALF;
+        head_stats<true, true>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
             const float m = sm.mean[threadIdx.x];
             amax = fmaxf(fabsf(sm.high[threadIdx.x] - m), fabsf(sm.low[threadIdx.x] - m));
             if (rank == 0) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = m;
         }
-        const float outer = outer_scale(block_max<CALL_THREADS>(amax, sm.scratch));
-        if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer;
+        const Fp4Outer outer = fp4_outer(outer_scale(block_max<CALL_THREADS>(amax, sm.scratch)));
+        if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
         for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<KEY_TILE, true>(op.x, op.in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
-                                          static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), call.rope);
+            rows_fp4_tile<KEY_TILE, true>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
+                                          static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), rope);
         }
     } else if (kind == 1) {
         const CallOperand& op = call.v;
-        head_stats(op.x, op.in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
+        TokenLayout in = op.in;
+        in.half = HALF;
+        head_stats<false, true>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
         for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            v_fp4_tile(op.x, op.in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32),
+            v_fp4_tile(op.x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32),
                        static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4), op.outer + size_t(head) * HEAD_DIM, *reinterpret_cast<V4Tile*>(tile_smem));
             __syncthreads();
         }
     } else {
         // Q: a mean per group of `smooth` tokens, whole groups per block
         const CallOperand& op = call.q;
+        TokenLayout in = op.in;
+        in.half = HALF;
         const int groups = (op.n_tokens + call.smooth - 1) / call.smooth, per = call.smooth / CALL_BLOCK, blocks = (op.n_tokens + CALL_BLOCK - 1) / CALL_BLOCK;
         float amax = 0.0f;
         for (int g = share(groups, rank); g < share(groups, rank + 1); ++g) {
             float s = 0.0f, lo = INFINITY, hi = -INFINITY;
             const int b1 = min((g + 1) * per, blocks);
             for (int b = g * per; b < b1; ++b) {
-                block_stats(op.x, op.in, call.rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
+                block_stats<true, true>(op.x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
                 if (threadIdx.x < HEAD_DIM)
                     s += sm.part[0][0][threadIdx.x], lo = fminf(lo, sm.part[0][1][threadIdx.x]), hi = fmaxf(hi, sm.part[0][2][threadIdx.x]);
                 __syncthreads();
@@ -303,8 +367,8 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         cg::this_cluster().sync();
         amax = 0.0f;
         for (int r = 0; r < CALL_CLUSTER; ++r) amax = fmaxf(amax, *cg::this_cluster().map_shared_rank(&q_amax, r));
-        const float outer = outer_scale(amax);
-        if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer;
+        const Fp4Outer outer = fp4_outer(outer_scale(amax));
+        if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
         const int t0 = share(op.tiles, rank), t1 = share(op.tiles, rank + 1), g0 = t0 * QUERY_TILE / call.smooth;
         const int touched = t1 > t0 ? min((t1 * QUERY_TILE - 1) / call.smooth, groups - 1) - g0 + 1 : 0;  // groups of this block's tiles (its last ones may lie past the end)
         for (int i = threadIdx.x; i < touched * HEAD_DIM; i += CALL_THREADS)
@@ -312,8 +376,8 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         __syncthreads();
         for (int t = t0; t < t1; ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<QUERY_TILE, false>(op.x, op.in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
-                                             op.codes + tile * (QUERY_TILE * HEAD_DIM / 2), static_cast<uint8_t*>(op.scales) + tile * (QUERY_TILE * 8), call.rope);
+            rows_fp4_tile<QUERY_TILE, false>(op.x, in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
+                                             op.codes + tile * (QUERY_TILE * HEAD_DIM / 2), static_cast<uint8_t*>(op.scales) + tile * (QUERY_TILE * 8), rope);
         }
     }
     cg::this_cluster().sync();
@@ -325,12 +389,16 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
     const long long clusters = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0) + q_tiles;
     if (clusters > (1 << 27)) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: too many heads and tiles");
     const dim3 grid(unsigned(clusters) * CALL_CLUSTER);
-    if (call.v_mode == UNICA_B200_V_TOKEN)
-        quantize_call_int8_kernel<UNICA_B200_V_TOKEN><<<grid, CALL_THREADS, 0, stream>>>(call);
-    else if (call.v_mode == UNICA_B200_V_OUTLIERS)
-        quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS><<<grid, CALL_THREADS, 0, stream>>>(call);
-    else
-        quantize_call_int8_kernel<UNICA_B200_V_CHANNEL><<<grid, CALL_THREADS, 0, stream>>>(call);
+    auto launch = [&](auto half, auto rope) {
+        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
+        auto kernel = call.v_mode == UNICA_B200_V_TOKEN      ? quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE>
+                      : call.v_mode == UNICA_B200_V_OUTLIERS ? quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, HALF, ROPE>
+                                                             : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE>;
+        kernel<<<grid, CALL_THREADS, 0, stream>>>(call);
+    };
+    const bool half = (call.q.x ? call.q : call.k.x ? call.k : call.v).in.half;
+    call.rope.table ? (half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))
+                    : (half ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{}));
     return unica_check_launch("quantize_call_int8");
 }
 
@@ -338,9 +406,11 @@ int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
     constexpr int SMEM = int(sizeof(V4Tile));
     static_assert(SMEM + sizeof(CallStats) + CALL_GROUPS * HEAD_DIM * 4 <= 99 * 1024, "two blocks per SM");
-    if (cudaFuncSetAttribute(quantize_call_fp4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-        return unica_check_launch("quantize_call_fp4 (shared memory size)");
-    quantize_call_fp4_kernel<<<dim3(3u * call.heads * CALL_CLUSTER), CALL_THREADS, SMEM, stream>>>(call);
+    const bool half = call.q.in.half;
+    auto kernel = call.rope.table ? (half ? quantize_call_fp4_kernel<true, true> : quantize_call_fp4_kernel<false, true>)
+                                  : (half ? quantize_call_fp4_kernel<true, false> : quantize_call_fp4_kernel<false, false>);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return unica_check_launch("quantize_call_fp4 (shared memory size)");
+    kernel<<<dim3(3u * call.heads * CALL_CLUSTER), CALL_THREADS, SMEM, stream>>>(call);
     return unica_check_launch("quantize_call_fp4");
 }
 

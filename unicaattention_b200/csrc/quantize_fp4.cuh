@@ -4,7 +4,7 @@
 
 #include <cuda_fp8.h>
 
-#include "common.cuh"
+#include "quantize_int8.cuh"
 
 namespace unica {
 
@@ -35,16 +35,37 @@ __device__ __forceinline__ uint32_t pack_e2m1x8(const float* v) {
     return word;
 }
 
+// An outer scale and its reciprocal.  x / scale is taken without a division, by Markstein's correction step (see
+// quotient_code2 in quantize_int8.cuh): bit for bit the IEEE quotient wherever it decides a code, given that the residual does
+// not underflow (outer scales below 1e-27 take the division) and that the divisor's mantissa is not all ones.
+struct Fp4Outer {
+    float value, inverse;
+    bool divide;
+};
+__device__ __forceinline__ Fp4Outer fp4_outer(float outer) { return Fp4Outer{outer, __frcp_rn(outer), outer < 1e-27f || needs_division(outer)}; }
+__device__ __forceinline__ float2 quotient2(float2 x, float2 inv2, float2 minus_scale2) {
+    const float2 q0 = mul2(x, inv2);
+    return fma2(fma2(q0, minus_scale2, x), inv2, q0);
+}
+
 // One block of 16 values: scale byte and 16 codes (two words).
-__device__ __forceinline__ void quantize_block16(float (&v)[16], float outer, uint32_t& byte, uint2& codes) {
-    float amax = 0.0f;
+__device__ __forceinline__ void quantize_block16(float2 (&v)[8], const Fp4Outer& outer, uint32_t& byte, uint2& codes) {
+    float amax = fmaxf(fabsf(v[0].x), fabsf(v[0].y));
 #pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    byte = to_e4m3(__fdiv_rn(amax * (1.0f / 6.0f), outer));
-    const float scale = from_e4m3(byte) * outer;
+    for (int i = 1; i < 8; ++i) amax = max3(amax, fabsf(v[i].x), fabsf(v[i].y));
+    const float sixth = amax * (1.0f / 6.0f), q0 = sixth * outer.inverse;
+    byte = to_e4m3(outer.divide ? __fdiv_rn(sixth, outer.value) : fmaf(fmaf(-q0, outer.value, sixth), outer.inverse, q0));
+    const float scale = from_e4m3(byte) * outer.value;
+    if (outer.divide || needs_division(scale)) {  // practically never
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = scale > 0.0f ? __fdiv_rn(v[i], scale) : 0.0f;
-    codes = make_uint2(pack_e2m1x8(v), pack_e2m1x8(v + 8));
+        for (int i = 0; i < 8; ++i) v[i] = scale > 0.0f ? make_float2(__fdiv_rn(v[i].x, scale), __fdiv_rn(v[i].y, scale)) : make_float2(0.0f, 0.0f);
+    } else {
+        const float inv = scale > 0.0f ? __frcp_rn(scale) : 0.0f;  // a block whose scale is 0 holds zeros
+        const float2 inv2 = make_float2(inv, inv), minus_scale2 = make_float2(-scale, -scale);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = quotient2(v[i], inv2, minus_scale2);
+    }
+    codes = make_uint2(pack_e2m1x8(&v[0].x), pack_e2m1x8(&v[4].x));
 }
 
 // Q or K minus its mean in NVFP4 along the channels: one tile of ROWS tokens (128: Q, 64: K) by a block of FP4_THREADS.
@@ -53,38 +74,40 @@ __device__ __forceinline__ void quantize_block16(float (&v)[16], float outer, ui
 // codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][32 lanes][4 words]
 // [4] bytes, K [32 lanes][4 words][4] bytes (see the store below).
 template <int ROWS, bool SLOTS, typename MeanOf>
-__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, float head_outer, int head,
+__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
                                               int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
                                               const RopeTable& rope) {
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
         const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;  // block of 16 channels
         const int token = SLOTS ? tile * ROWS + slot_key(row) : tile * ROWS + row;
-        float v[16];
+        float2 v[8];
         if (token < n_tokens) {
             const __nv_bfloat16* src = x + in.offset(head, token) + block * 16;
             const uint4 raw[2] = {load_bf16x8(src, in.half), load_bf16x8(src + 8, in.half)};
-            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw);
             const float* mu = mean_of(token);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 f = __bfloat1622float2(pairs[i]);
-                v[2 * i] = f.x, v[2 * i + 1] = f.y;
-            }
+            unpack8(raw[0], reinterpret_cast<float2(&)[4]>(v[0]));
+            unpack8(raw[1], reinterpret_cast<float2(&)[4]>(v[4]));
             if (rope.table) {  // rotate first: the mean is the rotated x's
                 const __half* f = rope.row(in, head, token);
                 rope8(*reinterpret_cast<float(*)[8]>(v), f, block * 16);
-                rope8(*reinterpret_cast<float(*)[8]>(v + 8), f, block * 16 + 8);
+                rope8(*reinterpret_cast<float(*)[8]>(v + 4), f, block * 16 + 8);
             }
+            if (mu) {
+                const float4* m4 = reinterpret_cast<const float4*>(mu + block * 16);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] -= mu ? mu[block * 16 + i] : 0.0f;
+                for (int i = 0; i < 4; ++i) {
+                    const float4 m = m4[i];
+                    v[2 * i] = sub2(v[2 * i], make_float2(m.x, m.y)), v[2 * i + 1] = sub2(v[2 * i + 1], make_float2(m.z, m.w));
+                }
+            }
         } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+            for (int i = 0; i < 8; ++i) v[i] = make_float2(0.0f, 0.0f);
         }
         uint32_t byte;
         uint2 packed;
-        quantize_block16(v, head_outer, byte, packed);
+        quantize_block16(v, outer, byte, packed);
         *reinterpret_cast<uint2*>(tile_codes + ((block / 2) * ROWS + row) * 16 + (block % 2) * 8) = packed;
         // the word of (K step = block / 4, row): Q [2][32 lanes][4]: word row / 32 of lane row % 32; K [32 lanes][4]: word 2 step +
         // row / 32 of lane row % 32: the 16 bytes tcgen05.cp hands to one tensor-memory lane
@@ -126,12 +149,12 @@ __device__ __forceinline__ void v_fp4_tile(const __nv_bfloat16* __restrict__ v, 
         const int c = item % HEAD_DIM, block = item / HEAD_DIM;  // block of 16 slots
         const float outer = fmaxf(fmaxf(high[c], -low[c]) * (1.0f / 2688.0f), 1e-30f);
         if (t == 0 && block == 0) v_outer[c] = outer;
-        float x[16];
+        float2 x[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = tile[block * 16 + i][c];
+        for (int i = 0; i < 8; ++i) x[i] = make_float2(tile[block * 16 + 2 * i][c], tile[block * 16 + 2 * i + 1][c]);
         uint32_t byte;
         uint2 packed;
-        quantize_block16(x, outer, byte, packed);
+        quantize_block16(x, fp4_outer(outer), byte, packed);
         *reinterpret_cast<uint2*>(tile_codes + ((block / 2) * V4_ROWS + c) * 16 + (block % 2) * 8) = packed;
         tile_sf[((c % 32) * 4 + c / 32) * 4 + block] = uint8_t(byte);  // word c / 32 of lane c % 32
     }

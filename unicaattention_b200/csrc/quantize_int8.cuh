@@ -137,6 +137,50 @@ __device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__
     }
 }
 
+// rows_int8_tile without a mean and without RoPE (Q): the tile stays in registers as it came, two elements to a register, and
+// its maximum is taken on the bfloat16 pairs (exact), which halves the registers and the instructions up to the scale.
+template <int ROWS, int NT = THREADS>
+__device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile, int n_tokens,
+                                                   int8_t* __restrict__ out, float* __restrict__ scale_out, float* scratch,
+                                                   const __nv_bfloat16* staged = nullptr) {
+    constexpr int ITEMS = ROWS * 8 / NT;  // (row, 16-channel chunk) items per thread
+    const int token0 = tile * ROWS;
+    uint4 raw[ITEMS][2];
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        raw[it][0] = raw[it][1] = make_uint4(0, 0, 0, 0);
+        if (token0 + row < n_tokens) {
+            const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : x + in.offset(head, token0 + row) + chunk * 16;
+            raw[it][0] = load_bf16x8(src, in.half), raw[it][1] = load_bf16x8(src + 8, in.half);
+        }
+    }
+    __nv_bfloat162 top = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw[it]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) top = __hmax2(top, __habs2(pairs[i]));
+    }
+    const float2 two = __bfloat1622float2(top);
+    const float scale = fmaxf(block_max<NT>(fmaxf(two.x, two.y), scratch) * (1.0f / 127.0f), 1e-12f);
+    const float inv = __frcp_rn(scale);
+    const float2 inv2 = make_float2(inv, inv), minus_scale2 = make_float2(-scale, -scale);
+    const bool divide = needs_division(scale);  // practically never
+    if (threadIdx.x == 0) *scale_out = scale;
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        float2 t[8];
+        unpack8(raw[it][0], reinterpret_cast<float2(&)[4]>(t[0]));
+        unpack8(raw[it][1], reinterpret_cast<float2(&)[4]>(t[4]));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t[i] = divide ? make_float2(code_by_division(t[i].x, scale), code_by_division(t[i].y, scale)) : quotient_code2(t[i], inv2, minus_scale2);
+        *reinterpret_cast<uint4*>(out + (chunk * ROWS + row) * 16) =
+            make_uint4(low_bytes(t[0], t[1]), low_bytes(t[2], t[3]), low_bytes(t[4], t[5]), low_bytes(t[6], t[7]));
+    }
+}
+
 // V in INT8, one block per tile of 64 keys.  PER_TOKEN false: one scale per channel, max(|low|, |high|) * (1/127) from
 // the channel's min and max over the head (low, high: [heads][128]); true: one scale per key over its channels, and
 // v_token [heads][tiles][2][64] gets log2 s and 1 / s of the tile's keys (zeros past n_tokens).  skip: [heads][n_tokens],
