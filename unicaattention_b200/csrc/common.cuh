@@ -105,8 +105,8 @@ struct RopeTable {
 // Eight channels starting at channel `dim` (a multiple of 8) of one token, rotated: out[2i] = c x[2i] - s x[2i+1],
 // out[2i+1] = s x[2i] + c x[2i+1], each product rounded, then the difference or sum: no fused multiply-add, as the
 // emulator computes it (bench/emulate.py:122-130).
-__device__ __forceinline__ void rope8(float (&v)[8], const __half* token_row, int dim) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(token_row + dim);
+// `raw`: the eight channels' (cos, sin) as the table holds them.
+__device__ __forceinline__ void rope8(float (&v)[8], const uint4& raw) {
     const __half2* cs = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -115,6 +115,10 @@ __device__ __forceinline__ void rope8(float (&v)[8], const __half* token_row, in
         v[2 * j] = __fsub_rn(__fmul_rn(r.x, x0), __fmul_rn(r.y, x1));
         v[2 * j + 1] = __fadd_rn(__fmul_rn(r.y, x0), __fmul_rn(r.x, x1));
     }
+}
+__device__ __forceinline__ void rope8(float (&v)[8], const __half* token_row, int dim) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(token_row + dim);  // one load
+    rope8(v, raw);
 }
 
 // status codes a kernel leaves in its status word (0: fine)

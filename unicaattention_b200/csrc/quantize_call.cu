@@ -6,7 +6,10 @@
 //   1. the blocks of a cluster take the statistics of an eighth of the head's 256-token blocks each,
 //   2. they read one another's partial results through distributed shared memory, all in the same order,
 //   3. and quantize an eighth of the head's tiles each; the tokens come out of L2 now.
-// What bounds it: latency (two dependent trips to memory and a cluster barrier each way).
+// What bounds it: latency (two dependent trips to memory and a cluster barrier each way) for few tokens; at 30 heads x 4128
+// tokens the instructions of the conversions, so the loads of a tile are issued while the one before is worked on, minima
+// and maxima are taken on bfloat16 pairs, and outliers are looked for by all warps (that size on a B200: INT8 88 -> 63 us,
+// with outliers 127 -> 101 us, NVFP4 93 -> 80 us).
 //
 // Sums run in the order of channel_stats_kernel and its finish kernel (quantize.cu), minima and maxima are exact: the
 // operands are bit for bit those of the separate passes.
@@ -33,11 +36,12 @@ struct CallStats {
     float part[CALL_PARTS][3][HEAD_DIM];  // sum, min, max of this block's 256-token blocks
     union {  // one after the other
         float lanes[3][CALL_LANES][HEAD_DIM];                              // the token lanes' sums on their way to one
-        VTileSmem v_tile;                                                  // a tile of V on its way round
+        V4Tile v4_tile[2];
+        VTileSmem v_tile[2];                                               // tiles of V on their way round
         unsigned long long candidates[CALL_TOKENS / CALL_CLUSTER + 1];  // the block's tokens, see find_outliers
     };
     float mean[HEAD_DIM], low[HEAD_DIM], high[HEAD_DIM];
-    float scratch[CALL_THREADS / 32];
+    float scratch[2][CALL_THREADS / 32];  // by turns, so that a tile's maximum does not have to wait for the last one's readers
 };
 // this block's share of `count` things
 __device__ __forceinline__ int share(int count, int rank) { return count * rank / CALL_CLUSTER; }
@@ -48,17 +52,27 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
                                             int n_tokens, CallStats& sm, float (&part)[3][HEAD_DIM]) {
     const int chunk = threadIdx.x % 16, lane = threadIdx.x / 16;
     float2 sum[4], low[4], high[4];
+    // minima and maxima of values that are not rotated are taken on the bfloat16 pairs as they come (exact)
+    const bool packed = !rope.table;
+    __nv_bfloat162 low2[4], high2[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) sum[i] = make_float2(0.0f, 0.0f), low[i] = make_float2(INFINITY, INFINITY), high[i] = make_float2(-INFINITY, -INFINITY);
+    for (int i = 0; i < 4; ++i) {
+        sum[i] = make_float2(0.0f, 0.0f), low[i] = make_float2(INFINITY, INFINITY), high[i] = make_float2(-INFINITY, -INFINITY);
+        low2[i] = __floats2bfloat162_rn(INFINITY, INFINITY), high2[i] = __floats2bfloat162_rn(-INFINITY, -INFINITY);
+    }
     const int first = b * CALL_BLOCK + lane;
     const __nv_bfloat16* src = x + in.offset(head, 0) + chunk * 8;
 #pragma unroll
     for (int part8 = 0; part8 < CALL_BLOCK / CALL_LANES; part8 += 8) {  // eight loads in flight
-        uint4 raw[8];
+        uint4 raw[8], turns[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int token = first + (part8 + j) * CALL_LANES;
-            raw[j] = token < n_tokens ? load_bf16x8(src + token * in.token, in.half) : make_uint4(0, 0, 0, 0);
+            raw[j] = turns[j] = make_uint4(0, 0, 0, 0);
+            if (token < n_tokens) {
+                raw[j] = load_bf16x8(src + token * in.token, in.half);
+                if (rope.table) turns[j] = *reinterpret_cast<const uint4*>(rope.row(in, head, token) + chunk * 8);
+            }
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -66,11 +80,13 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
             if (token >= n_tokens || skip(token)) continue;
             float2 v[4];
             unpack8(raw[j], v);
-            if (rope.table) rope8(*reinterpret_cast<float(*)[8]>(v), rope.row(in, head, token), chunk * 8);
+            if (rope.table) rope8(*reinterpret_cast<float(*)[8]>(v), turns[j]);
+            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 if (SUMS) sum[i] = add2(sum[i], v[i]);
-                if (RANGE) {
+                if (RANGE && packed) low2[i] = __hmin2(low2[i], pairs[i]), high2[i] = __hmax2(high2[i], pairs[i]);
+                if (RANGE && !packed) {
                     low[i] = make_float2(fminf(low[i].x, v[i].x), fminf(low[i].y, v[i].y));
                     high[i] = make_float2(fmaxf(high[i].x, v[i].x), fmaxf(high[i].y, v[i].y));
                 }
@@ -81,6 +97,7 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
     for (int i = 0; i < 4; ++i) {
         if (SUMS) *reinterpret_cast<float2*>(&sm.lanes[0][lane][chunk * 8 + 2 * i]) = sum[i];
         if (RANGE) {
+            if (packed) low[i] = __bfloat1622float2(low2[i]), high[i] = __bfloat1622float2(high2[i]);
             *reinterpret_cast<float2*>(&sm.lanes[1][lane][chunk * 8 + 2 * i]) = low[i];
             *reinterpret_cast<float2*>(&sm.lanes[2][lane][chunk * 8 + 2 * i]) = high[i];
         }
@@ -150,10 +167,13 @@ __device__ __forceinline__ void head_stats(const __nv_bfloat16* __restrict__ x, 
 }
 
 // The n_outliers keys with the largest max |v| of the head, ties to the lower key (what the reference's emulation takes), in
-// every block of the cluster: -1 where the head has fewer keys.
+// every block of the cluster: -1 where the head has fewer keys.  Every warp picks the largest of an eighth of the block's
+// tokens, then one warp per block picks among all blocks' picks.
+constexpr int CALL_WARPS = CALL_THREADS / 32, CALL_PICKS = CALL_WARPS * CALL_OUTLIERS;
 struct CallOutliers {
-    unsigned long long mine[CALL_OUTLIERS];  // this block's candidates: max |v| as bits, then the complement of the key
+    unsigned long long mine[CALL_PICKS];  // this block's picks: max |v| as bits, then the complement of the key; 0: none
     int keys[CALL_OUTLIERS];
+    uint32_t is_outlier[CALL_TOKENS / 32];  // a bit per token of the head
 };
 __device__ __forceinline__ unsigned long long larger(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 __device__ __forceinline__ unsigned long long warp_largest(unsigned long long x) {
@@ -161,49 +181,73 @@ __device__ __forceinline__ unsigned long long warp_largest(unsigned long long x)
     for (int d = 16; d > 0; d /= 2) x = larger(x, __shfl_xor_sync(0xffffffffu, x, d));
     return x;
 }
+// the `count` largest of a warp's values (N per lane), one after the other
+template <int N, typename Take>
+__device__ __forceinline__ void take_largest(unsigned long long (&value)[N], int count, Take take) {
+    for (int o = 0; o < count; ++o) {
+        unsigned long long best = value[0];
+#pragma unroll
+        for (int j = 1; j < N; ++j) best = larger(best, value[j]);
+        best = warp_largest(best);
+        take(o, best);
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (value[j] == best) value[j] = 0;
+    }
+}
 __device__ __forceinline__ void find_outliers(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, int head, int n_tokens, int n_outliers, int rank,
                                               unsigned long long* candidates, CallOutliers& sm) {
     const int t0 = share(n_tokens, rank), count = share(n_tokens, rank + 1) - t0;
     const int chunk = threadIdx.x % 16, lane = threadIdx.x / 16;
-#pragma unroll 4
-    for (int i = lane; i < (count + CALL_LANES - 1) / CALL_LANES * CALL_LANES; i += CALL_LANES) {
-        float amax = 0.0f;
-        if (i < count) {
-            float x[8];
-            load8(x, v + in.offset(head, t0 + i) + chunk * 8, in.half);
+    for (int i = threadIdx.x; i < CALL_TOKENS / 32; i += CALL_THREADS) sm.is_outlier[i] = 0;
+    const __nv_bfloat16* first = v + in.offset(head, t0) + chunk * 8;
+    for (int i0 = 0; i0 < count; i0 += 8 * CALL_LANES) {  // eight loads in flight
+        uint4 raw[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(x[j]));
+        for (int j = 0; j < 8; ++j) {
+            const int i = i0 + j * CALL_LANES + lane;
+            raw[j] = i < count ? load_bf16x8(first + i * in.token, in.half) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int d = 8; d > 0; d /= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-        if (chunk == 0 && i < count) candidates[i] = (static_cast<unsigned long long>(__float_as_uint(amax)) << 32) | (0xffffffffu - unsigned(t0 + i));
+        for (int j = 0; j < 8; ++j) {
+            const int i = i0 + j * CALL_LANES + lane;
+            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
+            const __nv_bfloat162 top = __hmax2(__hmax2(__habs2(pairs[0]), __habs2(pairs[1])), __hmax2(__habs2(pairs[2]), __habs2(pairs[3])));
+            const float2 two = __bfloat1622float2(top);
+            float amax = fmaxf(two.x, two.y);
+#pragma unroll
+            for (int d = 8; d > 0; d /= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+            if (chunk == 0 && i < count) candidates[i] = (static_cast<unsigned long long>(__float_as_uint(amax)) << 32) | (0xffffffffu - unsigned(t0 + i));
+        }
     }
     __syncthreads();
-    if (threadIdx.x < 32) {  // one warp: the largest, n_outliers times
-        for (int o = 0; o < n_outliers; ++o) {
-            unsigned long long best = 0;
-            for (int i = threadIdx.x; i < count; i += 32) best = larger(best, candidates[i]);
-            best = warp_largest(best);
-            if (threadIdx.x == 0) sm.mine[o] = best;
-            for (int i = threadIdx.x; i < count; i += 32)
-                if (candidates[i] == best) candidates[i] = 0;
-            __syncwarp();
+    {
+        unsigned long long value[CALL_TOKENS / CALL_CLUSTER / CALL_THREADS + 1];
+#pragma unroll
+        for (int j = 0; j < CALL_TOKENS / CALL_CLUSTER / CALL_THREADS + 1; ++j) {
+            const int i = j * CALL_THREADS + threadIdx.x;
+            value[j] = i < count ? candidates[i] : 0;
         }
+        take_largest(value, n_outliers, [&](int o, unsigned long long best) {
+            if (threadIdx.x % 32 == 0) sm.mine[threadIdx.x / 32 * CALL_OUTLIERS + o] = best;
+        });
     }
     cg::this_cluster().sync();
     if (threadIdx.x < 32) {
-        unsigned long long mine[2];  // eight blocks' eight candidates, two per lane
+        constexpr int PER_LANE = CALL_CLUSTER * CALL_PICKS / 32;
+        unsigned long long value[PER_LANE];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = threadIdx.x * 2 + j;
-            mine[j] = i % CALL_OUTLIERS < n_outliers ? cg::this_cluster().map_shared_rank(&sm, i / CALL_OUTLIERS)->mine[i % CALL_OUTLIERS] : 0;
+        for (int j = 0; j < PER_LANE; ++j) {  // lanes side by side on one block's picks
+            const int i = j * 32 + threadIdx.x;
+            value[j] = i % CALL_OUTLIERS < n_outliers ? cg::this_cluster().map_shared_rank(&sm, i / CALL_PICKS)->mine[i % CALL_PICKS] : 0;
         }
-        for (int o = 0; o < n_outliers; ++o) {
-            const unsigned long long best = warp_largest(larger(mine[0], mine[1]));
-            if (threadIdx.x == 0) sm.keys[o] = best ? int(0xffffffffu - unsigned(best)) : -1;
-            if (mine[0] == best) mine[0] = 0;
-            if (mine[1] == best) mine[1] = 0;
-        }
+        take_largest(value, n_outliers, [&](int o, unsigned long long best) {
+            if (threadIdx.x == 0) {
+                const int key = best ? int(0xffffffffu - unsigned(best)) : -1;
+                sm.keys[o] = key;
+                if (key >= 0) sm.is_outlier[key / 32] |= 1u << (key % 32);
+            }
+        });
     }
     __syncthreads();
 }
@@ -212,14 +256,22 @@ struct NoSkip {
     __device__ __forceinline__ bool operator()(int) const { return false; }
 };
 struct SkipKeys {
-    const int* keys;
-    int count;
-    __device__ __forceinline__ bool operator()(int token) const {
-        bool found = false;
-        for (int i = 0; i < count; ++i) found |= keys[i] == token;
-        return found;
-    }
+    const uint32_t* is_outlier;
+    __device__ __forceinline__ bool operator()(int token) const { return (is_outlier[token / 32] >> (token % 32)) & 1; }
 };
+
+// Tiles first .. last - 1 in order, each loaded while the one before is worked on.
+template <typename Raw, typename Load, typename Finish>
+__device__ __forceinline__ void each_tile(int first, int last, Load load, Finish finish) {
+    if (first >= last) return;
+    Raw raw, next;
+    load(raw, first);
+    for (int t = first; t < last; ++t) {
+        if (t + 1 < last) load(next, t + 1);
+        finish(raw, t);
+        raw = next;
+    }
+}
 
 // V_MODE: UNICA_B200_V_*; HALF, ROPE: the input is float16, Q and K are rotated (template parameters so that the other calls
 // carry none of it).  Clusters: heads of K, heads of V, then eight tiles of Q each.
@@ -237,12 +289,13 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         const int head = cluster;
         head_stats<true, false>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
-        for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
-            const size_t tile = size_t(head) * op.tiles + t;
-            rows_int8_tile<KEY_TILE>(op.x, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
-                                     static_cast<float*>(op.scales) + tile, rope, sm.scratch);
-            __syncthreads();
-        }
+        each_tile<RowsRaw<KEY_TILE>>(
+            share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { rows_load<KEY_TILE>(raw, op.x, in, head, t, op.n_tokens); },
+            [&](const auto& raw, int t) {
+                const size_t tile = size_t(head) * op.tiles + t;
+                rows_int8_finish<KEY_TILE>(raw, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
+                                           static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
+            });
     } else if ((cluster -= clusters_k) < clusters_v) {
         const CallOperand& op = call.v;
         TokenLayout in = op.in;
@@ -250,17 +303,18 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         const int head = cluster;
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
-            for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
-                v_int8_tile<decltype(per_token)::value>(op.x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes),
-                                                        scale, call.v_token, sm.v_tile);
-                __syncthreads();
-            }
+            each_tile<VRaw>(
+                share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { v_load(raw, op.x, in, skip, head, t, op.n_tokens); },
+                [&](const auto& raw, int t) {
+                    v_int8_finish<decltype(per_token)::value>(raw, sm.low, sm.high, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale,
+                                                              call.v_token, sm.v_tile[t & 1]);
+                });
         };
         if constexpr (V_MODE == UNICA_B200_V_TOKEN) {
             tiles(std::true_type{}, NoSkip{});
         } else if constexpr (V_MODE == UNICA_B200_V_OUTLIERS) {
             find_outliers(op.x, in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
-            const SkipKeys skip{outliers.keys, call.n_outliers};
+            const SkipKeys skip{outliers.is_outlier};
             head_stats<false, true>(op.x, in, none, skip, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, skip);
             if (rank == 0) {  // the outliers' rows over the channel scales
@@ -290,9 +344,9 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
             int8_t* codes = reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM);
             float* scale = static_cast<float*>(op.scales) + tile;
             if constexpr (ROPE)
-                rows_int8_tile<QUERY_TILE>(op.x, in, nullptr, head, t, op.n_tokens, codes, scale, rope, sm.scratch);
+                rows_int8_tile<QUERY_TILE>(op.x, in, nullptr, head, t, op.n_tokens, codes, scale, rope, sm.scratch[0]);
             else
-                rows_int8_tile_raw<QUERY_TILE>(op.x, in, head, t, op.n_tokens, codes, scale, sm.scratch);
+                rows_int8_tile_raw<QUERY_TILE>(op.x, in, head, t, op.n_tokens, codes, scale, sm.scratch[0]);
         }
     }
     cg::this_cluster().sync();  // nobody leaves while another block may still read its shared memory
@@ -301,12 +355,12 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
 // max |x - mean| of the block's values -> the outer scale of all: see nvfp4_outer_rows_kernel
 __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (1.0f / 2688.0f), 1e-30f); }
 
-// Clusters: heads of K, of V, of Q.
+// Clusters: heads of K, of V, of Q.  Rotated inputs keep twice the loads in flight: with three blocks per SM their registers
+// spilled (2 x 16 heads x 777 tokens: 49 us, with two 42 us).
 template <bool HALF, bool ROPE>
-__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
-    extern __shared__ __align__(16) uint8_t tile_smem[];  // V4Tile
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0};
     const int rank = int(blockIdx.x) % CALL_CLUSTER;
     const int kind = int(blockIdx.x) / CALL_CLUSTER / call.heads, head = int(blockIdx.x) / CALL_CLUSTER % call.heads;
@@ -321,9 +375,9 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
             amax = fmaxf(fabsf(sm.high[threadIdx.x] - m), fabsf(sm.low[threadIdx.x] - m));
             if (rank == 0) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = m;
         }
-        const Fp4Outer outer = fp4_outer(outer_scale(block_max<CALL_THREADS>(amax, sm.scratch)));
+        const Fp4Outer outer = fp4_outer(outer_scale(block_max<CALL_THREADS>(amax, sm.scratch[0])));
         if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
-        for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
+        for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {  // (no barrier in a tile: the warps run ahead of one another)
             const size_t tile = size_t(head) * op.tiles + t;
             rows_fp4_tile<KEY_TILE, true>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
                                           static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), rope);
@@ -333,12 +387,13 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         TokenLayout in = op.in;
         in.half = HALF;
         head_stats<false, true>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
-        for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {
-            const size_t tile = size_t(head) * op.tiles + t;
-            v_fp4_tile(op.x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32),
-                       static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4), op.outer + size_t(head) * HEAD_DIM, *reinterpret_cast<V4Tile*>(tile_smem));
-            __syncthreads();
-        }
+        each_tile<VRaw>(
+            share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, op.x, in, head, t, op.n_tokens); },
+            [&](const auto& raw, int t) {
+                const size_t tile = size_t(head) * op.tiles + t;
+                v_fp4_finish(raw, sm.low, sm.high, t, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
+                             op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
+            });
     } else {
         // Q: a mean per group of `smooth` tokens, whole groups per block
         const CallOperand& op = call.q;
@@ -361,7 +416,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
                 __stcg(op.mean + (size_t(head) * groups + g) * HEAD_DIM + threadIdx.x, m);
             }
         }
-        amax = block_max<CALL_THREADS>(amax, sm.scratch);
+        amax = block_max<CALL_THREADS>(amax, sm.scratch[0]);
         if (threadIdx.x == 0) q_amax = amax;
         __threadfence();
         cg::this_cluster().sync();
@@ -404,13 +459,10 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
 
 int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
-    constexpr int SMEM = int(sizeof(V4Tile));
-    static_assert(SMEM + sizeof(CallStats) + CALL_GROUPS * HEAD_DIM * 4 <= 99 * 1024, "two blocks per SM");
     const bool half = call.q.in.half;
     auto kernel = call.rope.table ? (half ? quantize_call_fp4_kernel<true, true> : quantize_call_fp4_kernel<false, true>)
                                   : (half ? quantize_call_fp4_kernel<true, false> : quantize_call_fp4_kernel<false, false>);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return unica_check_launch("quantize_call_fp4 (shared memory size)");
-    kernel<<<dim3(3u * call.heads * CALL_CLUSTER), CALL_THREADS, SMEM, stream>>>(call);
+    kernel<<<dim3(3u * call.heads * CALL_CLUSTER), CALL_THREADS, 0, stream>>>(call);
     return unica_check_launch("quantize_call_fp4");
 }
 

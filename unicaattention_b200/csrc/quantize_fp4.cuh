@@ -73,27 +73,44 @@ __device__ __forceinline__ void quantize_block16(float2 (&v)[8], const Fp4Outer&
 // mean_of(token): the 128 means that go with the token, or null.
 // codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][32 lanes][4 words]
 // [4] bytes, K [32 lanes][4 words][4] bytes (see the store below).
-template <int ROWS, bool SLOTS, typename MeanOf>
-__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
-                                              int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
-                                              const RopeTable& rope) {
+// In two halves, so that a caller with several tiles can have the next one's loads under way while it works on one.
+template <int ROWS, bool SLOTS>
+__device__ __forceinline__ void rows_fp4_load(RowsRaw<ROWS, FP4_THREADS>& raw, const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile,
+                                              int n_tokens) {
+    const __nv_bfloat16* first = x + in.offset(head, tile * ROWS);
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
         const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;  // block of 16 channels
+        const int at = SLOTS ? slot_key(row) : row;
+        raw.piece[it][0] = raw.piece[it][1] = make_uint4(0, 0, 0, 0);
+        if (tile * ROWS + at < n_tokens) {
+            const __nv_bfloat16* src = first + at * in.token + block * 16;
+            raw.piece[it][0] = load_bf16x8(src, in.half), raw.piece[it][1] = load_bf16x8(src + 8, in.half);
+        }
+    }
+}
+template <int ROWS, bool SLOTS, typename MeanOf>
+__device__ __forceinline__ void rows_fp4_finish(const RowsRaw<ROWS, FP4_THREADS>& raw, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
+                                                int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
+                                                const RopeTable& rope) {
+#pragma unroll
+    for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
+        const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;
         const int token = SLOTS ? tile * ROWS + slot_key(row) : tile * ROWS + row;
+        uint4 turns[2];  // the table's row, asked for under no condition: the compiler may then ask for several at once
+        if (rope.table) {
+            const uint4* f = reinterpret_cast<const uint4*>(rope.row(in, head, min(token, n_tokens - 1)) + block * 16);
+            turns[0] = f[0], turns[1] = f[1];
+        }
         float2 v[8];
+        unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(v[0]));
+        unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(v[4]));
         if (token < n_tokens) {
-            const __nv_bfloat16* src = x + in.offset(head, token) + block * 16;
-            const uint4 raw[2] = {load_bf16x8(src, in.half), load_bf16x8(src + 8, in.half)};
-            const float* mu = mean_of(token);
-            unpack8(raw[0], reinterpret_cast<float2(&)[4]>(v[0]));
-            unpack8(raw[1], reinterpret_cast<float2(&)[4]>(v[4]));
             if (rope.table) {  // rotate first: the mean is the rotated x's
-                const __half* f = rope.row(in, head, token);
-                rope8(*reinterpret_cast<float(*)[8]>(v), f, block * 16);
-                rope8(*reinterpret_cast<float(*)[8]>(v + 4), f, block * 16 + 8);
+                rope8(*reinterpret_cast<float(*)[8]>(v), turns[0]);
+                rope8(*reinterpret_cast<float(*)[8]>(v + 4), turns[1]);
             }
-            if (mu) {
+            if (const float* mu = mean_of(token)) {
                 const float4* m4 = reinterpret_cast<const float4*>(mu + block * 16);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -101,9 +118,6 @@ __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ 
                     v[2 * i] = sub2(v[2 * i], make_float2(m.x, m.y)), v[2 * i + 1] = sub2(v[2 * i + 1], make_float2(m.z, m.w));
                 }
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = make_float2(0.0f, 0.0f);
         }
         uint32_t byte;
         uint2 packed;
@@ -115,6 +129,14 @@ __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ 
         tile_sf[word * 4 + block % 4] = uint8_t(byte);
     }
 }
+template <int ROWS, bool SLOTS, typename MeanOf>
+__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
+                                              int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
+                                              const RopeTable& rope) {
+    RowsRaw<ROWS, FP4_THREADS> raw;
+    rows_fp4_load<ROWS, SLOTS>(raw, x, in, head, tile, n_tokens);
+    rows_fp4_finish<ROWS, SLOTS>(raw, in, mean_of, outer, head, tile, n_tokens, tile_codes, tile_sf, rope);
+}
 
 // V in NVFP4 along the keys, per channel: one tile of 64 keys (slot order) by a block of FP4_THREADS.  low/high: the channel's
 // min and max over the head ([128], this head's); v_outer [128] is written with tile 0.  tile: shared memory, free again after
@@ -122,27 +144,22 @@ __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ 
 // codes: the tile's [2 chunks of 32 slots][144 rows][16] bytes, rows 128..143 all ones (code 0x2);
 // sf: [2 blocks][32 lanes][4 words] of 4 bytes: block 0 word c / 32 of lane c % 32 = channel c's four bytes, block 1 word 0 of
 // lanes 0..15 = ones (0x38) for rows 128..143, zeros elsewhere.
-using V4Tile = float[KEY_TILE][HEAD_DIM + 1];
-__device__ __forceinline__ void v_fp4_tile(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, const float* low, const float* high, int head, int t,
-                                           int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf, float* __restrict__ v_outer,
-                                           V4Tile& tile) {  // by slot
-    for (int item = threadIdx.x; item < KEY_TILE * 16; item += FP4_THREADS) {
-        const int slot = item / 16, chunk = item % 16, key = t * KEY_TILE + slot_key(slot);
-        float f[8];
-        if (key < n_tokens) {
-            const uint4 raw = load_bf16x8(v + in.offset(head, key) + chunk * 8, in.half);
-            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
+using V4Tile = __nv_bfloat16[KEY_TILE][HEAD_DIM + 8];  // (rows 16-byte aligned)
+__device__ __forceinline__ void v_fp4_load(VRaw& raw, const __nv_bfloat16* __restrict__ v, const TokenLayout& in, int head, int t, int n_tokens) {
+    const int chunk = threadIdx.x % 16;
+    const __nv_bfloat16* first = v + in.offset(head, t * KEY_TILE) + chunk * 8;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 p = __bfloat1622float2(pairs[i]);
-                f[2 * i] = p.x, f[2 * i + 1] = p.y;
-            }
-        } else {
+    for (int it = 0; it < KEY_TILE * 16 / FP4_THREADS; ++it) {
+        const int key = slot_key(it * (FP4_THREADS / 16) + threadIdx.x / 16);
+        raw.piece[it] = t * KEY_TILE + key < n_tokens ? load_bf16x8(first + key * in.token, in.half) : make_uint4(0, 0, 0, 0);
+    }
+}
+__device__ __forceinline__ void v_fp4_finish(const VRaw& raw, const float* low, const float* high, int t, uint8_t* __restrict__ tile_codes,
+                                             uint8_t* __restrict__ tile_sf, float* __restrict__ v_outer, V4Tile& tile) {  // by slot
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) tile[slot][chunk * 8 + i] = f[i];
+    for (int it = 0; it < KEY_TILE * 16 / FP4_THREADS; ++it) {
+        const int slot = it * (FP4_THREADS / 16) + threadIdx.x / 16, chunk = threadIdx.x % 16;
+        *reinterpret_cast<uint4*>(&tile[slot][chunk * 8]) = raw.piece[it];
     }
     __syncthreads();
     for (int item = threadIdx.x; item < HEAD_DIM * 4; item += FP4_THREADS) {
@@ -151,7 +168,7 @@ __device__ __forceinline__ void v_fp4_tile(const __nv_bfloat16* __restrict__ v, 
         if (t == 0 && block == 0) v_outer[c] = outer;
         float2 x[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = make_float2(tile[block * 16 + 2 * i][c], tile[block * 16 + 2 * i + 1][c]);
+        for (int i = 0; i < 8; ++i) x[i] = make_float2(__bfloat162float(tile[block * 16 + 2 * i][c]), __bfloat162float(tile[block * 16 + 2 * i + 1][c]));
         uint32_t byte;
         uint2 packed;
         quantize_block16(x, fp4_outer(outer), byte, packed);
@@ -164,6 +181,13 @@ __device__ __forceinline__ void v_fp4_tile(const __nv_bfloat16* __restrict__ v, 
     }
     if (threadIdx.x < 128)  // second block: rows 128..143 (ones) are word 0 of lanes 0..15, the rest zeros
         reinterpret_cast<uint32_t*>(tile_sf)[128 + threadIdx.x] = threadIdx.x % 4 == 0 && threadIdx.x / 4 < 16 ? 0x38383838u : 0u;
+}
+__device__ __forceinline__ void v_fp4_tile(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, const float* low, const float* high, int head, int t,
+                                           int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf, float* __restrict__ v_outer,
+                                           V4Tile& tile) {
+    VRaw raw;
+    v_fp4_load(raw, v, in, head, t, n_tokens);
+    v_fp4_finish(raw, low, high, t, tile_codes, tile_sf, v_outer, tile);
 }
 
 }  // namespace unica

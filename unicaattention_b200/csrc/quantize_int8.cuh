@@ -83,36 +83,52 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float2 (&v)[4]) {
 // scratch: NT / 32 floats of shared memory, free again after the next __syncthreads().  NT: the block's threads.
 // staged: the tile's rows already in shared memory as the streaming kernels lay them out (see staged_chunk; then x is not
 // read), or null.
+//
+// In two halves, so that a caller with several tiles can have the next one's loads under way while it works on one.
 template <int ROWS, int NT = THREADS>
-__device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const float* mean, int head,
-                                               int tile, int n_tokens, int8_t* __restrict__ out, float* __restrict__ scale_out,
-                                               const RopeTable& rope, float* scratch, const __nv_bfloat16* staged = nullptr) {
-    constexpr int ITEMS = ROWS * 8 / NT;  // (row, 16-channel chunk) items per thread
+struct RowsRaw {
+    uint4 piece[ROWS * 8 / NT][2];  // (row, 16-channel chunk) items of a thread, as bfloat16; zeros past the last token
+};
+template <int ROWS, int NT = THREADS>
+__device__ __forceinline__ void rows_load(RowsRaw<ROWS, NT>& raw, const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile,
+                                          int n_tokens, const __nv_bfloat16* staged = nullptr) {
+    const __nv_bfloat16* first = staged ? staged : x + in.offset(head, tile * ROWS);
+#pragma unroll
+    for (int it = 0; it < ROWS * 8 / NT; ++it) {
+        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        raw.piece[it][0] = raw.piece[it][1] = make_uint4(0, 0, 0, 0);
+        if (tile * ROWS + row < n_tokens) {
+            const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : first + row * in.token + chunk * 16;
+            raw.piece[it][0] = load_bf16x8(src, in.half), raw.piece[it][1] = load_bf16x8(src + 8, in.half);
+        }
+    }
+}
+template <int ROWS, int NT = THREADS>
+__device__ __forceinline__ void rows_int8_finish(const RowsRaw<ROWS, NT>& raw, const TokenLayout& in, const float* mean, int head, int tile, int n_tokens,
+                                                 int8_t* __restrict__ out, float* __restrict__ scale_out, const RopeTable& rope, float* scratch) {
+    constexpr int ITEMS = ROWS * 8 / NT;
     const int token0 = tile * ROWS;
     float2 v[ITEMS][8];
     float local = 0.0f;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
         const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(v[it][0]));
+        unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(v[it][4]));
         if (token0 + row < n_tokens) {
-            const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : x + in.offset(head, token0 + row) + chunk * 16;
-            float2 a[4], b[4];
-            unpack8(load_bf16x8(src, in.half), a);
-            unpack8(load_bf16x8(src + 8, in.half), b);
             if (rope.table) {  // rotate first, then take the mean (of the rotated x) away
                 const __half* f = rope.row(in, head, token0 + row);
-                rope8(*reinterpret_cast<float(*)[8]>(a), f, chunk * 16);
-                rope8(*reinterpret_cast<float(*)[8]>(b), f, chunk * 16 + 8);
+                rope8(*reinterpret_cast<float(*)[8]>(v[it]), f, chunk * 16);
+                rope8(*reinterpret_cast<float(*)[8]>(v[it] + 4), f, chunk * 16 + 8);
             }
+            if (mean) {
+                const float4* m4 = reinterpret_cast<const float4*>(mean + chunk * 16);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2* m2 = reinterpret_cast<const float2*>(mean + chunk * 16);
-                v[it][i] = mean ? sub2(a[i], m2[i]) : a[i];
-                v[it][4 + i] = mean ? sub2(b[i], m2[4 + i]) : b[i];
+                for (int i = 0; i < 4; ++i) {
+                    const float4 m = m4[i];
+                    v[it][2 * i] = sub2(v[it][2 * i], make_float2(m.x, m.y)), v[it][2 * i + 1] = sub2(v[it][2 * i + 1], make_float2(m.z, m.w));
+                }
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[it][i] = make_float2(0.0f, 0.0f);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) local = max3(local, fabsf(v[it][i].x), fabsf(v[it][i].y));
@@ -136,6 +152,14 @@ __device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__
             make_uint4(low_bytes(t[0], t[1]), low_bytes(t[2], t[3]), low_bytes(t[4], t[5]), low_bytes(t[6], t[7]));
     }
 }
+template <int ROWS, int NT = THREADS>
+__device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const float* mean, int head,
+                                               int tile, int n_tokens, int8_t* __restrict__ out, float* __restrict__ scale_out,
+                                               const RopeTable& rope, float* scratch, const __nv_bfloat16* staged = nullptr) {
+    RowsRaw<ROWS, NT> raw;
+    rows_load<ROWS, NT>(raw, x, in, head, tile, n_tokens, staged);
+    rows_int8_finish<ROWS, NT>(raw, in, mean, head, tile, n_tokens, out, scale_out, rope, scratch);
+}
 
 // rows_int8_tile without a mean and without RoPE (Q): the tile stays in registers as it came, two elements to a register, and
 // its maximum is taken on the bfloat16 pairs (exact), which halves the registers and the instructions up to the scale.
@@ -143,22 +167,13 @@ template <int ROWS, int NT = THREADS>
 __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile, int n_tokens,
                                                    int8_t* __restrict__ out, float* __restrict__ scale_out, float* scratch,
                                                    const __nv_bfloat16* staged = nullptr) {
-    constexpr int ITEMS = ROWS * 8 / NT;  // (row, 16-channel chunk) items per thread
-    const int token0 = tile * ROWS;
-    uint4 raw[ITEMS][2];
-#pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
-        raw[it][0] = raw[it][1] = make_uint4(0, 0, 0, 0);
-        if (token0 + row < n_tokens) {
-            const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : x + in.offset(head, token0 + row) + chunk * 16;
-            raw[it][0] = load_bf16x8(src, in.half), raw[it][1] = load_bf16x8(src + 8, in.half);
-        }
-    }
+    constexpr int ITEMS = ROWS * 8 / NT;
+    RowsRaw<ROWS, NT> raw;
+    rows_load<ROWS, NT>(raw, x, in, head, tile, n_tokens, staged);
     __nv_bfloat162 top = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-        const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw[it]);
+        const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw.piece[it]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) top = __hmax2(top, __habs2(pairs[i]));
     }
@@ -172,8 +187,8 @@ __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restri
     for (int it = 0; it < ITEMS; ++it) {
         const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
         float2 t[8];
-        unpack8(raw[it][0], reinterpret_cast<float2(&)[4]>(t[0]));
-        unpack8(raw[it][1], reinterpret_cast<float2(&)[4]>(t[4]));
+        unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(t[0]));
+        unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(t[4]));
 #pragma unroll
         for (int i = 0; i < 8; ++i) t[i] = divide ? make_float2(code_by_division(t[i].x, scale), code_by_division(t[i].y, scale)) : quotient_code2(t[i], inv2, minus_scale2);
         *reinterpret_cast<uint4*>(out + (chunk * ROWS + row) * 16) =
@@ -195,41 +210,45 @@ struct VTileSmem {
     float key_scale[KEY_TILE], key_inv[KEY_TILE];
 };
 // low, high: this head's [128] (global or shared memory); skip(token): the key is written as zeros; tiles: key tiles per head;
-// v_scale [heads][128] or null (the caller writes it); sm: free again after a __syncthreads().
-template <bool PER_TOKEN, typename Skip>
-__device__ __forceinline__ void v_int8_tile(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, const float* low, const float* high,
-                                            Skip skip, int head, int t, int tiles, int n_tokens,
-                                            int8_t* __restrict__ v8, float* __restrict__ v_scale, float* __restrict__ v_token,
-                                            VTileSmem& sm) {
+// v_scale [heads][128] or null (the caller writes it); sm: free again after a __syncthreads().  In two halves, like the rows.
+struct VRaw {
+    uint4 piece[KEY_TILE * 16 / THREADS];
+};
+template <typename Skip>
+__device__ __forceinline__ void v_load(VRaw& raw, const __nv_bfloat16* __restrict__ v, const TokenLayout& in, Skip skip, int head, int t, int n_tokens) {
+    const int chunk = threadIdx.x % 16;  // 8 channels
+    const __nv_bfloat16* first = v + in.offset(head, t * KEY_TILE) + chunk * 8;
+#pragma unroll
+    for (int it = 0; it < KEY_TILE * 16 / THREADS; ++it) {
+        const int key = it * (THREADS / 16) + threadIdx.x / 16, token = t * KEY_TILE + key;
+        raw.piece[it] = token < n_tokens && !skip(token) ? load_bf16x8(first + key * in.token, in.half) : make_uint4(0, 0, 0, 0);
+    }
+}
+template <bool PER_TOKEN>
+__device__ __forceinline__ void v_int8_finish(const VRaw& raw, const float* low, const float* high, int head, int t, int tiles, int n_tokens,
+                                              int8_t* __restrict__ v8, float* __restrict__ v_scale, float* __restrict__ v_token, VTileSmem& sm) {
     // The tile goes through shared memory as bf16, keys x channels, and comes out transposed: a thread then owns one
     // channel and 16 keys, i.e. one 16-byte row of the operand image, and a warp writes 512 contiguous bytes.
     auto& tile = sm.tile;
-    auto& key_scale = sm.key_scale;
-    auto& key_inv = sm.key_inv;
-    const int token0 = t * KEY_TILE;
-    const int chunk = threadIdx.x % 16;  // 8 channels
+    const int chunk = threadIdx.x % 16;
 #pragma unroll
     for (int it = 0; it < KEY_TILE * 16 / THREADS; ++it) {
         const int key = it * (THREADS / 16) + threadIdx.x / 16;
-        const bool valid = token0 + key < n_tokens;
-        uint4 raw = make_uint4(0, 0, 0, 0);
-        if (valid && !skip(token0 + key))
-            raw = load_bf16x8(v + in.offset(head, token0 + key) + chunk * 8, in.half);
-        *reinterpret_cast<uint4*>(&tile[key][chunk * 8]) = raw;
+        const bool valid = t * KEY_TILE + key < n_tokens;
+        *reinterpret_cast<uint4*>(&tile[key][chunk * 8]) = raw.piece[it];
         if (PER_TOKEN) {  // one scale per key over its channels: the 16 threads of a key share their maxima
-            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
-            float amax = 0.0f;
+            const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw.piece[it]);
+            __nv_bfloat162 top = __habs2(pairs[0]);  // exact in any format
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __bfloat1622float2(pairs[i]);
-                amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-            }
+            for (int i = 1; i < 4; ++i) top = __hmax2(top, __habs2(pairs[i]));
+            const float2 f = __bfloat1622float2(top);
+            float amax = fmaxf(f.x, f.y);
 #pragma unroll
             for (int d = 8; d > 0; d /= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffff, amax, d));
             if (chunk == 0) {
                 const float s = fmaxf(amax * (1.0f / 127.0f), 1e-12f);
-                key_scale[key] = s;
-                key_inv[key] = __frcp_rn(s);
+                sm.key_scale[key] = s;
+                sm.key_inv[key] = __frcp_rn(s);
                 float* tok = v_token + (size_t(head) * tiles + t) * 2 * KEY_TILE;
                 tok[key] = valid ? log2f(s) : 0.0f;
                 tok[KEY_TILE + key] = valid ? __fdiv_rn(1.0f, s) : 0.0f;
@@ -237,7 +256,16 @@ __device__ __forceinline__ void v_int8_tile(const __nv_bfloat16* __restrict__ v,
         }
     }
     __syncthreads();
-    v_int8_emit<PER_TOKEN>(tile, false, key_scale, key_inv, low, high, head, t, tiles, v8, v_scale);
+    v_int8_emit<PER_TOKEN>(tile, false, sm.key_scale, sm.key_inv, low, high, head, t, tiles, v8, v_scale);
+}
+template <bool PER_TOKEN, typename Skip>
+__device__ __forceinline__ void v_int8_tile(const __nv_bfloat16* __restrict__ v, const TokenLayout& in, const float* low, const float* high,
+                                            Skip skip, int head, int t, int tiles, int n_tokens,
+                                            int8_t* __restrict__ v8, float* __restrict__ v_scale, float* __restrict__ v_token,
+                                            VTileSmem& sm) {
+    VRaw raw;
+    v_load(raw, v, in, skip, head, t, n_tokens);
+    v_int8_finish<PER_TOKEN>(raw, low, high, head, t, tiles, n_tokens, v8, v_scale, v_token, sm);
 }
 
 // The second half of v_int8_tile: the tile in shared memory (keys x channels, zeros past the last key; float16 bits if
