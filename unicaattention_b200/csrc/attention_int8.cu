@@ -499,8 +499,6 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
     for (int b = 0; b < min(2, total); ++b) pv_arrive(b);  // the accumulators are free to begin with
     int g = 0, i = 0;
     float2 o[HEAD_DIM / 2], y[2][16];
-#pragma unroll
-    for (int j = 0; j < HEAD_DIM / 2; ++j) o[j] = make_float2(0.0f, 0.0f);
     // The tiles' accumulators come in four pieces of 32 channels through two sets of registers: while one piece is added up
     // the next is on its way, also from one tile to the next if its P.V is complete by then.
     // P.V(g) was issued after the softmax of tile g had delivered its record, so where the accumulator is, the record is too.
@@ -515,31 +513,34 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
     load(0, 0, y[0]);
     float2 record = sm.st[0][row];  // tile maximum, row sum
     float p_sum = V_TOKEN ? float(sm.p_sum[0][row]) : 0.0f;
+    auto next_record = [&](int tile) {
+        record = sm.st[slot<ST_RING>(tile)][row];
+        if (V_TOKEN) p_sum = float(sm.p_sum[slot<ST_RING>(tile)][row]);
+    };
 
     for (int item = blockIdx.x; item < a.items.count; item += gridDim.x, ++i) {
-        float m = -INFINITY, den = 0.0f, bias = 0.0f;  // bias: what V8's bias has added to every sum since it was last taken out
+        // `m` is the exponent the sums are kept at, not the running maximum: out = sum over tiles of 2^(tile max - m) *
+        // acc, the same for the denominator, and the common factor cancels at the end.  The textbook form moves m to
+        // every new maximum and multiplies out and den by 2^(m_old - m_new) each time; here m is the first tile's maximum and
+        // moves only when a tile's is more than 2^REFERENCE_SLACK above it.
+        float m = record.x, beta = 1.0f, den = 0.0f, bias = 0.0f;  // bias: what V8's bias has added to every sum since it was last taken out
+#pragma unroll
+        for (int j = 0; j < HEAD_DIM / 2; ++j) o[j] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
         for (int t = 0; t < k_tiles; ++t, ++g) {
             // Is the next tile's accumulator complete?  Asked now, looked at after the first piece: the answer takes some sixty
-            // cycles.  (All lanes get the same one; the vote says so to the compiler.)
+            // cycles.  (All lanes get the same one; the vote says so to the compiler.)  Its record is read then too, and its
+            // factor is ready before this tile is done.
             const bool more = g + 1 < total, asked = mbar_try(&sm.acc_full[slot<2>(g + 1)], round_parity<2>(g + 1));
-            // `m` is the exponent the sums are kept at, not the running maximum: out = sum over tiles of 2^(tile max - m) *
-            // acc, the same for the denominator, and the common factor cancels at the end.  The textbook form moves m to
-            // every new maximum and multiplies out and den by 2^(m_old - m_new) each time; here m moves only when a tile
-            // maximum is more than 2^REFERENCE_SLACK above it (and at an item's first tile, where the factor is 0).
             if (record.x > m + REFERENCE_SLACK) {
                 const float alpha = ex2(m - record.x);
-                m = record.x;
-                den = alpha == 0.0f ? 0.0f : den * alpha;
-                bias = alpha == 0.0f ? 0.0f : bias * alpha;
+                m = record.x, beta = 1.0f;
+                den *= alpha, bias *= alpha;
 #pragma unroll
-                for (int j = 0; j < HEAD_DIM / 2; ++j) o[j] = alpha == 0.0f ? make_float2(0.0f, 0.0f) : mul2(o[j], make_float2(alpha, alpha));
+                for (int j = 0; j < HEAD_DIM / 2; ++j) o[j] = mul2(o[j], make_float2(alpha, alpha));
             }
             __syncwarp();
-            const float beta = ex2(record.x - m);
             const float2 beta2 = make_float2(beta * BETA_UNIT, beta * BETA_UNIT);
-            den += record.y * beta;
-            bias += (V_TOKEN ? p_sum : record.y) * (beta * (V8_BIAS * SUM_UNIT));
             bool next_there = false;
 #pragma unroll
             for (int piece = 0; piece < 3; ++piece) {
@@ -548,19 +549,23 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
                 load(g, piece + 1, y[(piece + 1) % 2]);
                 flush32(y[piece % 2], o + 16 * piece, beta2);
                 reg_fence16(y[piece % 2]);
-                if (piece == 0) next_there = __all_sync(0xffffffffu, asked && more);
+                if (piece == 0) {
+                    den += record.y * beta;
+                    bias += (V_TOKEN ? p_sum : record.y) * (beta * (V8_BIAS * SUM_UNIT));
+                    next_there = __all_sync(0xffffffffu, asked && more);
+                    if (next_there) {
+                        tc_fence_after();
+                        next_record(g + 1);
+                    }
+                }
             }
             tmem_wait_ld();
             reg_fence16(y[1]);
             tc_fence_before();
             if (g + 2 < total) pv_arrive(g + 2);  // the accumulator has been read: P.V(g + 2) may overwrite it
             if (g + P_RING < total) p_free_arrive(g);
-            if (next_there) {
-                tc_fence_after();
-                load(g + 1, 0, y[0]);
-                record = sm.st[slot<ST_RING>(g + 1)][row];
-                if (V_TOKEN) p_sum = float(sm.p_sum[slot<ST_RING>(g + 1)][row]);
-            }
+            if (next_there) load(g + 1, 0, y[0]);
+            beta = ex2(record.x - m);
             flush32(y[1], o + 48, beta2);
             if (t % BIAS_TILES == BIAS_TILES - 1 || t + 1 == k_tiles) {
                 const float2 bias2 = make_float2(-bias, -bias);
@@ -571,8 +576,8 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
             if (more && !next_there) {
                 ok &= wait_for(g + 1);
                 load(g + 1, 0, y[0]);
-                record = sm.st[slot<ST_RING>(g + 1)][row];
-                if (V_TOKEN) p_sum = float(sm.p_sum[slot<ST_RING>(g + 1)][row]);
+                next_record(g + 1);
+                beta = ex2(record.x - m);
             }
         }
 
