@@ -56,7 +56,7 @@ constexpr int SCORES_WARP = 0, PV_WARP = 1, FLUSH_WARP = 4, SOFTMAX_WARP = 8, AT
 constexpr int LAUNCH_REGISTERS = 128, SOFTMAX_REGISTERS = 120, FLUSH_REGISTERS = 232, SERVICE_REGISTERS = 40;
 static_assert(128 * (2 * SOFTMAX_REGISTERS + FLUSH_REGISTERS + SERVICE_REGISTERS) <= ATT_THREADS * LAUNCH_REGISTERS, "the split must fit the launch");
 constexpr int K_RING = 6;   // K8 tiles in shared memory: tile g + K_RING - S_RING is fetched when S(g) is issued (see scores_warp)
-constexpr int V_RING = 8;   // V8 tiles (and the keys' scales, per token): tile g is fetched when S(g) is issued
+constexpr int V_RING = 8;   // V8 tiles (and the keys' scales, per token): tile g - V_LATER is fetched when S(g) is issued
 constexpr int S_RING = 4;   // score buffers in tensor memory
 constexpr int P_RING = 4;   // P^ images in shared memory
 constexpr int ST_RING = 8;  // (tile maximum, row sum) records on their way from the softmax to the flush threads
@@ -182,14 +182,19 @@ __device__ __forceinline__ void issue_pv(uint32_t d, uint64_t p_desc, uint64_t v
 // S(g), as soon as K8(g) has landed and the softmax of tile g - S_RING has handed the scores buffer back; and all copies, none
 // of which has to wait for anything:
 //   K8(g + K_RING - S_RING)  (from g = S_RING on) takes the slot of K8(g - S_RING), whose scores have been read
-//   V8(g)                    takes the slot of V8(g - V_RING): the softmax of tile g - S_RING began after the flush of tile
-//                            g - S_RING - P_RING had seen its P.V complete (p_free_sync)
+//   V8(g - V_LATER)          takes the slot of V8(g - V_LATER - V_RING): the softmax of tile g - S_RING, which has just handed
+//                            its buffer back, began after the flush of tile g - S_RING - P_RING had seen its P.V complete
+//                            (p_free_sync).  Why later: this warp is busy for most of a tile's time, and P.V(g) is tiles away
+//                            (copied with S(g), between its instructions and the copy of K8, 37 heads x 8192 tokens took 1.074
+//                            ms per channel and 1.352 per token; so 1.066 and 1.329).  Why before the waits below: the flush
+//                            leaves an item once the first P.V of the next is complete, so with k_tiles key tiles per head
+//                            what frees Q8's slot for the item that starts with tile g is P.V(g - k_tiles).
 //   Q8 of the item after the next, when V8's argument says that the flush has left the item before (Q_AHEAD tiles into the
 //                            next; with fewer key tiles per head than that, when it is needed)
 // The whole warp runs the loop and one elected lane issues.  A wait that gave up changes nothing here: instructions on
 // whatever lies in the buffers do no harm (the result is not stored), and every hand-over still finds its receiver.
-static_assert(V_RING == S_RING + P_RING, "see above");
-constexpr int Q_AHEAD = V_RING;
+constexpr int V_LATER = 2, Q_AHEAD = V_RING + V_LATER;
+static_assert(V_RING >= S_RING + P_RING, "see above");
 template <bool V_TOKEN>
 __device__ __forceinline__ void scores_warp(AttSmem& sm, const AttArgs& a, int k_tiles, uint32_t tmem) {
     const uint64_t q_desc0 = smem_desc(smem_u32(sm.q[0]), QUERY_TILE * 16, 128), k_desc0 = smem_desc(smem_u32(sm.k[0]), KEY_TILE * 16, 128);
@@ -219,40 +224,51 @@ __device__ __forceinline__ void scores_warp(AttSmem& sm, const AttArgs& a, int k
     copy_q(0);
     for (int i = 0; i < K_RING; ++i) copy_k();
     if (n_items > 1) copy_q(1);
-    int n = 0, t = 0, slot_k = 0, parity_k = 0;
+    // V8's next tile
+    const int v_later = k_tiles > 1 ? V_LATER : 1;
+    int nv = 0, tv = 0, v_tile = 0;
     size_t tile = size_t(head_of(0)) * k_tiles;
+    auto copy_v = [&]() {
+        const int slot_v = slot<V_RING>(v_tile++);
+        if (V_TOKEN) {
+            if (elect_one()) {
+                mbar_expect_tx(&sm.v_full[slot_v], V_BYTES + TOK_BYTES);
+                bulk_load(sm.v[slot_v], a.v8 + tile * V_BYTES, V_BYTES, &sm.v_full[slot_v]);
+                bulk_load(sm.tok[slot_v], a.v_token + tile * (2 * KEY_TILE), TOK_BYTES, &sm.v_full[slot_v]);
+            }
+            __syncwarp();
+        } else {
+            copy_elected(sm.v[slot_v], a.v8 + tile * V_BYTES, V_BYTES, &sm.v_full[slot_v]);
+        }
+        ++tile;
+        if (++tv == k_tiles) tv = 0, tile = size_t(head_of(++nv)) * k_tiles;
+    };
+    int n = 0, t = 0, slot_k = 0, parity_k = 0;
 #pragma unroll 1
     for (int g = 0; g < total; ++g) {
+        s_free_sync(g);
+        if (g >= v_later) copy_v();
         if (t == 0) {
             if (n >= 2 && k_tiles <= Q_AHEAD) copy_q(n);
             mbar_wait_line(&sm.q_full[slot<2>(n)], round_parity<2>(n), &sm.abort_flag, a.status, STATUS_WAIT_TILE);
         }
         mbar_wait_line(&sm.k_full[slot_k], parity_k, &sm.abort_flag, a.status, STATUS_WAIT_TILE);
-        s_free_sync(g);
+        __syncwarp();
         tc_fence_after();
         issue_scores(tmem + COL_S + slot<S_RING>(g) * KEY_TILE, desc_at(q_desc0, slot<2>(n) * (Q_BYTES / 16)), desc_at(k_desc0, slot_k * (K_BYTES / 16)),
                      &sm.s_full[slot<S_RING>(g)]);
         if (++slot_k == K_RING) slot_k = 0, parity_k ^= 1;
-        if (V_TOKEN) {
-            if (elect_one()) {
-                mbar_expect_tx(&sm.v_full[slot<V_RING>(g)], V_BYTES + TOK_BYTES);
-                bulk_load(sm.v[slot<V_RING>(g)], a.v8 + tile * V_BYTES, V_BYTES, &sm.v_full[slot<V_RING>(g)]);
-                bulk_load(sm.tok[slot<V_RING>(g)], a.v_token + tile * (2 * KEY_TILE), TOK_BYTES, &sm.v_full[slot<V_RING>(g)]);
-            }
-            __syncwarp();
-        } else {
-            copy_elected(sm.v[slot<V_RING>(g)], a.v8 + tile * V_BYTES, V_BYTES, &sm.v_full[slot<V_RING>(g)]);
-        }
         if (g >= S_RING) copy_k();
-        ++tile;
         if (k_tiles > Q_AHEAD && t == Q_AHEAD && n >= 1 && n + 1 < n_items) copy_q(n + 1);
         if (++t == k_tiles) {
             commit_elected(&sm.q_free[slot<2>(n)]);
             t = 0, ++n;
-            tile = size_t(head_of(n)) * k_tiles;
         }
     }
-    for (int b = 0; b < S_RING; ++b) s_free_sync(b);  // every buffer has been handed back once more than it was used
+    for (int b = 0; b < S_RING; ++b) {
+        s_free_sync(total + b);  // every buffer has been handed back once more than it was used
+        if (b < v_later && total + b >= v_later) copy_v();
+    }
     commit_elected(&sm.drain[0]);  // whatever was issued must finish before tensor memory is freed
     mbar_wait_line(&sm.drain[0], 0, &sm.never, nullptr, 0);
     // After a wait that gave up, copies may still be in flight: the block's shared memory must not go away under them.
