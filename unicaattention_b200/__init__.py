@@ -169,15 +169,15 @@ def block_stats(x: torch.Tensor, rope: torch.Tensor | None = None) -> torch.Tens
 
 def wave_layout(heads: int, n_queries: int, n_keys: int, v_token: int, device) -> dict:
     """The reference picks between a 4-warp and an 8-warp block per call to fill its last wave (unica/__init__.py:281-285).
-    Here every kernel has one block shape (accurate: one tile of 128 queries per block of 16 warps, one block per SM;
-    fast: two query tiles per block of 12 warps), so there is nothing to pick: always {}.  What the last wave costs is
-    what wave_plan() reports."""
+    Here every kernel has one block shape, persistent and one per SM, each taking tiles in turn (accurate: 128 queries, 16
+    warps; fast: two such tiles, 20 warps), so there is nothing to pick: always {}.  What the last round costs is what
+    wave_plan() reports."""
     return {}
 
 
 def wave_plan(heads: int, n_queries: int, kernel: str = DEFAULT_KERNEL, device=None) -> dict:
-    """How a call's blocks fall on the SMs: blocks (all of equal length: every query tile meets every key), blocks per wave
-    (one per SM), waves, and the share of the SM time of those waves that does work.  batch * heads for `heads`."""
+    """How a call's items (query tiles, or pairs of them) fall on the SMs' persistent blocks: blocks (items, all of equal
+    length: every query tile meets every key), blocks per wave (one per SM), waves, and the share of the SM time of those waves that does work.  batch * heads for `heads`."""
     rows = 256 if kernel == "attention_fp4" else 128
     blocks = heads * math.ceil(n_queries / rows)
     per_wave = sm_count(torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device))
