@@ -42,6 +42,7 @@ STATS_TOKENS = 256
 ROPE_PAIRS = HEAD_DIM // 2
 MAX_OUTLIERS = 8  # outlier keys per head the accurate kernel adds back
 LOG2E = 1.4426950408889634
+SCALE_LOG2 = HEAD_DIM**-0.5 * LOG2E
 
 # The two production modes, under the reference's kernel names (unica/__init__.py:34-40, 88-89).
 KERNELS = ("attention_int8pv_tma", "attention_fp4")
@@ -84,7 +85,7 @@ def readable(x: torch.Tensor) -> torch.Tensor:
     """x itself if the kernels can read it in place (contiguous last dimension, 16-byte aligned tokens), else a
     contiguous copy (unica/__init__.py:103-108)."""
     batch, head, token, channel = x.stride()
-    if channel == 1 and not (batch | head | token) % 8 and not x.data_ptr() % 16:
+    if channel == 1 and not (batch | head | token) & 7 and not x.data_ptr() & 15:
         return x
     in_place = channel == 1 and x.data_ptr() % 16 == 0 and all(x.stride(i) % 8 == 0 or x.shape[i] == 1 for i in range(3))
     return x if in_place else x.contiguous()
@@ -465,17 +466,18 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
             raise ValueError("out must be a tensor of q's shape and dtype on q's device, 16-byte aligned rows with contiguous channels")
     elif peer_out:
         raise ValueError("peer_out needs out")
-    if not (q.dtype == k.dtype == v.dtype and q.dtype in (torch.bfloat16, torch.float16)):
+    dtype, shape, k_shape = q.dtype, q.shape, k.shape  # (asked for once: a tensor's attribute costs a tenth of a microsecond)
+    if not (dtype is k.dtype is v.dtype and (dtype is torch.bfloat16 or dtype is torch.float16)):
         raise TypeError(f"q, k, v must all be bfloat16 or all float16, got {q.dtype}, {k.dtype}, {v.dtype}")
     if not (q.is_cuda and k.is_cuda and v.is_cuda):
         raise ValueError("q, k, v must be on the GPU")
-    if q.dim() != 4 or q.shape[-1] != HEAD_DIM:
+    if len(shape) != 4 or shape[3] != HEAD_DIM:
         raise ValueError(f"q must be [batch, heads, tokens, {HEAD_DIM}], got {tuple(q.shape)}")
-    if k.shape != v.shape or k.shape[:2] != q.shape[:2] or k.shape[-1] != HEAD_DIM:
+    batch, heads, n_queries, _ = shape
+    if k_shape != v.shape or len(k_shape) != 4 or k_shape[0] != batch or k_shape[1] != heads or k_shape[3] != HEAD_DIM:
         raise ValueError(f"k and v must be [batch, heads, n_keys, {HEAD_DIM}] like q, "
                          f"got q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
-    batch, heads, n_queries, _ = q.shape
-    n_keys = k.shape[2]
+    n_keys = k_shape[2]
     if n_keys == 0:
         raise ValueError("k and v must hold at least one token")
     if rope is not None:
@@ -540,19 +542,20 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
     table, table_stride = (0, 0) if rope is None else rope_args(rope, q)
     if rope is not None:
         table = table.value
-    half = int(q.dtype == torch.float16)
-    layouts = (*q.stride()[:3], heads, half, *k.stride()[:3], heads, half, *v.stride()[:3], heads, half, *out.stride()[:3], heads, half)
+    half, device = int(q.dtype is torch.float16), q.device
+    qs, ks, vs, os_ = q.stride(), k.stride(), v.stride(), out.stride()
+    layouts = (qs[0], qs[1], qs[2], heads, half, ks[0], ks[1], ks[2], heads, half, vs[0], vs[1], vs[2], heads, half, os_[0], os_[1], os_[2], heads, half)
     sizes = (batch * heads, n_queries, n_keys, int(fast), v_mode, outliers, smooth if fast else 0)
-    where = (table, table_stride, 0 if peers is None else ctypes.addressof(peers), status_word(q.device).data_ptr(),
-             torch.cuda.current_stream().cuda_stream)
-    scale = HEAD_DIM**-0.5 * LOG2E
+    where = (table, table_stride, 0 if peers is None else ctypes.addressof(peers), status_word(device).data_ptr(),
+             torch._C._cuda_getCurrentRawStream(device.index))
+    scale = SCALE_LOG2
     key = (*sizes, rope is None)
     size = _WORKSPACE_BYTES.get(key)
     if size is None:
         if len(_WORKSPACE_BYTES) > 4096:
             _WORKSPACE_BYTES.clear()
         size = _WORKSPACE_BYTES[key] = lib.attention_workspace(lib.pack_call(0, 0, 0, 0, 0, 0, *where, *layouts, *sizes, 0, scale))
-    workspace = torch.empty(size, dtype=torch.uint8, device=q.device)
+    workspace = torch.empty(size, dtype=torch.uint8, device=device)
     lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
                                      n_peers, scale))
     return True
