@@ -544,6 +544,7 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+    wait_for_previous_kernel();
 
     if (warp >= F4_SOFTMAX_WARP) {
         set_registers<F4_SOFTMAX_REGISTERS, F4_LAUNCH_REGISTERS>();
@@ -575,7 +576,7 @@ using namespace unica;
 int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4, const void* sfv,
                          const float* qk_outer, const float* k_outer, const float* v_outer, const float* bias, int q_blocks, int smooth_q, void* out,
                          void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads, int n_queries, int n_keys,
-                         float scale_log2, uint32_t* p_words, int* status, void* stream) {
+                         float scale_log2, uint32_t* p_words, int* status, void* stream, bool overlapped) {
     if (!q4 || !sfq || !k4 || !sfk || !v4 || !sfv || !qk_outer || !v_outer || !out) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: null pointer");
     if (heads <= 0 || heads > 65535 || n_queries <= 0 || n_keys <= 0)
         return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: heads must be in 1..65535, n_queries and n_keys positive");
@@ -612,7 +613,7 @@ int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, c
             if (cudaDeviceGetAttribute(&blocks, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
             if (device < MAX_DEVICES) blocks_of[instance][device].store(blocks, std::memory_order_release);
         }
-        kernel<<<args.items.count < blocks ? args.items.count : blocks, F4_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(args);
+        launch_after(kernel, dim3(args.items.count < blocks ? args.items.count : blocks), F4_THREADS, smem, static_cast<cudaStream_t>(stream), overlapped, args);
         return unica_check_launch("attention_fp4");
     };
     return p_words ? launch(attention_fp4_kernel<true>, 1) : launch(attention_fp4_kernel<false>, 0);

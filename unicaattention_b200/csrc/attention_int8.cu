@@ -649,6 +649,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_int8_kernel(const __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+    wait_for_previous_kernel();
 
     if (warp >= FLUSH_WARP && warp < SOFTMAX_WARP) {
         set_registers<FLUSH_REGISTERS, LAUNCH_REGISTERS>();
@@ -735,7 +736,7 @@ using namespace unica;
 int unica_attention_int8(const int8_t* q8, const float* q_scale, const int8_t* k8, const float* k_scale, const int8_t* v8,
                           const float* v_scale, const float* v_token, int v_mode, const int* outlier_keys, const float* outlier_rows,
                           int n_outliers, void* out, void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads,
-                          int n_queries, int n_keys, float scale_log2, int* status, void* stream) {
+                          int n_queries, int n_keys, float scale_log2, int* status, void* stream, bool overlapped) {
     if (!q8 || !q_scale || !k8 || !k_scale || !v8 || !v_scale || !out) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_int8: null pointer");
     if (heads <= 0 || heads > 65535 || n_queries <= 0 || n_keys <= 0)
         return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_int8: heads must be in 1..65535, n_queries and n_keys positive");
@@ -777,7 +778,7 @@ int unica_attention_int8(const int8_t* q8, const float* q_scale, const int8_t* k
             if (cudaDeviceGetAttribute(&blocks, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("attention_int8 (device)");
             if (device < MAX_DEVICES) blocks_of[instance][device].store(blocks, std::memory_order_release);
         }
-        kernel<<<args.items.count < blocks ? args.items.count : blocks, ATT_THREADS, smem, s>>>(args);
+        launch_after(kernel, dim3(args.items.count < blocks ? args.items.count : blocks), ATT_THREADS, smem, s, overlapped, args);
         return unica_check_launch("attention_int8");
     };
     return v_mode == UNICA_B200_V_TOKEN      ? launch(attention_int8_kernel<true, false>, 1)

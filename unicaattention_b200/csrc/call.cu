@@ -123,7 +123,7 @@ int call_accurate(const unica_b200_call& c, const Plan& p, int* launches) {
     }
     ++*launches;
     return unica_attention_int8(p.q8, p.q_scale, p.k8, p.k_scale, p.v8, p.v_scale, p.v_token, c.v_mode, p.outlier_keys, p.outlier_rows, c.n_outliers, c.out, c.peer_out,
-                                c.n_peers, c.out_layout, c.heads, c.n_queries, c.n_keys, c.scale_log2, c.status, c.stream);
+                                c.n_peers, c.out_layout, c.heads, c.n_queries, c.n_keys, c.scale_log2, c.status, c.stream, true);
 }
 
 int call_fast(const unica_b200_call& c, const Plan& p, int* launches) {
@@ -163,15 +163,12 @@ int call_fast(const unica_b200_call& c, const Plan& p, int* launches) {
         *launches += 3;
     }
     if (p.bias) {
-        if (int e = c.rope ? unica_b200_smooth_bias_rope(c.k, c.k_layout, p.k_mean, p.q_mean, c.rope, c.rope_batch_stride, c.heads, p.groups, c.n_keys, c.scale_log2, p.bias,
-                                                         c.status, c.stream)
-                           : unica_b200_smooth_bias(c.k, c.k_layout, p.k_mean, p.q_mean, c.heads, p.groups, c.n_keys, c.scale_log2, p.bias, c.status, c.stream))
-            return e;
+        if (int e = unica_smooth_bias(c.k, c.k_layout, p.k_mean, p.q_mean, rope, c.heads, p.groups, c.n_keys, c.scale_log2, p.bias, c.status, c.stream, true)) return e;
         ++*launches;
     }
     ++*launches;
     return unica_attention_fp4(p.q4, p.q_sf, p.k4, p.k_sf, p.v4, p.v_sf, p.q_outer, p.k_outer, p.v_outer, p.bias, p.bias ? p.groups : 0, c.smooth_q, c.out, c.peer_out, c.n_peers,
-                               c.out_layout, c.heads, c.n_queries, c.n_keys, c.scale_log2, nullptr, c.status, c.stream);
+                               c.out_layout, c.heads, c.n_queries, c.n_keys, c.scale_log2, nullptr, c.status, c.stream, true);
 }
 
 }  // namespace

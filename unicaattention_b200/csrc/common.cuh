@@ -150,6 +150,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, int bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// A kernel launched to overlap the one before it in the stream (launch_after in capi.h) waits here until that one is complete
+// and its results are visible; launched in the usual way it does not wait.  The kernel before says when the next one's
+// blocks may be set up, in whatever room its own leave: all of them have then started, so none can be kept out.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // Non-blocking: has the phase of parity `parity` completed?
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, int parity) {
     uint32_t done;

@@ -277,6 +277,7 @@ __device__ __forceinline__ void each_tile(int first, int last, Load load, Finish
 // carry none of it).  Clusters: heads of K, heads of V, then eight tiles of Q each.
 template <int V_MODE, bool HALF, bool ROPE>
 __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
+    let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ CallOutliers outliers;
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0}, none{nullptr, 0};
@@ -359,6 +360,7 @@ __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (
 // spilled (2 x 16 heads x 777 tokens: 49 us, with two 42 us).
 template <bool HALF, bool ROPE>
 __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+    let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0};

@@ -9,6 +9,8 @@
 // contraction index in the low nibble), and the scale bytes in the order the attention kernel copies them into tensor
 // memory.  Keys inside a 64-key tile are stored in the reference's slot order (bench/emulate.py:116-119): the 16-key
 // scale blocks of P and V are defined on that order, so it is part of the numerics.
+#include <atomic>
+
 #include "capi.h"
 #include "quantize_fp4.cuh"
 
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
     const int head = blockIdx.y, b0 = blockIdx.z * BIAS_BLOCKS, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int k_tiles = (n_keys + KEY_TILE - 1) / KEY_TILE, pairs = (k_tiles + 1) / 2;
     volatile int* abort_flag = &sm.abort_flag;
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         mbar_init(&sm.done[0], 1);
@@ -115,6 +118,7 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(&sm.tmem_base, 2 * BIAS_BLOCKS);
+    wait_for_previous_kernel();
     // the means of this pass's query blocks, rows past the last block zero
     for (int item = threadIdx.x; item < BIAS_BLOCKS * (HEAD_DIM / 4); item += BIAS_THREADS) {
         const int r = item % BIAS_BLOCKS, c4 = item / BIAS_BLOCKS;
@@ -322,37 +326,43 @@ extern "C" int unica_b200_quantize_v_fp4(const void* v, unica_token_layout layou
     return unica_check_launch("quantize_v_fp4");
 }
 
-static int smooth_bias(const void* k, unica_token_layout layout, const float* k_mean, const float* q_mean, RopeTable rope, int heads,
-                       int q_blocks, int n_keys, float scale_log2, float* bias, int* status, void* stream) {
+int unica_smooth_bias(const void* k, unica_token_layout layout, const float* k_mean, const float* q_mean, RopeTable rope, int heads, int q_blocks,
+                      int n_keys, float scale_log2, float* bias, int* status, void* stream, bool overlapped) {
     if (!k || !k_mean || !q_mean || !bias || !status) return unica_fail(UNICA_B200_ERR_ARGUMENT, "smooth_bias: null pointer");
     if (heads <= 0 || q_blocks <= 0 || n_keys <= 0) return unica_fail(UNICA_B200_ERR_ARGUMENT, "smooth_bias: heads, q_blocks and n_keys must be positive");
     if (int e = unica_check_device()) return e;
     const int tiles = (n_keys + KEY_TILE - 1) / KEY_TILE, pairs = (tiles + 1) / 2, passes = (q_blocks + BIAS_BLOCKS - 1) / BIAS_BLOCKS;
     if (heads > 65535 || passes > 65535) return unica_fail(UNICA_B200_ERR_ARGUMENT, "smooth_bias: more than 65535 heads or passes of 64 query blocks");
     constexpr int SMEM = int(sizeof(BiasSmem)) + 128;
-    if (cudaFuncSetAttribute(smooth_bias_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-        return unica_check_launch("smooth_bias (shared memory size)");
     // a block per SM (its images take most of the shared memory); at most four full waves of blocks, each walking over
     // its strip of key-tile pairs with the query blocks' images built once
-    int device = 0, sms = 148;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-        return unica_check_launch("smooth_bias (device)");
+    constexpr int MAX_DEVICES = 64;
+    static std::atomic<int> sms_of[MAX_DEVICES];  // set up once per device; 0: not yet
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return unica_check_launch("smooth_bias (device)");
+    int sms = device < MAX_DEVICES ? sms_of[device].load(std::memory_order_acquire) : 0;
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+            cudaFuncSetAttribute(smooth_bias_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+            return unica_check_launch("smooth_bias (device, shared memory size)");
+        if (device < MAX_DEVICES) sms_of[device].store(sms, std::memory_order_release);
+    }
     const long long others = (long long)heads * passes;
     const int strips = int(std::min<long long>(pairs, std::max<long long>(1, 4LL * sms / others)));
-    smooth_bias_kernel<<<dim3(strips, heads, passes), BIAS_THREADS, SMEM, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(k), to_layout(layout), k_mean, q_mean, q_blocks, n_keys, scale_log2, bias, rope, status);
+    launch_after(smooth_bias_kernel, dim3(strips, heads, passes), BIAS_THREADS, SMEM, static_cast<cudaStream_t>(stream), overlapped,
+                 static_cast<const __nv_bfloat16*>(k), to_layout(layout), k_mean, q_mean, q_blocks, n_keys, scale_log2, bias, rope, status);
     return unica_check_launch("smooth_bias");
 }
 
 extern "C" int unica_b200_smooth_bias(const void* k, unica_token_layout layout, const float* k_mean, const float* q_mean,
                                       int heads, int q_blocks, int n_keys, float scale_log2, float* bias, int* status, void* stream) {
-    return smooth_bias(k, layout, k_mean, q_mean, RopeTable{nullptr, 0}, heads, q_blocks, n_keys, scale_log2, bias, status, stream);
+    return unica_smooth_bias(k, layout, k_mean, q_mean, RopeTable{nullptr, 0}, heads, q_blocks, n_keys, scale_log2, bias, status, stream);
 }
 
 extern "C" int unica_b200_smooth_bias_rope(const void* k, unica_token_layout layout, const float* k_mean, const float* q_mean,
                                            const void* rope, long long rope_batch_stride, int heads, int q_blocks, int n_keys,
                                            float scale_log2, float* bias, int* status, void* stream) {
     if (!rope) return unica_fail(UNICA_B200_ERR_ARGUMENT, "smooth_bias_rope: null table");
-    return smooth_bias(k, layout, k_mean, q_mean, RopeTable{static_cast<const __half*>(rope), rope_batch_stride}, heads, q_blocks, n_keys,
+    return unica_smooth_bias(k, layout, k_mean, q_mean, RopeTable{static_cast<const __half*>(rope), rope_batch_stride}, heads, q_blocks, n_keys,
                        scale_log2, bias, status, stream);
 }
