@@ -104,6 +104,37 @@ def test_smooth_bias_is_exact_to_float():
     assert bool(torch.isneginf(bias[..., ~valid]).all())  # slots past the last key
 
 
+@pytest.mark.parametrize("rotated", [False, True])
+@pytest.mark.parametrize("blocks,n_keys", [(1, 1), (31, 129), (32, 64), (33, 63)])
+def test_smooth_bias_around_the_line_between_its_kernels(blocks, n_keys, rotated):
+    import unicaattention_b200 as unica
+
+    g = torch.Generator().manual_seed(blocks)
+    q_mean = torch.randn((1, 3, blocks, 128), generator=g).cuda()
+    k = (torch.randn((1, 3, n_keys, 128), generator=g) + 0.5).half().cuda()
+    angle = torch.rand((1, n_keys, 64), generator=g) * 6
+    cos, sin = angle.cos().half().float().cuda(), angle.sin().half().float().cuda()  # the kernels keep them in float16
+    table = torch.stack([torch.stack([cos, -sin], -1), torch.stack([sin, cos], -1)], -2)[:, :, None].contiguous() if rotated else None
+    k_mean = torch.randn((1, 3, 128), generator=g).cuda()
+    bias = unica.smooth_bias(k, k_mean, q_mean, **({"rope": table} if rotated else {}))
+    unica.check_status()
+    x = k.bfloat16().double()
+    if rotated:
+        cos, sin = cos.double()[:, None], sin.double()[:, None]
+        even, odd = x[..., 0::2], x[..., 1::2]
+        x = torch.stack([cos * even - sin * odd, sin * even + cos * odd], -1).flatten(-2)
+    centred = x - k_mean.double()[..., None, :]
+    expected = (q_mean.double() @ centred.transpose(-1, -2)) * (128**-0.5 * 1.4426950408889634)
+    slot_key = torch.tensor(unica.fp4.SLOT_KEY, device="cuda")
+    tiles = (n_keys + 63) // 64
+    order = (torch.arange(tiles, device="cuda")[:, None] * 64 + slot_key).flatten()
+    valid = order < n_keys
+    got, want = bias[..., valid].double(), expected[..., order[valid]]
+    bound = (q_mean.abs().double() @ (x.abs() + k_mean.abs().double()[..., None, :]).transpose(-1, -2))[..., order[valid]] * 2.0**-20 + 1e-6
+    assert ((got - want).abs() <= bound).all(), ((got - want).abs() / bound).max()
+    assert bool(torch.isneginf(bias[..., ~valid]).all())
+
+
 def test_smooth_bias_many_query_blocks_and_an_odd_tile_count():
     """More than 64 query blocks (several passes of the kernel's 64 columns, the last one partly empty) and an odd number
     of key tiles (the last pair of tiles half empty)."""

@@ -154,6 +154,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // and its results are visible; launched in the usual way it does not wait.  The kernel before says when the next one's
 // blocks may be set up, in whatever room its own leave: all of them have then started, so none can be kept out.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What the kernel before wrote is read with this where a pointer is const __restrict__: such loads may be moved across the wait.
+__device__ __forceinline__ float4 load_result4(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Non-blocking: has the phase of parity `parity` completed?

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
         const int r = item % BIAS_BLOCKS, c4 = item / BIAS_BLOCKS;
         float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (b0 + r < q_blocks) {
-            const float4 m = *reinterpret_cast<const float4*>(q_mean + (size_t(head) * q_blocks + b0 + r) * HEAD_DIM + c4 * 4);
+            const float4 m = load_result4(q_mean + (size_t(head) * q_blocks + b0 + r) * HEAD_DIM + c4 * 4);
             x[0] = m.x, x[1] = m.y, x[2] = m.z, x[3] = m.w;
         }
         float4 hi, lo;
@@ -143,7 +143,10 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
 #pragma unroll
     for (int half = 0; half < 2; ++half)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) mine[half][j] = mean[half * BIAS_HALF + g0 * 8 + j];
+        for (int j = 0; j < 16; j += 4) {
+            const float4 m = load_result4(mean + half * BIAS_HALF + g0 * 8 + j);
+            mine[half][j] = m.x, mine[half][j + 1] = m.y, mine[half][j + 2] = m.z, mine[half][j + 3] = m.w;
+        }
     auto key_of = [&](int pair) { return (2 * pair + r / KEY_TILE) * KEY_TILE + slot_key(r % KEY_TILE); };
     auto fetch = [&](int pair, int half, uint4 (&raw)[2]) {  // 32 contiguous bytes of the key's row
         const int key = key_of(pair);
@@ -270,6 +273,81 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
     }
 }
 
+// The same terms for few query blocks, on the CUDA cores: with 9 of the tensor kernel's 64 columns in use (30 heads x 4128
+// tokens) its images, hand-overs and start cost 46 us where the 32 MB of K and 4 MB of terms take 6; this form takes 17.
+// Eight lanes have a key, sixteen channels each, rotated and centred as above, and four keys at a time; per query block the
+// lanes' products of the four keys are added up across the eight by halving, four shuffles for four sums.  What bounds it:
+// issue, of which the packed multiply-adds are four cycles per key and query block (a thread per key with the means as broadcasts
+// was bound by the loads' returns, four channels per lane by shuffles and selections: both 26 us).
+constexpr int FEW_THREADS = 128, FEW_KEYS = 4, FEW_SLOTS = 4 * FEW_KEYS, FEW_BLOCKS = 32;
+__global__ void __launch_bounds__(FEW_THREADS) smooth_bias_few_kernel(const __nv_bfloat16* __restrict__ k, TokenLayout in, const float* __restrict__ k_mean,
+                                                                      const float* __restrict__ q_mean, int q_blocks, int n_keys, float scale_log2,
+                                                                      float* __restrict__ bias, RopeTable rope) {
+    static_assert(FEW_THREADS / 32 * FEW_SLOTS == KEY_TILE && HEAD_DIM == 16 * 8, "a block per key tile");
+    __shared__ float4 means[FEW_BLOCKS][4][8];  // a lane's sixteen channels (pieces of eight: lane, lane + 8) are [..][0..3][lane]
+    let_next_kernel_start();
+    const int tile = blockIdx.x, head = blockIdx.y, k_tiles = gridDim.x, lane = threadIdx.x % 32, sub = lane % 8;
+    const int slot0 = threadIdx.x / 32 * FEW_SLOTS + lane / 8 * FEW_KEYS;
+    auto key_of = [&](int i) { return tile * KEY_TILE + slot_key(slot0 + i); };
+    uint4 raw[FEW_KEYS][2];
+#pragma unroll
+    for (int i = 0; i < FEW_KEYS; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            raw[i][j] = key_of(i) < n_keys ? load_bf16x8(k + in.offset(head, key_of(i)) + (8 * j + sub) * 8, in.half) : make_uint4(0, 0, 0, 0);
+    wait_for_previous_kernel();  // the means are its results, K is not
+    for (int i = threadIdx.x; i < q_blocks * 32; i += FEW_THREADS) {
+        const int c4 = i % 32;  // channels 4 c4 .. + 3: piece c4 / 2, half c4 % 2 of it
+        means[i / 32][c4 / 16 * 2 + c4 % 2][c4 / 2 % 8] = load_result4(q_mean + (size_t(head) * q_blocks + i / 32) * HEAD_DIM + c4 * 4);
+    }
+    float2 d[FEW_KEYS][2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float4 c0 = load_result4(k_mean + head * HEAD_DIM + (8 * j + sub) * 8), c1 = load_result4(k_mean + head * HEAD_DIM + (8 * j + sub) * 8 + 4);
+#pragma unroll
+        for (int i = 0; i < FEW_KEYS; ++i) {
+            unpack8(raw[i][j], d[i][j]);
+            if (rope.table) rope8(*reinterpret_cast<float(*)[8]>(d[i][j]), rope.row(in, head, min(key_of(i), n_keys - 1)), (8 * j + sub) * 8);
+            d[i][j][0] = add2(d[i][j][0], make_float2(-c0.x, -c0.y)), d[i][j][1] = add2(d[i][j][1], make_float2(-c0.z, -c0.w));
+            d[i][j][2] = add2(d[i][j][2], make_float2(-c1.x, -c1.y)), d[i][j][3] = add2(d[i][j][3], make_float2(-c1.z, -c1.w));
+        }
+    }
+    __syncthreads();
+    const int mine = sub / 4 * 2 + sub / 2 % 2;  // the key whose sum the halving leaves in this lane (and in its neighbour)
+    const bool live = key_of(mine) < n_keys;     // slots past the last key: -inf keeps them out of the softmax
+    float* at = bias + (size_t(head) * q_blocks * k_tiles + tile) * KEY_TILE + slot0 + mine;
+#pragma unroll 1
+    for (int g = 0; g < q_blocks; ++g) {
+        float2 sum[FEW_KEYS];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 m = means[g][2 * j + h][sub];
+#pragma unroll
+                for (int i = 0; i < FEW_KEYS; ++i) {
+                    const float2 first = make_float2(m.x, m.y);
+                    sum[i] = j + h == 0 ? mul2(d[i][j][2 * h], first) : fma2(d[i][j][2 * h], first, sum[i]);
+                    sum[i] = fma2(d[i][j][2 * h + 1], make_float2(m.z, m.w), sum[i]);
+                }
+            }
+        float v[FEW_KEYS];
+#pragma unroll
+        for (int i = 0; i < FEW_KEYS; ++i) v[i] = sum[i].x + sum[i].y;
+        // a lane keeps the half of its sums that its bit names and gives the others away
+        const bool upper4 = sub & 4, upper2 = sub & 2;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float theirs = __shfl_xor_sync(0xffffffffu, upper4 ? v[i] : v[i + 2], 4);
+            v[i] = (upper4 ? v[i + 2] : v[i]) + theirs;
+        }
+        const float theirs = __shfl_xor_sync(0xffffffffu, upper2 ? v[0] : v[1], 2);
+        v[0] = (upper2 ? v[1] : v[0]) + theirs;
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        if (sub % 2 == 0) at[size_t(g) * k_tiles * KEY_TILE] = live ? v[0] * scale_log2 : -INFINITY;
+    }
+}
+
 }  // namespace unica
 
 using namespace unica;
@@ -333,6 +411,11 @@ int unica_smooth_bias(const void* k, unica_token_layout layout, const float* k_m
     if (int e = unica_check_device()) return e;
     const int tiles = (n_keys + KEY_TILE - 1) / KEY_TILE, pairs = (tiles + 1) / 2, passes = (q_blocks + BIAS_BLOCKS - 1) / BIAS_BLOCKS;
     if (heads > 65535 || passes > 65535) return unica_fail(UNICA_B200_ERR_ARGUMENT, "smooth_bias: more than 65535 heads or passes of 64 query blocks");
+    if (q_blocks <= FEW_BLOCKS) {  // up to here the form without the tensor core is the faster one: 2 blocks 14 -> 4 us, 9: 46 -> 17, 16: 115 -> 57, 32: 218 -> 178
+        launch_after(smooth_bias_few_kernel, dim3(tiles, heads), FEW_THREADS, 0, static_cast<cudaStream_t>(stream), overlapped, static_cast<const __nv_bfloat16*>(k),
+                     to_layout(layout), k_mean, q_mean, q_blocks, n_keys, scale_log2, bias, rope);
+        return unica_check_launch("smooth_bias");
+    }
     constexpr int SMEM = int(sizeof(BiasSmem)) + 128;
     // a block per SM (its images take most of the shared memory); at most four full waves of blocks, each walking over
     // its strip of key-tile pairs with the query blocks' images built once

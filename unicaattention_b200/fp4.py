@@ -99,8 +99,8 @@ def quantize_v4(v: torch.Tensor) -> tuple[FP4V, torch.Tensor]:
 
 def smooth_bias(k: torch.Tensor, k_mean: torch.Tensor, q_mean: torch.Tensor, qk_outer: torch.Tensor | None = None,
                 padded_keys: int | None = None, rope=None) -> torch.Tensor:
-    """The scores' share of Q's block means, added back exactly: q_mean[block] . (k - k_mean) to FP32 accuracy (on the
-    tensor core, each value as two tf32 parts), times
+    """The scores' share of Q's block means, added back exactly: q_mean[block] . (k - k_mean) to FP32 accuracy (for more
+    than 32 blocks on the tensor core, each value as two tf32 parts), times
     log2(e) / sqrt(128) (the attention kernel adds it to scores that are already in the log2 domain; the reference's
     table is divided by qk_outer instead, an argument kept here for the call's sake).  Keys of each 64-key tile in slot
     order, 0 past the last key.  Returns float32 [batch, heads, blocks, ceil64(n_keys)]."""
