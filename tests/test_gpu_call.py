@@ -61,3 +61,19 @@ def test_short_operands_equal_the_separate_passes(tokens):
     assert torch.equal(k8, want8) and torch.equal(scale, want_scale)
     assert all(torch.equal(a, b) for a, b in zip(unica.quantize_v_channel(v), unica.quantize_v(v)))
     unica.check_status()
+
+
+@pytest.mark.parametrize("rotated", [False, True])
+@pytest.mark.parametrize("preset", PRESETS)
+@pytest.mark.parametrize("keys", [255, 1024, 1025])
+def test_many_short_heads_equal_the_same_heads_alone(keys, preset, rotated):
+    """Enough heads for the one-launch quantizers to take clusters of four blocks (up to 1024 tokens), against one head at a time."""
+    import unicaattention_b200 as unica
+
+    q, k, v = (x.cuda() for x in qkv(1, 48, keys, keys, seed=keys, channel_scale=True))
+    settings = dict(unica.PRESETS[preset], **({"rope": rope(keys)} if rotated else {}))
+    out = unica.attention(q, k, v, **settings)
+    unica.check_status()
+    for head in (0, 17, 47):
+        alone = unica.attention(*(x[:, head:head + 1] for x in (q, k, v)), **settings)
+        assert torch.equal(alone, out[:, head:head + 1]), (keys, preset, head)

@@ -1,7 +1,7 @@
 // The quantization of a short call (up to CALL_TOKENS tokens) in ONE launch: Q, K and V of all heads, statistics included.
 //
 // The separate passes need three to eight launches for this, each a few microseconds on the device and as many on the host:
-// for 4 heads x 1024 tokens that was most of the call.  Here the grid is made of clusters of eight blocks, each of which is
+// for 4 heads x 1024 tokens that was most of the call.  Here the grid is made of clusters of eight blocks (four for many short heads), each of which is
 // given a head's K, a head's V or (NVFP4) a head's Q, and in INT8 eight tiles of Q, which need no statistics:
 //   1. the blocks of a cluster take the statistics of an eighth of the head's 256-token blocks each,
 //   2. they read one another's partial results through distributed shared memory, all in the same order,
@@ -44,7 +44,8 @@ struct CallStats {
     float scratch[2][CALL_THREADS / 32];  // by turns, so that a tile's maximum does not have to wait for the last one's readers
 };
 // this block's share of `count` things
-__device__ __forceinline__ int share(int count, int rank) { return count * rank / CALL_CLUSTER; }
+template <int CLUSTER = CALL_CLUSTER>
+__device__ __forceinline__ int share(int count, int rank) { return count * rank / CLUSTER; }
 
 // Sum, min and max per channel of 256-token block `b` into part[3][128]: channel_stats_kernel's arithmetic.
 template <bool SUMS, bool RANGE, typename Skip>
@@ -117,35 +118,35 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
 }
 
 // The head's mean (SUMS), min and max (RANGE) into sm of every block of the cluster.  Every thread of the cluster calls it.
-template <bool SUMS, bool RANGE, typename Skip>
+template <bool SUMS, bool RANGE, int CLUSTER = CALL_CLUSTER, typename Skip>
 __device__ __forceinline__ void head_stats(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const RopeTable& rope, Skip skip, int head,
                                            int n_tokens, int rank, CallStats& sm) {
-    const int blocks = (n_tokens + CALL_BLOCK - 1) / CALL_BLOCK, b0 = share(blocks, rank), b1 = share(blocks, rank + 1);
+    const int blocks = (n_tokens + CALL_BLOCK - 1) / CALL_BLOCK, b0 = share<CLUSTER>(blocks, rank), b1 = share<CLUSTER>(blocks, rank + 1);
     for (int b = b0; b < b1; ++b) block_stats<SUMS, RANGE>(x, in, rope, skip, head, b, n_tokens, sm, sm.part[b - b0]);
     cg::this_cluster().sync();
     if (threadIdx.x < HEAD_DIM) {
         // all blocks' partial results asked for before the first is added up: a trip to another SM takes some hundred cycles
         float s = 0.0f, lo = INFINITY, hi = -INFINITY;
-        float theirs_s[CALL_CLUSTER], theirs_lo[CALL_CLUSTER], theirs_hi[CALL_CLUSTER];
-        const int most = (blocks + CALL_CLUSTER - 1) / CALL_CLUSTER;
+        float theirs_s[CLUSTER], theirs_lo[CLUSTER], theirs_hi[CLUSTER];
+        const int most = (blocks + CLUSTER - 1) / CLUSTER;
         if (most == 1) {
 #pragma unroll
-            for (int r = 0; r < CALL_CLUSTER; ++r) {
+            for (int r = 0; r < CLUSTER; ++r) {
                 const CallStats* theirs = cg::this_cluster().map_shared_rank(&sm, r);
                 if (SUMS) theirs_s[r] = theirs->part[0][0][threadIdx.x];
                 if (RANGE) theirs_lo[r] = theirs->part[0][1][threadIdx.x], theirs_hi[r] = theirs->part[0][2][threadIdx.x];
             }
 #pragma unroll
-            for (int r = 0; r < CALL_CLUSTER; ++r)
-                if (share(blocks, r + 1) > share(blocks, r)) {  // the others hold nothing
+            for (int r = 0; r < CLUSTER; ++r)
+                if (share<CLUSTER>(blocks, r + 1) > share<CLUSTER>(blocks, r)) {  // the others hold nothing
                     if (SUMS) s += theirs_s[r];
                     if (RANGE) lo = fminf(lo, theirs_lo[r]), hi = fmaxf(hi, theirs_hi[r]);
                 }
         } else {
 #pragma unroll
-            for (int r = 0; r < CALL_CLUSTER; ++r) {
+            for (int r = 0; r < CLUSTER; ++r) {
                 const CallStats* theirs = cg::this_cluster().map_shared_rank(&sm, r);
-                const int parts = share(blocks, r + 1) - share(blocks, r);
+                const int parts = share<CLUSTER>(blocks, r + 1) - share<CLUSTER>(blocks, r);
                 float part_s[CALL_PARTS], part_lo[CALL_PARTS], part_hi[CALL_PARTS];
 #pragma unroll
                 for (int i = 0; i < CALL_PARTS; ++i) {
@@ -274,24 +275,24 @@ __device__ __forceinline__ void each_tile(int first, int last, Load load, Finish
 }
 
 // V_MODE: UNICA_B200_V_*; HALF, ROPE: the input is float16, Q and K are rotated (template parameters so that the other calls
-// carry none of it).  Clusters: heads of K, heads of V, then eight tiles of Q each.
-template <int V_MODE, bool HALF, bool ROPE>
-__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
+// carry none of it).  Clusters: heads of K, heads of V, then CLUSTER tiles of Q each.
+template <int V_MODE, bool HALF, bool ROPE, int CLUSTER>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
     let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ CallOutliers outliers;
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0}, none{nullptr, 0};
-    const int rank = int(blockIdx.x) % CALL_CLUSTER, clusters_k = call.k.x ? call.heads : 0, clusters_v = call.v.x ? call.heads : 0;
-    int cluster = int(blockIdx.x) / CALL_CLUSTER;
+    const int rank = int(blockIdx.x) % CLUSTER, clusters_k = call.k.x ? call.heads : 0, clusters_v = call.v.x ? call.heads : 0;
+    int cluster = int(blockIdx.x) / CLUSTER;
     if (cluster < clusters_k) {
         const CallOperand& op = call.k;
         TokenLayout in = op.in;
         in.half = HALF;
         const int head = cluster;
-        head_stats<true, false>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, false, CLUSTER>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
         each_tile<RowsRaw<KEY_TILE>>(
-            share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { rows_load<KEY_TILE>(raw, op.x, in, head, t, op.n_tokens); },
+            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { rows_load<KEY_TILE>(raw, op.x, in, head, t, op.n_tokens); },
             [&](const auto& raw, int t) {
                 const size_t tile = size_t(head) * op.tiles + t;
                 rows_int8_finish<KEY_TILE>(raw, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
@@ -305,7 +306,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
             each_tile<VRaw>(
-                share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { v_load(raw, op.x, in, skip, head, t, op.n_tokens); },
+                share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_load(raw, op.x, in, skip, head, t, op.n_tokens); },
                 [&](const auto& raw, int t) {
                     v_int8_finish<decltype(per_token)::value>(raw, sm.low, sm.high, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale,
                                                               call.v_token, sm.v_tile[t & 1]);
@@ -316,7 +317,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         } else if constexpr (V_MODE == UNICA_B200_V_OUTLIERS) {
             find_outliers(op.x, in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
             const SkipKeys skip{outliers.is_outlier};
-            head_stats<false, true>(op.x, in, none, skip, head, op.n_tokens, rank, sm);
+            head_stats<false, true, CLUSTER>(op.x, in, none, skip, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, skip);
             if (rank == 0) {  // the outliers' rows over the channel scales
                 for (int i = threadIdx.x; i < call.n_outliers * HEAD_DIM; i += CALL_THREADS) {
@@ -332,7 +333,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
                 }
             }
         } else {
-            head_stats<false, true>(op.x, in, none, NoSkip{}, head, op.n_tokens, rank, sm);
+            head_stats<false, true, CLUSTER>(op.x, in, none, NoSkip{}, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, NoSkip{});
         }
     } else {
@@ -340,7 +341,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         const CallOperand& op = call.q;
         TokenLayout in = op.in;
         in.half = HALF;
-        const int tile = cluster * CALL_CLUSTER + rank, head = tile / op.tiles, t = tile % op.tiles;
+        const int tile = cluster * CLUSTER + rank, head = tile / op.tiles, t = tile % op.tiles;
         if (head < call.heads) {
             int8_t* codes = reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM);
             float* scale = static_cast<float*>(op.scales) + tile;
@@ -358,19 +359,19 @@ __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (
 
 // Clusters: heads of K, of V, of Q.  Rotated inputs keep twice the loads in flight: with three blocks per SM their registers
 // spilled (2 x 16 heads x 777 tokens: 49 us, with two 42 us).
-template <bool HALF, bool ROPE>
-__global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+template <bool HALF, bool ROPE, int CLUSTER>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0};
-    const int rank = int(blockIdx.x) % CALL_CLUSTER;
-    const int kind = int(blockIdx.x) / CALL_CLUSTER / call.heads, head = int(blockIdx.x) / CALL_CLUSTER % call.heads;
+    const int rank = int(blockIdx.x) % CLUSTER;
+    const int kind = int(blockIdx.x) / CLUSTER / call.heads, head = int(blockIdx.x) / CLUSTER % call.heads;
     if (kind == 0) {
         const CallOperand& op = call.k;
         TokenLayout in = op.in;
         in.half = HALF;
-        head_stats<true, true>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, true, CLUSTER>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
             const float m = sm.mean[threadIdx.x];
@@ -379,7 +380,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         }
         const Fp4Outer outer = fp4_outer(outer_scale(block_max<CALL_THREADS>(amax, sm.scratch[0])));
         if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
-        for (int t = share(op.tiles, rank); t < share(op.tiles, rank + 1); ++t) {  // (no barrier in a tile: the warps run ahead of one another)
+        for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {  // (no barrier in a tile: the warps run ahead of one another)
             const size_t tile = size_t(head) * op.tiles + t;
             rows_fp4_tile<KEY_TILE, true>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
                                           static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), rope);
@@ -388,9 +389,9 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         const CallOperand& op = call.v;
         TokenLayout in = op.in;
         in.half = HALF;
-        head_stats<false, true>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<false, true, CLUSTER>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
         each_tile<VRaw>(
-            share(op.tiles, rank), share(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, op.x, in, head, t, op.n_tokens); },
+            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, op.x, in, head, t, op.n_tokens); },
             [&](const auto& raw, int t) {
                 const size_t tile = size_t(head) * op.tiles + t;
                 v_fp4_finish(raw, sm.low, sm.high, t, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
@@ -403,7 +404,7 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         in.half = HALF;
         const int groups = (op.n_tokens + call.smooth - 1) / call.smooth, per = call.smooth / CALL_BLOCK, blocks = (op.n_tokens + CALL_BLOCK - 1) / CALL_BLOCK;
         float amax = 0.0f;
-        for (int g = share(groups, rank); g < share(groups, rank + 1); ++g) {
+        for (int g = share<CLUSTER>(groups, rank); g < share<CLUSTER>(groups, rank + 1); ++g) {
             float s = 0.0f, lo = INFINITY, hi = -INFINITY;
             const int b1 = min((g + 1) * per, blocks);
             for (int b = g * per; b < b1; ++b) {
@@ -423,10 +424,10 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
         __threadfence();
         cg::this_cluster().sync();
         amax = 0.0f;
-        for (int r = 0; r < CALL_CLUSTER; ++r) amax = fmaxf(amax, *cg::this_cluster().map_shared_rank(&q_amax, r));
+        for (int r = 0; r < CLUSTER; ++r) amax = fmaxf(amax, *cg::this_cluster().map_shared_rank(&q_amax, r));
         const Fp4Outer outer = fp4_outer(outer_scale(amax));
         if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
-        const int t0 = share(op.tiles, rank), t1 = share(op.tiles, rank + 1), g0 = t0 * QUERY_TILE / call.smooth;
+        const int t0 = share<CLUSTER>(op.tiles, rank), t1 = share<CLUSTER>(op.tiles, rank + 1), g0 = t0 * QUERY_TILE / call.smooth;
         const int touched = t1 > t0 ? min((t1 * QUERY_TILE - 1) / call.smooth, groups - 1) - g0 + 1 : 0;  // groups of this block's tiles (its last ones may lie past the end)
         for (int i = threadIdx.x; i < touched * HEAD_DIM; i += CALL_THREADS)
             q_means[i / HEAD_DIM][i % HEAD_DIM] = __ldcg(op.mean + (size_t(head) * groups + g0) * HEAD_DIM + i);
@@ -442,15 +443,21 @@ __global__ void __cluster_dims__(CALL_CLUSTER, 1, 1) __launch_bounds__(CALL_THRE
 
 int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
-    const long long q_tiles = call.q.x ? (static_cast<long long>(call.heads) * call.q.tiles + CALL_CLUSTER - 1) / CALL_CLUSTER : 0;
-    const long long clusters = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0) + q_tiles;
+    const long long q_tiles = call.q.x ? static_cast<long long>(call.heads) * call.q.tiles : 0, kv_heads = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0);
+    // as in quantize_call_fp4: 32 heads x 777 50.6 -> 43.3 us a call, 40 x 1024 70.5 -> 62; the tiles of Q fill gaps, and where only
+    // they make a second wave (24 x 1000) four blocks per head were 2 us slower
+    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && call.k.n_tokens <= 4 * CALL_BLOCK && kv_heads * CALL_CLUSTER > 3 * 148;
+    const int cluster = four ? 4 : CALL_CLUSTER;
+    const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
     if (clusters > (1 << 27)) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: too many heads and tiles");
-    const dim3 grid(unsigned(clusters) * CALL_CLUSTER);
+    const dim3 grid(unsigned(clusters) * cluster);
     auto launch = [&](auto half, auto rope) {
         constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
-        auto kernel = call.v_mode == UNICA_B200_V_TOKEN      ? quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE>
-                      : call.v_mode == UNICA_B200_V_OUTLIERS ? quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, HALF, ROPE>
-                                                             : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE>;
+        auto kernel = call.v_mode == UNICA_B200_V_OUTLIERS ? quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, HALF, ROPE, CALL_CLUSTER>
+                      : call.v_mode == UNICA_B200_V_TOKEN ? (four ? quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, 4>
+                                                                  : quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, CALL_CLUSTER>)
+                                                          : (four ? quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, 4>
+                                                                  : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, CALL_CLUSTER>);
         kernel<<<grid, CALL_THREADS, 0, stream>>>(call);
     };
     const bool half = (call.q.x ? call.q : call.k.x ? call.k : call.v).in.half;
@@ -461,10 +468,19 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
 
 int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
-    const bool half = call.q.in.half;
-    auto kernel = call.rope.table ? (half ? quantize_call_fp4_kernel<true, true> : quantize_call_fp4_kernel<false, true>)
-                                  : (half ? quantize_call_fp4_kernel<true, false> : quantize_call_fp4_kernel<false, false>);
-    kernel<<<dim3(3u * call.heads * CALL_CLUSTER), CALL_THREADS, 0, stream>>>(call);
+    // Four blocks per head where a head's statistics are four 256-token blocks at most, if eight blocks per head are more than
+    // the chip takes at once: half of the eight have nothing to do in the first step, and a second wave costs its latency again
+    // (2 x 16 heads x 777 tokens, rotated: 41.7 -> 38 us, and 75.6 -> 68.1 for the call; 40 x 1024 not rotated 37 -> 30).
+    const int longest = call.q.n_tokens > call.k.n_tokens ? call.q.n_tokens : call.k.n_tokens;
+    const bool four = longest <= 4 * CALL_BLOCK && 3 * call.heads * CALL_CLUSTER > 148 * (call.rope.table ? 2 : 3);
+    auto launch = [&](auto half, auto rope) {
+        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
+        const int cluster = four ? 4 : CALL_CLUSTER;
+        auto kernel = four ? quantize_call_fp4_kernel<HALF, ROPE, 4> : quantize_call_fp4_kernel<HALF, ROPE, CALL_CLUSTER>;
+        kernel<<<dim3(3u * call.heads * cluster), CALL_THREADS, 0, stream>>>(call);
+    };
+    call.rope.table ? (call.q.in.half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))
+                    : (call.q.in.half ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{}));
     return unica_check_launch("quantize_call_fp4");
 }
 
