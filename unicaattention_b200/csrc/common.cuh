@@ -69,29 +69,6 @@ struct PeerOutputs {
     int count;
 };
 
-// Output rows on their way out through shared memory, so that a warp writes whole 256-byte rows (two per instruction)
-// instead of 32 separate pieces of 16 bytes: that matters little for this GPU's memory and much for rows that cross
-// NVLink to a peer.  A warp owns 32 rows of 128 bf16 in `staged` (8 KB); the 16-byte pieces of a row are swapped about
-// by the row number, so neither the row-per-thread writes nor the row-per-half-warp reads meet bank conflicts.
-__device__ __forceinline__ void stage_piece(uint8_t* staged, int row_in_warp, int piece, uint4 value) {
-    *reinterpret_cast<uint4*>(staged + row_in_warp * 256 + ((piece ^ (row_in_warp & 15)) * 16)) = value;
-}
-// The warp's 32 staged rows (query rows first_row ..) to `out` and to every peer; all lanes call it after __syncwarp().
-__device__ __forceinline__ void store_staged_rows(const uint8_t* staged, int lane, int first_row, int n_queries, int head,
-                                                  __nv_bfloat16* out, const TokenLayout& layout, const PeerOutputs& peers) {
-    const int piece = lane % 16;
-#pragma unroll 4
-    for (int pair = 0; pair < 16; ++pair) {
-        const int r = 2 * pair + lane / 16;
-        const uint4 value = *reinterpret_cast<const uint4*>(staged + r * 256 + ((piece ^ (r & 15)) * 16));
-        if (first_row + r < n_queries) {
-            const size_t at = layout.offset(head, first_row + r) + piece * 8;
-            *reinterpret_cast<uint4*>(out + at) = value;
-            for (int peer = 0; peer < peers.count; ++peer) *reinterpret_cast<uint4*>(peers.out[peer] + at) = value;
-        }
-    }
-}
-
 // RoPE inside the quantizers (the reference's rope_chunk, csrc/flash.cu:250-268): (cos, sin) per pair of channels in fp16,
 // [batch or 1][n_tokens][64][2]; batch_stride in halves, 0 when one table serves every batch.  table null: no rotation.
 struct RopeTable {
@@ -347,91 +324,6 @@ __device__ __forceinline__ bool mbar_wait_line(uint64_t* bar, int parity, int* a
     return false;
 }
 
-// Two barriers at once: both probes are in flight together, so a lone thread pays one probe latency (some 250 cycles)
-// instead of two.  parity_b < 0: there is no second barrier.
-template <unsigned SLEEP_NS = WAIT_SLEEP_NS>
-__device__ __forceinline__ bool mbar_probe_many2(uint64_t* bar_a, int parity_a, uint64_t* bar_b, int parity_b) {
-    uint32_t done;
-    if constexpr (SLEEP_NS > 0) {
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q, r;\n\t"
-            ".reg .u32 left;\n\t"
-            "mov.u32 left, %5;\n"
-            "UNICA_WAIT2_AGAIN:\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
-            "and.pred r, p, q;\n\t"
-            "@r bra UNICA_WAIT2_DONE;\n\t"
-            "nanosleep.u32 %6;\n\t"
-            "sub.u32 left, left, 1;\n\t"
-            "setp.ne.u32 q, left, 0;\n\t"
-            "@q bra UNICA_WAIT2_AGAIN;\n"
-            "UNICA_WAIT2_DONE:\n\t"
-            "selp.u32 %0, 1, 0, r;\n\t"
-            "}"
-            : "=r"(done)
-            : "r"(smem_u32(bar_a)), "r"(parity_a), "r"(smem_u32(bar_b)), "r"(parity_b), "n"(WAIT_PROBES), "n"(SLEEP_NS)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q, r;\n\t"
-            ".reg .u32 left;\n\t"
-            "mov.u32 left, %5;\n"
-            "UNICA_SPIN2_AGAIN:\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
-            "and.pred r, p, q;\n\t"
-            "@r bra UNICA_SPIN2_DONE;\n\t"
-            "sub.u32 left, left, 1;\n\t"
-            "setp.ne.u32 q, left, 0;\n\t"
-            "@q bra UNICA_SPIN2_AGAIN;\n"
-            "UNICA_SPIN2_DONE:\n\t"
-            "selp.u32 %0, 1, 0, r;\n\t"
-            "}"
-            : "=r"(done)
-            : "r"(smem_u32(bar_a)), "r"(parity_a), "r"(smem_u32(bar_b)), "r"(parity_b), "n"(WAIT_PROBES)
-            : "memory");
-    }
-    return done != 0;
-}
-template <unsigned SLEEP_NS = WAIT_SLEEP_NS>
-__device__ __forceinline__ bool mbar_wait2(uint64_t* bar_a, int parity_a, uint64_t* bar_b, int parity_b, volatile int* abort_flag, int* status,
-                                           int code) {
-    if (parity_b < 0) return mbar_wait<SLEEP_NS>(bar_a, parity_a, abort_flag, status, code);
-    if constexpr (SLEEP_NS == 0 && UNICA_WAIT_HINT_NS > 0) {  // one look at both with the probes in flight together, then suspended waits
-        uint32_t seen;
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q;\n\t"
-            ".reg .u32 a, b;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
-            "selp.u32 a, 1, 0, p;\n\t"
-            "selp.u32 b, 2, 0, q;\n\t"
-            "or.b32 %0, a, b;\n\t"
-            "}"
-            : "=r"(seen)
-            : "r"(smem_u32(bar_a)), "r"(parity_a), "r"(smem_u32(bar_b)), "r"(parity_b)
-            : "memory");
-        if (seen == 3) return true;
-        if (!(seen & 1) && !mbar_wait<0>(bar_a, parity_a, abort_flag, status, code)) return false;
-        return (seen & 2) || mbar_wait<0>(bar_b, parity_b, abort_flag, status, code);
-    }
-    if (mbar_probe_many2<SLEEP_NS>(bar_a, parity_a, bar_b, parity_b)) return true;
-    const long long start = clock64();
-    while (true) {
-        if (mbar_probe_many2<SLEEP_NS>(bar_a, parity_a, bar_b, parity_b)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - start > WAIT_LIMIT_CYCLES) {
-            *abort_flag = 1;
-            if (status) atomicCAS(status, 0, code);
-            return false;
-        }
-    }
-}
-
 // The same for a whole warp: every lane waits, and all get the same answer.  The vote also reconverges the warp, which
 // the .sync.aligned tensor-memory instructions that usually follow require: a tcgen05.ld executed by part of a warp
 // never completes.
@@ -595,15 +487,6 @@ __device__ __forceinline__ void reg_fence4(float2 (&v)[4]) {
     asm volatile("" : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[3].x), "+f"(v[3].y) : : "memory");
 }
 
-// 32 consecutive columns of this thread's lane set to one value.
-__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
-        "r"(v)
-        : "memory");
-}
-
 // The same from a block of registers the caller keeps alive: tcgen05.st takes consecutive registers, so a single value
 // would be copied into as many registers before every store.  fill_block_init() makes the block; the `volatile` moves
 // keep the compiler from folding it back into one register.
@@ -679,15 +562,6 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, ui
         "}\n" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate))
         : "memory");
-}
-// x = hi + lo up to 2^-24 |x|, both with tf32's 11 significant bits (round to nearest): three tf32 products
-// hi.hi + lo.hi + hi.lo then carry an FP32 product to about 2^-22.
-__device__ __forceinline__ void tf32_split(float x, float& hi, float& lo) {
-    uint32_t bits;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(bits) : "f"(x));
-    hi = __uint_as_float(bits);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(bits) : "f"(x - hi));  // the difference is exact
-    lo = __uint_as_float(bits);
 }
 
 // D[tmem] (+)= A[smem] . B[smem]^T, issued by one thread.
