@@ -29,8 +29,7 @@
 //   - nothing waits in a loop where it can be helped: hand-overs between warps are named barriers, on which the hardware
 //     blocks a warp (probing loops had grown to half of all issued instructions), and the copies are issued where their
 //     slots are known to be free, so that nobody polls for them;
-//   - the accumulators are added up without a conversion to float (flush32), P^ is rounded and packed by multiplications into
-//     the denormal range (softmax_tile);
+//   - the accumulators are added up without a conversion to float (flush32), and P^ is rounded without one (softmax_tile);
 //   - the flush warps load the next accumulator while they add up the present one, the softmax warps ask for their next scores
 //     while the exponentials run: a probe's answer takes some sixty cycles.
 //
@@ -71,7 +70,6 @@ constexpr int SCALE_BYTES = HEAD_DIM * 4;       // 512
 constexpr int TMEM_COLUMNS = 512;
 constexpr int COL_S = 0, COL_ACC = 256;
 constexpr int OUTLIER_BATCH = 16;  // outlier keys whose rows are in shared memory at a time (the epilogue of the outliers mode)
-constexpr float P_SHIFT = 23.0f, P_UNIT = 1.17549435e-38f;  // 2^-126: see the rounding of P^ in softmax_tile
 constexpr float REFERENCE_SLACK = 60.0f;  // log2: how far a tile maximum may rise above a row's reference exponent
 
 struct __align__(128) AttSmem {
@@ -312,7 +310,7 @@ __device__ __forceinline__ float load_scale(const float* p) {  // volatile: the 
 template <bool V_TOKEN, bool MASKED>
 __device__ __forceinline__ bool softmax_tile(AttSmem& sm, uint32_t ts, int g, int row, float c, int valid,
                                              const uint32_t (&magic)[FILL_BLOCK]) {
-    const float2 c2 = make_float2(c, c), minus_magic = make_float2(-MAGIC, -MAGIC);
+    const float2 c2 = make_float2(c, c), minus_magic = make_float2(-MAGIC, -MAGIC), plus_magic = make_float2(MAGIC, MAGIC);
     const float4* log_s4 = reinterpret_cast<const float4*>(sm.tok[slot<V_RING>(g)]);
     const float4* inv_s4 = reinterpret_cast<const float4*>(sm.tok[slot<V_RING>(g)] + KEY_TILE);
     uint8_t* p_row = sm.p[slot<P_RING>(g)] + row * 16;
@@ -348,16 +346,16 @@ __device__ __forceinline__ bool softmax_tile(AttSmem& sm, uint32_t ts, int g, in
     // P^ = rint(255 * 2^(score * c - tile max)).  Per channel the float read back is MAGIC + score, so the exponent is
     // x * c + (offset - MAGIC * c) in ONE fused multiply-add; what the rounding of that constant loses (it is about
     // 2^11 in size) is put back exactly: `low` is the lost part, and the product p * 2^low happens inside the
-    // multiplication that rounds p to a byte: 2^-149 times an integer is the denormal float whose bits are that integer, so
-    // scaling p by 2^-149 (2^-23 of it in the exponent) rounds it to an integer, and two such integers are packed into
-    // 16 bits by an exact multiply-add.
-    const float offset = (LOG2_255 - tile_max) - P_SHIFT;
-    float2 base2 = make_float2(offset, offset), k2 = make_float2(P_UNIT, P_UNIT);
+    // multiply-add that rounds p to a byte.  The exponent's argument itself ends below 8, where a float's step is 2^-21 (four
+    // times that with a factor of 2^-23 taken into it to scale P^ on its way: 1.3e-5 of the bytes 1 .. 64 then missed their
+    // exact rounding, 2.7e-6 so).
+    const float offset = LOG2_255 - tile_max;
+    float2 base2 = make_float2(offset, offset), k2 = make_float2(1.0f, 1.0f);
     if (!V_TOKEN) {
         const float a_hi = __fmul_rn(-MAGIC, c), a_lo = __fmaf_rn(-MAGIC, c, -a_hi);  // -MAGIC * c = a_hi + a_lo exactly
         const float sum = __fadd_rn(a_hi, offset), bb = __fsub_rn(sum, a_hi);
         const float low = __fadd_rn(__fadd_rn(__fsub_rn(a_hi, __fsub_rn(sum, bb)), __fsub_rn(offset, bb)), a_lo);  // a_hi + offset = sum + ..
-        const float k = __fmaf_rn(low, 0.693147181f, 1.0f) * P_UNIT;  // 2^low, |low| < 2^-12
+        const float k = __fmaf_rn(low, 0.693147181f, 1.0f);  // 2^low, |low| < 2^-12
         base2 = make_float2(sum, sum), k2 = make_float2(k, k);
     }
     // (mbarrier.try_wait may hold the warp for microseconds when the phase is not complete, and after an item's last tiles
@@ -382,12 +380,13 @@ __device__ __forceinline__ bool softmax_tile(AttSmem& sm, uint32_t ts, int g, in
             }
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) e[j] = mul2(e[j], k2);  // the bits of each are rint(p)
+        for (int j = 0; j < 8; ++j) e[j] = V_TOKEN ? add2(e[j], plus_magic) : fma2(e[j], k2, plus_magic);  // the low byte of each is rint(p)
         uint32_t w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float2 two = fma2(e[2 * i + 1], make_float2(256.0f, 256.0f), e[2 * i]);  // keys 0 and 2 | keys 1 and 3
-            w[i] = __byte_perm(__float_as_uint(two.x), __float_as_uint(two.y), 0x5140);
+            const uint32_t lo = __byte_perm(__float_as_uint(e[2 * i].x), __float_as_uint(e[2 * i].y), 0x0040);
+            const uint32_t hi = __byte_perm(__float_as_uint(e[2 * i + 1].x), __float_as_uint(e[2 * i + 1].y), 0x0040);
+            w[i] = __byte_perm(lo, hi, 0x5410);
             if (!V_TOKEN && MASKED) {  // keys past the end weigh nothing
                 const int left = valid - (step * 16 + i * 4);
                 w[i] = left >= 4 ? w[i] : left <= 0 ? 0u : (w[i] & ((1u << (8 * left)) - 1u));
@@ -397,7 +396,7 @@ __device__ __forceinline__ bool softmax_tile(AttSmem& sm, uint32_t ts, int g, in
         *reinterpret_cast<uint4*>(p_row + step * (QUERY_TILE * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (V_TOKEN) sm.p_sum[slot<ST_RING>(g)][row] = uint16_t(isum[0] + isum[1]);
-    sm.st[slot<ST_RING>(g)][row] = make_float2(tile_max, V_TOKEN ? (fsum.x + fsum.y) * 8388608.0f : __uint2float_rn(isum[0] + isum[1]));
+    sm.st[slot<ST_RING>(g)][row] = make_float2(tile_max, V_TOKEN ? fsum.x + fsum.y : __uint2float_rn(isum[0] + isum[1]));
     fence_proxy_async();
     __syncwarp();
     pv_arrive(g);  // P^(g) and its record delivered
