@@ -63,6 +63,21 @@ def test_short_operands_equal_the_separate_passes(tokens):
     unica.check_status()
 
 
+@pytest.mark.parametrize("heads", [55, 60, 112])
+@pytest.mark.parametrize("tokens", [1024, 1025, 4128, 8192])
+def test_short_operands_of_many_heads(tokens, heads):
+    """K alone and V alone, with and without enough heads for clusters of four blocks, which have room for 4096 tokens."""
+    import unicaattention_b200 as unica
+
+    x = (torch.randn(1, heads, tokens, 128, generator=torch.Generator("cuda").manual_seed(tokens), device="cuda") + 0.5).bfloat16()
+    k8, scale, mean = unica.quantize_k(x)
+    assert torch.equal(mean, unica.rope_stats(x)[0])
+    want8, want_scale = unica.quantize_int8(x, mean, 64)
+    assert torch.equal(k8, want8) and torch.equal(scale, want_scale)
+    assert all(torch.equal(a, b) for a, b in zip(unica.quantize_v_channel(x), unica.quantize_v(x)))
+    unica.check_status()
+
+
 @pytest.mark.parametrize("rotated", [False, True])
 @pytest.mark.parametrize("preset", PRESETS)
 @pytest.mark.parametrize("keys", [255, 1024, 1025])

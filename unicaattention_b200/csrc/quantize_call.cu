@@ -446,8 +446,10 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
     const long long q_tiles = call.q.x ? static_cast<long long>(call.heads) * call.q.tiles : 0, kv_heads = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0);
     // as in quantize_call_fp4: 32 heads x 777 50.6 -> 43.3 us a call, 40 x 1024 70.5 -> 62; the tiles of Q fill gaps, and where only
     // they make a second wave (24 x 1000) four blocks per head were 2 us slower
-    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && call.k.n_tokens <= 4 * CALL_BLOCK && kv_heads * CALL_CLUSTER > 3 * 148;
+    const int keys = call.k.n_tokens > call.v.n_tokens ? call.k.n_tokens : call.v.n_tokens;  // (a call may have one of the two alone)
+    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= 4 * CALL_BLOCK && kv_heads * CALL_CLUSTER > 3 * 148;
     const int cluster = four ? 4 : CALL_CLUSTER;
+    if (keys > cluster * CALL_PARTS * CALL_BLOCK) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: more tokens than a cluster's blocks have room for");
     const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
     if (clusters > (1 << 27)) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: too many heads and tiles");
     const dim3 grid(unsigned(clusters) * cluster);
