@@ -18,7 +18,8 @@
  * Operand layouts written by the quantizers and read by the attention kernels (all per head, tiles in token order):
  *   Q8   [q_tiles][8][128 rows][16]  int8, q_tiles rounded up to even, 16 KB per tile of 128 queries
  *   K8   [k_tiles][8][ 64 rows][16]  int8, 8 KB per tile of 64 keys          (chunk c, row r: channels 16c..16c+15 of key r)
- *   V8   [k_tiles][4][128 chan][16]  code + 128 as an unsigned byte, 8 KB per tile (chunk c, channel d: keys 16c..16c+15)
+ *   V8   [k_tiles][4][128 chan][16]  unsigned bytes, 8 KB per tile (chunk c, channel d: keys 16c..16c+15): 128 + code in tiles of
+ *        even number, 128 - code in odd ones
  *   v_token [k_tiles][2][64] float: log2 s_j then 1 / s_j of the tile's keys (per-token mode)
  * These are the shared-memory images tcgen05.mma reads (K-major, no swizzle: core matrices of 8 rows x 16 bytes), so a
  * tile is one contiguous bulk copy.  Rows past the last token are zeros.
@@ -137,7 +138,7 @@ int unica_b200_quantize_v_int8_fused(const void* v, unica_token_layout layout, i
 
 /* Replaces attention_int8pv_tma (csrc/flash.cu:806-959; launched from unica/__init__.py:179-189).  The accurate mode:
  * S = Q8.K8^T on tcgen05 kind::i8, softmax in the log2 domain against each 64-key tile's own maximum, P as u8,
- * P.V8 on kind::i8 (u8 x u8: V8 carries + 128), flushed into a float accumulator with alpha / beta every tile.
+ * P.V8 on kind::i8 (u8 x u8: V8 carries 128), flushed into a float accumulator with alpha / beta every tile.
  * out: bf16 in out_layout.  scale_log2 = log2(e) / sqrt(128).  status: device int the kernel leaves non-zero if one
  * of its bounded waits gave up (must be 0 on entry), or NULL.
  * v_mode UNICA_B200_V_OUTLIERS (the reference's V_OUTLIERS, csrc/flash.cu:748-790): V8 per channel with each head's

@@ -329,8 +329,8 @@ def quantize_v(v: torch.Tensor, layout: int = 2, per_token: bool = False, outlie
     """v ~ v8 * scale (unica/__init__.py:402-444).  Per channel (default): one scale per channel over the head's
     tokens, float32 [batch, heads, 128].  per_token: one scale per token over its channels; returns v8, a scale of ones
     and float32 [batch, heads, tiles, 2, 64] = log2 s then 1 / s of each tile's keys (zeros past N).
-    v8: int8 [batch, heads, tiles, 4, 128, 16] (tile, 16-key chunk, channel, key: the K-major operand of P.V, each byte the
-    code plus 128);
+    v8: int8 [batch, heads, tiles, 4, 128, 16] (tile, 16-key chunk, channel, key: the K-major operand of P.V, each byte
+    128 plus the code in even tiles, 128 minus the code in odd ones);
     `decode_v8` gives [batch, heads, N, 128].  `layout` is accepted for compatibility: there is one layout here.
     outliers: the per-channel scale without the `outliers` (<= 8) keys of each head with the largest max |v|, which are
     written as zeros; returns v8, scale, those keys (int32 [batch, heads, outliers], -1: none) and their rows over the
@@ -386,8 +386,9 @@ def v_outliers(v: torch.Tensor, count: int) -> torch.Tensor:
 def decode_v8(v8: torch.Tensor, n: int) -> torch.Tensor:
     """quantize_v's codes as plain int8 [batch, heads, n, 128]."""
     batch, heads, tiles = v8.shape[:3]
-    codes = v8.permute(0, 1, 2, 3, 5, 4).reshape(batch, heads, tiles * V8_PAD_KEYS, HEAD_DIM)[:, :, :n]
-    return codes ^ -128  # stored as the unsigned byte code + 128
+    codes = v8 ^ -128  # stored as the unsigned byte 128 + code ...
+    codes[:, :, 1::2].neg_()  # ... or 128 - code (the codes are -127 .. 127)
+    return codes.permute(0, 1, 2, 3, 5, 4).reshape(batch, heads, tiles * V8_PAD_KEYS, HEAD_DIM)[:, :, :n]
 
 
 # ----------------------------------------------------------------------------------------------------------------------

@@ -21,7 +21,9 @@ constexpr int HEAD_DIM = 128;
 constexpr int KEY_TILE = 64;     // keys per tile: the K scale block and the softmax tile of the numerics contract
 constexpr int QUERY_TILE = 128;  // query rows per tile: the Q scale block, and M of one tcgen05.mma
 constexpr float LOG2_255 = 7.99435343685886f;
-constexpr float V8_BIAS = 128.0f;  // V8 is stored as code + 128, an unsigned byte (see flush32 in attention_int8.cu)
+// V8 is stored as an unsigned byte: V8_BIAS plus the code in key tiles of even number, V8_BIAS minus the code in odd ones, whose
+// sums are then subtracted: what the bias adds to one tile's sums it takes from the next one's (see flush32 in attention_int8.cu).
+constexpr float V8_BIAS = 128.0f;
 
 // Where token `token` of head `head_index` (= batch * heads + head) starts in a [batch, heads, tokens, 128] tensor with
 // a contiguous last dimension and any other strides; strides in elements.  Field for field the reference's struct

@@ -200,7 +200,8 @@ __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restri
 // the channel's min and max over the head (low, high: [heads][128]); true: one scale per key over its channels, and
 // v_token [heads][tiles][2][64] gets log2 s and 1 / s of the tile's keys (zeros past n_tokens).  skip: [heads][n_tokens],
 // 1 = the key is written as zeros (outlier keys), or null.
-// v8: [heads][tiles][4 chunks of 16 keys][128 channels][16] bytes, code + V8_BIAS: the K-major B operand of P.V.  v_scale [heads][128].
+// v8: [heads][tiles][4 chunks of 16 keys][128 channels][16] bytes, V8_BIAS plus the code (even tiles) or minus it (odd
+// ones; see V8_BIAS): the K-major B operand of P.V.  v_scale [heads][128].
 template <bool PER_TOKEN, int NT = THREADS, bool STAGED = false>
 __device__ __forceinline__ void v_int8_emit(const __nv_bfloat16 (*tile)[HEAD_DIM], bool half, const float* key_scale, const float* key_inv,
                                             const float* low, const float* high, int head, int t, int tiles, int8_t* __restrict__ v8,
@@ -284,6 +285,8 @@ __device__ __forceinline__ void v_int8_emit(const __nv_bfloat16 (*tile)[HEAD_DIM
         inv2 = make_float2(__frcp_rn(scale2.x), __frcp_rn(scale2.y));
     }
     if (t == 0 && v_scale && keys == 0) *reinterpret_cast<float2*>(v_scale + head * HEAD_DIM + c) = scale2;
+    const float sign = t & 1 ? -1.0f : 1.0f;
+    scale2.x *= sign, scale2.y *= sign, inv2.x *= sign, inv2.y *= sign;  // minus the quotient, and rounded alike, where the sign is
     float2 minus_scale2 = make_float2(-scale2.x, -scale2.y);
     bool divide = !PER_TOKEN && (needs_division(scale2.x) || needs_division(scale2.y));
     // row (16-key chunk, channel) of the image, this thread's KEYS bytes of it, eight keys at a time
@@ -304,7 +307,7 @@ __device__ __forceinline__ void v_int8_emit(const __nv_bfloat16 (*tile)[HEAD_DIM
                 x = make_float2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u));
             }
             if (PER_TOKEN) {
-                const float s = key_scale[key], inv = key_inv[key];
+                const float s = sign * key_scale[key], inv = sign * key_inv[key];
                 scale2 = make_float2(s, s), inv2 = make_float2(inv, inv), minus_scale2 = make_float2(-s, -s);
                 divide = needs_division(s);
             }
