@@ -4,7 +4,10 @@
 2. quantize_int8 and quantize_fp4_rows with rope= are, bit for bit, the quantization of rope(x) - mean;
 3. attention(q, k, v, rope=table) is the emulation on the rotated q and k, for every preset, one table for the batch
    or one per batch item;
-4. the compact table is kept while the same table comes back, also under torch.inference_mode."""
+4. the compact table is kept while the same table comes back, also under torch.inference_mode, and is safe to use from other
+   threads and streams."""
+
+import weakref
 
 import numpy as np
 import pytest
@@ -135,3 +138,62 @@ def test_table_checks_and_cache():
     a = unica.compact_rope(changed)
     changed[:, 0] = changed[:, 1]
     assert unica.compact_rope(changed) is not a  # modified in place: converted again
+
+
+def tables(count):
+    """Different tables of the same size."""
+    return [torch.from_numpy(oracle.wan_rope_table(T, H, W)).roll(i, 1).cuda() for i in range(count)]
+
+
+def test_a_table_replaced_during_a_call_stays_until_the_launch(monkeypatch):
+    import unicaattention_b200 as unica
+
+    q, k, v, _ = inputs()
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    mine, other = tables(2)
+    want = unica.attention(qd, kd, vd, rope=mine)
+    kept = weakref.ref(unica.compact_rope(mine))
+    launch = unica.lib.attention_call
+
+    def another_thread_comes_first(call):
+        unica.compact_rope(other)
+        assert kept() is not None, "the call's table was freed before its launch"
+        launch(call)
+
+    monkeypatch.setattr(unica.lib, "attention_call", another_thread_comes_first)
+    assert unica.attention(qd, kd, vd, rope=mine).equal(want)
+    unica.check_status()
+
+
+def test_tables_and_streams(monkeypatch):
+    import unicaattention_b200 as unica
+
+    q, k, v, _ = inputs()
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    mine, *others = tables(4)
+    want = unica.attention(qd, kd, vd, rope=mine.clone())
+    side, stack = torch.cuda.Stream(), torch.stack
+    side.wait_stream(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+
+    def slow_stack(*args, **kwargs):  # the conversion, 50 ms late
+        torch.cuda._sleep(100_000_000)
+        return stack(*args, **kwargs)
+
+    with monkeypatch.context() as patch:
+        patch.setattr(torch, "stack", slow_stack)
+        unica.compact_rope(mine)
+    converted = torch.cuda.current_stream().record_event()
+    with torch.cuda.stream(side):  # converted on another stream: waits for it
+        out = unica.attention(qd, kd, vd, rope=mine)
+    side.synchronize()
+    assert converted.query(), "the side stream did not wait for the conversion"
+    assert out.equal(want)
+    with torch.cuda.stream(side):  # replaced while the side stream has yet to read it: its memory must not go to the tables after it
+        torch.cuda._sleep(100_000_000)
+        out = unica.attention(qd, kd, vd, rope=mine)
+    for other in others:
+        unica.compact_rope(other)
+    torch.cuda.synchronize()
+    assert out.equal(want)
+    unica.check_status()

@@ -221,36 +221,51 @@ def rope_table(rope: torch.Tensor, batch: int, n_queries: int, n_keys: int) -> t
     return rope
 
 
-# The table compacted last: (weak reference to it, its version, the compact table).  The blocks of a sampling step share
-# one table, so it is converted once; a weak reference rather than an address, because the next step's table may be
-# given the old one's memory.
-_compact_rope: tuple = (lambda: None, -1, None)
+# The table compacted last: (weak reference to it, its version, the compact table, the stream it was converted on, an event there
+# after the conversion).  The blocks of a sampling step share one table, so it is converted once; a weak reference rather than an
+# address, because the next step's table may be given the old one's memory.
+_compact_rope: tuple = (lambda: None, -1, None, 0, None)
 
 
 def compact_rope(rope: torch.Tensor) -> torch.Tensor:
     """The table as the kernels read it: (cos, sin) per pair in fp16, [batch or 1, tokens, 64, 2].  The table must hold
-    rotations [[c, -s], [s, c]].  Kept while the same table object, unmodified, comes back."""
+    rotations [[c, -s], [s, c]].  Kept while the same table object, unmodified, comes back.  The current stream may read it: one
+    that it was not converted on waits for the conversion, and the table's memory, once replaced, for that stream."""
     global _compact_rope
     version = None if rope.is_inference() else rope._version  # inference tensors have no version counter
-    kept, kept_version, compact = _compact_rope
+    kept, kept_version, compact, home, converted = _compact_rope
     if kept() is rope and kept_version == version:
+        if converted is not None and torch._C._cuda_getCurrentRawStream(compact.device.index) != home:
+            stream = torch.cuda.current_stream(compact.device)
+            with torch.cuda.device(compact.device):
+                capturing = torch.cuda.is_current_stream_capturing()
+            if not capturing:  # a capture takes no event from outside it; what was queued before one began has been waited for
+                stream.wait_event(converted)
+                compact.record_stream(stream)
         return compact
     cos, sin = rope[..., 0, 0], rope[..., 1, 0]
     if not (torch.equal(rope[..., 1, 1], cos) and torch.equal(rope[..., 0, 1], -sin)):
         raise ValueError("rope must hold rotations [[cos, -sin], [sin, cos]], as WAN's table does")
     compact = torch.stack([cos, sin], -1)[:, :, 0].half().contiguous()
-    _compact_rope = (weakref.ref(rope), version, compact)
+    home, converted = 0, None
+    if compact.is_cuda:
+        stream = torch.cuda.current_stream(compact.device)
+        home, converted = stream.cuda_stream, stream.record_event()
+    _compact_rope = (weakref.ref(rope), version, compact, home, converted)
     return compact
 
 
 def rope_args(rope: torch.Tensor | None, x: torch.Tensor) -> tuple:
-    """The (table, batch stride) arguments of the *_rope entry points for x [batch, heads, tokens, 128]; () without rope."""
+    """The (table, batch stride) arguments of the *_rope entry points for x [batch, heads, tokens, 128]; () without rope.  The
+    table's pointer object holds the table: keep it until the launch is queued."""
     if rope is None:
         return ()
     compact = compact_rope(rope_table(rope, x.shape[0], x.shape[2], x.shape[2]))
     if compact.device != x.device:
         raise ValueError(f"rope is on {compact.device}, the tensors on {x.device}")
-    return lib.ptr(compact), compact.stride(0) if compact.shape[0] > 1 else 0
+    table = lib.ptr(compact)
+    table.owner = compact  # another thread's call may replace the kept table at any time
+    return table, compact.stride(0) if compact.shape[0] > 1 else 0
 
 
 # ----------------------------------------------------------------------------------------------------------------------
@@ -540,14 +555,12 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
         v_mode, outliers = lib.V_OUTLIERS, settings["V_OUTLIERS"]
         if n_keys > lib.CALL_TOKENS or not 0 < outliers <= MAX_OUTLIERS:
             return False
-    table, table_stride = (0, 0) if rope is None else rope_args(rope, q)
-    if rope is not None:
-        table = table.value
+    table, table_stride = (None, 0) if rope is None else rope_args(rope, q)
     half, device = int(q.dtype is torch.float16), q.device
     qs, ks, vs, os_ = q.stride(), k.stride(), v.stride(), out.stride()
     layouts = (qs[0], qs[1], qs[2], heads, half, ks[0], ks[1], ks[2], heads, half, vs[0], vs[1], vs[2], heads, half, os_[0], os_[1], os_[2], heads, half)
     sizes = (batch * heads, n_queries, n_keys, int(fast), v_mode, outliers, smooth if fast else 0)
-    where = (table, table_stride, 0 if peers is None else ctypes.addressof(peers), status_word(device).data_ptr(),
+    where = (0 if table is None else table.value, table_stride, 0 if peers is None else ctypes.addressof(peers), status_word(device).data_ptr(),
              torch._C._cuda_getCurrentRawStream(device.index))
     scale = SCALE_LOG2
     key = (*sizes, rope is None)
