@@ -286,7 +286,7 @@ int unica_b200_peak(int kind, int n, int count, int blocks, double* cycles_per_i
  * bit those of the single steps in the order of unica/__init__.py:288-356.  kernel: UNICA_B200_ACCURATE (v_mode,
  * n_outliers for UNICA_B200_V_OUTLIERS, which is limited to 8192 keys here) or UNICA_B200_FAST (smooth_q: 0 or a multiple of
  * 256).  rope: a (cos, sin) table as the _rope entry points take it, or NULL.  peer_out, n_peers: as in the _peers entry
- * points.  launches: how many kernels were queued. */
+ * points.  q, k, v and out may differ in element type (their layouts' dtype).  launches: how many kernels were queued. */
 #define UNICA_B200_ACCURATE 0
 #define UNICA_B200_FAST 1
 typedef struct {

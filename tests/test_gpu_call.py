@@ -92,3 +92,29 @@ def test_many_short_heads_equal_the_same_heads_alone(keys, preset, rotated):
     for head in (0, 17, 47):
         alone = unica.attention(*(x[:, head:head + 1] for x in (q, k, v)), **settings)
         assert torch.equal(alone, out[:, head:head + 1]), (keys, preset, head)
+
+
+@pytest.mark.parametrize("preset", PRESETS)
+@pytest.mark.parametrize("halves", ["k", "v", "qv", "k out"])
+@pytest.mark.parametrize("keys", [300, 8192])
+def test_each_tensor_by_its_own_element_type(keys, halves, preset):
+    """The C entry point with float16 and bfloat16 mixed: a float16 tensor counts as its rounding to bfloat16."""
+    import ctypes
+
+    import unicaattention_b200 as unica
+
+    q, k, v = (x.cuda() for x in qkv(1, 2, 300, keys, seed=keys))
+    q, k, v = (x.half() if name in halves.split()[0] else x for name, x in zip("qkv", (q, k, v)))
+    want = unica.attention(*(x.bfloat16() for x in (q, k, v)), **unica.PRESETS[preset])
+    out = torch.empty_like(want, dtype=torch.float16 if "out" in halves else torch.bfloat16)
+    settings = unica.TILE | unica.PRESETS[preset]
+    mode = 1 if settings["V_TOKEN"] else 2 if settings["V_OUTLIERS"] else 0
+    layouts = [n for x in (q, k, v, out) for n in (*x.stride()[:3], 2, int(x.dtype == torch.float16))]
+    where = (0, 0, 0, unica.status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    sizes = (2, 300, keys, int(preset == "fast"), mode, settings["V_OUTLIERS"], settings["SMOOTH_Q"], 0, unica.SCALE_LOG2)
+    size = unica.lib.attention_workspace(unica.lib.pack_call(0, 0, 0, 0, 0, 0, *where, *layouts, *sizes))
+    workspace, queued = torch.empty(size, dtype=torch.uint8, device="cuda"), ctypes.c_int()
+    pointers = [x.data_ptr() for x in (q, k, v, out, workspace)]
+    assert unica.lib.library().unica_b200_attention_call(unica.lib.pack_call(*pointers, size, *where, *layouts, *sizes), ctypes.byref(queued)) == 0
+    unica.check_status()
+    assert out.equal(want.to(out.dtype)) and queued.value >= 2

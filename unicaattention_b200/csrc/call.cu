@@ -90,8 +90,7 @@ int call_accurate(const unica_b200_call& c, const Plan& p, int* launches) {
         quantize.v = operand(c.v, c.v_layout, c.n_keys, p.k_tiles, p.v8, p.v_scale, nullptr, nullptr);
     }
     if (p.short_q || p.short_k) {
-        if (int e = quantize_call_int8(quantize, static_cast<cudaStream_t>(c.stream))) return e;
-        ++*launches;
+        if (int e = quantize_call_int8(quantize, static_cast<cudaStream_t>(c.stream), launches)) return e;
     }
     if (!p.short_q) {
         if (int e = c.rope ? unica_b200_quantize_int8_rope(c.q, c.q_layout, nullptr, c.rope, c.rope_batch_stride, c.heads, c.n_queries, QUERY_TILE, p.q_tiles, p.q8,

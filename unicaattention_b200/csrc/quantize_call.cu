@@ -357,9 +357,10 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
 // max |x - mean| of the block's values -> the outer scale of all: see nvfp4_outer_rows_kernel
 __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (1.0f / 2688.0f), 1e-30f); }
 
-// Clusters: heads of K, of V, of Q.  Rotated inputs keep twice the loads in flight: with three blocks per SM their registers
+// HALF: the inputs are float16 (1) or bfloat16 (0), or each what its layout says.  Clusters: heads of K, of V, of Q.  Rotated inputs keep twice the loads in flight: with three blocks per SM their registers
 // spilled (2 x 16 heads x 777 tokens: 49 us, with two 42 us).
-template <bool HALF, bool ROPE, int CLUSTER>
+constexpr int EACH_ITS_OWN = 2;
+template <int HALF, bool ROPE, int CLUSTER>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     let_next_kernel_start();
     __shared__ CallStats sm;
@@ -370,7 +371,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     if (kind == 0) {
         const CallOperand& op = call.k;
         TokenLayout in = op.in;
-        in.half = HALF;
+        if (HALF != EACH_ITS_OWN) in.half = HALF;
         head_stats<true, true, CLUSTER>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
@@ -388,7 +389,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     } else if (kind == 1) {
         const CallOperand& op = call.v;
         TokenLayout in = op.in;
-        in.half = HALF;
+        if (HALF != EACH_ITS_OWN) in.half = HALF;
         head_stats<false, true, CLUSTER>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
         each_tile<VRaw>(
             share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, op.x, in, head, t, op.n_tokens); },
@@ -401,7 +402,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         // Q: a mean per group of `smooth` tokens, whole groups per block
         const CallOperand& op = call.q;
         TokenLayout in = op.in;
-        in.half = HALF;
+        if (HALF != EACH_ITS_OWN) in.half = HALF;
         const int groups = (op.n_tokens + call.smooth - 1) / call.smooth, per = call.smooth / CALL_BLOCK, blocks = (op.n_tokens + CALL_BLOCK - 1) / CALL_BLOCK;
         float amax = 0.0f;
         for (int g = share<CLUSTER>(groups, rank); g < share<CLUSTER>(groups, rank + 1); ++g) {
@@ -441,8 +442,24 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     cg::this_cluster().sync();
 }
 
-int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
+int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launches) {
     if (int e = unica_check_device()) return e;
+    const CallOperand* operands[] = {&call.q, &call.k, &call.v};
+    const CallOperand* first = nullptr;
+    for (const CallOperand* op : operands) {
+        if (!op->x) continue;
+        if (!first) first = op;
+        if (op->in.half == first->in.half) continue;
+        for (const CallOperand* alone : operands) {  // element types differ: the kernel has one, so each operand alone
+            if (!alone->x) continue;
+            CallQuantize one = call;
+            if (alone != &call.q) one.q = {};
+            if (alone != &call.k) one.k = {};
+            if (alone != &call.v) one.v = {};
+            if (int e = quantize_call_int8(one, stream, launches)) return e;
+        }
+        return UNICA_B200_OK;
+    }
     const long long q_tiles = call.q.x ? static_cast<long long>(call.heads) * call.q.tiles : 0, kv_heads = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0);
     // as in quantize_call_fp4: 32 heads x 777 50.6 -> 43.3 us a call, 40 x 1024 70.5 -> 62; the tiles of Q fill gaps, and where only
     // they make a second wave (24 x 1000) four blocks per head were 2 us slower
@@ -462,7 +479,8 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream) {
                                                                   : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, CALL_CLUSTER>);
         kernel<<<grid, CALL_THREADS, 0, stream>>>(call);
     };
-    const bool half = (call.q.x ? call.q : call.k.x ? call.k : call.v).in.half;
+    const bool half = first->in.half;
+    if (launches) ++*launches;
     call.rope.table ? (half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))
                     : (half ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{}));
     return unica_check_launch("quantize_call_int8");
@@ -477,8 +495,10 @@ int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     const bool four = longest <= 4 * CALL_BLOCK && 3 * call.heads * CALL_CLUSTER > 148 * (call.rope.table ? 2 : 3);
     auto launch = [&](auto half, auto rope) {
         constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
-        const int cluster = four ? 4 : CALL_CLUSTER;
-        auto kernel = four ? quantize_call_fp4_kernel<HALF, ROPE, 4> : quantize_call_fp4_kernel<HALF, ROPE, CALL_CLUSTER>;
+        const bool mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
+        const int cluster = four && !mixed ? 4 : CALL_CLUSTER;
+        auto kernel = mixed ? quantize_call_fp4_kernel<EACH_ITS_OWN, ROPE, CALL_CLUSTER>
+                      : four ? quantize_call_fp4_kernel<HALF, ROPE, 4> : quantize_call_fp4_kernel<HALF, ROPE, CALL_CLUSTER>;
         kernel<<<dim3(3u * call.heads * cluster), CALL_THREADS, 0, stream>>>(call);
     };
     call.rope.table ? (call.q.in.half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))

@@ -31,7 +31,8 @@ struct CallQuantize {
     float* outlier_rows;  // [heads][n_outliers][128]
     int smooth;          // NVFP4: tokens per group of Q's means, a multiple of 256
 };
-int quantize_call_int8(const CallQuantize& call, cudaStream_t stream);
+// launches: counts them, or null
+int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launches = nullptr);
 int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream);
 
 }  // namespace unica
