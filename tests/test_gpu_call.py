@@ -118,3 +118,22 @@ def test_each_tensor_by_its_own_element_type(keys, halves, preset):
     assert unica.lib.library().unica_b200_attention_call(unica.lib.pack_call(*pointers, size, *where, *layouts, *sizes), ctypes.byref(queued)) == 0
     unica.check_status()
     assert out.equal(want.to(out.dtype)) and queued.value >= 2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("tokens", [100, 8192, 8200])
+def test_outlier_keys_that_are_not_numbers(tokens, value, dtype):
+    """A key with a NaN or an infinity is an outlier before every finite one, at any length, and shows in the output."""
+    import unicaattention_b200 as unica
+
+    q, k, v = (x.to(dtype).cuda() for x in qkv(1, 2, 64, tokens, seed=tokens))
+    bad, large = tokens // 3, tokens - 1
+    v[:, :, large] *= 50
+    v[:, 1, bad, 77] = value
+    _, _, keys, rows = unica.quantize_v(v, outliers=8)
+    assert torch.equal(keys.long().sort(-1).values, unica.v_outliers(v, 8).sort(-1).values)
+    assert bad in keys[0, 1] and large in keys[0, 1] and bad not in keys[0, 0]
+    out = unica.attention(q, k, v, **unica.PRESETS["outliers"])
+    unica.check_status()
+    assert not out[:, 1, :, 77].isfinite().any() and out[:, 1, :, :77].isfinite().all() and out[:, 0].isfinite().all()

@@ -167,8 +167,8 @@ __device__ __forceinline__ void head_stats(const __nv_bfloat16* __restrict__ x, 
     __syncthreads();
 }
 
-// The n_outliers keys with the largest max |v| of the head, ties to the lower key (what the reference's emulation takes), in
-// every block of the cluster: -1 where the head has fewer keys.  Every warp picks the largest of an eighth of the block's
+// The n_outliers keys with the largest max |v| of the head, ties to the lower key (what the reference's emulation takes), NaN above
+// all numbers (as torch's topk has it), in every block of the cluster: -1 where the head has fewer keys.  Every warp picks the largest of an eighth of the block's
 // tokens, then one warp per block picks among all blocks' picks.
 constexpr int CALL_WARPS = CALL_THREADS / 32, CALL_PICKS = CALL_WARPS * CALL_OUTLIERS;
 struct CallOutliers {
@@ -213,12 +213,12 @@ __device__ __forceinline__ void find_outliers(const __nv_bfloat16* __restrict__ 
         for (int j = 0; j < 8; ++j) {
             const int i = i0 + j * CALL_LANES + lane;
             const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
-            const __nv_bfloat162 top = __hmax2(__hmax2(__habs2(pairs[0]), __habs2(pairs[1])), __hmax2(__habs2(pairs[2]), __habs2(pairs[3])));
+            const __nv_bfloat162 top = __hmax2_nan(__hmax2_nan(__habs2(pairs[0]), __habs2(pairs[1])), __hmax2_nan(__habs2(pairs[2]), __habs2(pairs[3])));
             const float2 two = __bfloat1622float2(top);
-            float amax = fmaxf(two.x, two.y);
+            unsigned amax = max(__float_as_uint(two.x), __float_as_uint(two.y));  // (the bits of non-negative floats are in their order)
 #pragma unroll
-            for (int d = 8; d > 0; d /= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-            if (chunk == 0 && i < count) candidates[i] = (static_cast<unsigned long long>(__float_as_uint(amax)) << 32) | (0xffffffffu - unsigned(t0 + i));
+            for (int d = 8; d > 0; d /= 2) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+            if (chunk == 0 && i < count) candidates[i] = (static_cast<unsigned long long>(amax) << 32) | (0xffffffffu - unsigned(t0 + i));
         }
     }
     __syncthreads();
