@@ -87,16 +87,21 @@ __global__ void __launch_bounds__(HEAD_DIM) channel_stats_finish_kernel(const fl
     high[o] = hi;
 }
 
-// One block per tile.  Grid (tiles, heads).
-template <int ROWS>
+// One block per tile.  ONCE: see rows_int8_tile_once.  Grid (tiles, heads).
+template <int ROWS, bool ONCE>
 __global__ void __launch_bounds__(THREADS) quantize_rows_int8_kernel(const __nv_bfloat16* __restrict__ x, TokenLayout in,
                                                                       const float* __restrict__ mean, int n_tokens,
                                                                       int8_t* __restrict__ codes, float* __restrict__ scales,
                                                                       RopeTable rope) {
     __shared__ float scratch[THREADS / 32];
     const int head = blockIdx.y, tile = blockIdx.x;
-    rows_int8_tile<ROWS>(x, in, mean ? mean + head * HEAD_DIM : nullptr, head, tile, n_tokens,
-                         codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM), scales + size_t(head) * gridDim.x + tile, rope, scratch);
+    const float* mu = mean ? mean + head * HEAD_DIM : nullptr;
+    int8_t* out = codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM);
+    float* scale = scales + size_t(head) * gridDim.x + tile;
+    if (ONCE)
+        rows_int8_tile_once<ROWS>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
+    else
+        rows_int8_tile<ROWS>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
 }
 
 template <bool PER_TOKEN>
@@ -232,10 +237,8 @@ static int quantize_int8(const void* x, unica_token_layout layout, const float* 
     if (tiles < (n_tokens + block_tokens - 1) / block_tokens) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_int8: tiles does not cover n_tokens");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
-    if (block_tokens == 128)
-        quantize_rows_int8_kernel<128><<<dim3(tiles, heads), THREADS, 0, s>>>(xb, to_layout(layout), mean, n_tokens, codes, scales, rope);
-    else
-        quantize_rows_int8_kernel<64><<<dim3(tiles, heads), THREADS, 0, s>>>(xb, to_layout(layout), mean, n_tokens, codes, scales, rope);
+    auto kernel = block_tokens == 128 ? quantize_rows_int8_kernel<128, false> : rope.table ? quantize_rows_int8_kernel<64, true> : quantize_rows_int8_kernel<64, false>;
+    kernel<<<dim3(tiles, heads), THREADS, 0, s>>>(xb, to_layout(layout), mean, n_tokens, codes, scales, rope);
     return unica_check_launch("quantize_int8");
 }
 

@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 2) quantize_q_int8_stream_kern
         ring_wait();  // all but the two newest groups: both halves of this tile are there
         __syncthreads();
         const int tile = int(blockIdx.x) + i * int(gridDim.x), head = tile / tiles, t = tile - head * tiles;
-        rows_int8_tile_raw<128, STREAM_THREADS>(x, in, head, t, n_tokens, codes + size_t(tile) * (128 * HEAD_DIM), scales + tile, scratch_max,
-                                                reinterpret_cast<const __nv_bfloat16*>(ring + (2 * i % RING_STAGES) * RING_TILE_BYTES));
+        rows_int8_tile_once<128, STREAM_THREADS>(x, in, nullptr, head, t, n_tokens, codes + size_t(tile) * (128 * HEAD_DIM), scales + tile, RopeTable{nullptr, 0},
+                                                 scratch_max, reinterpret_cast<const __nv_bfloat16*>(ring + (2 * i % RING_STAGES) * RING_TILE_BYTES));
         __syncthreads();  // its two stages are free
         fetch();
         fetch();
