@@ -121,11 +121,13 @@ int unica_b200_quantize_q_int8_stream(const void* q, unica_token_layout layout, 
 /* Statistics and quantization of K in one launch: what unica_b200_channel_stats (per = 0) followed by
  * unica_b200_quantize_int8 (block_tokens 64, mean = the statistics' mean) do (csrc/flash.cu:287-372; unica/__init__.py:
  * 363-378, 592-612), with the second read of K served by L2 instead of HBM.  codes, scales as unica_b200_quantize_int8
- * writes them, tiles = ceil(n_tokens / 64); mean [heads][128] is written too (the order in which its terms are added
- * differs from unica_b200_channel_stats', so its last bit can; it is fixed for a device and a token count).
+ * writes them, tiles = ceil(n_tokens / 64); mean [heads][128] is written too (its terms are added in the order of
+ * unica_b200_channel_stats up to 8192 tokens, in another above, so that its last bit can differ; the order is fixed for a device
+ * and a token count).
  * scratch: UNICA_B200_FUSED_SCRATCH_BYTES of device memory, 16-byte aligned, that no other call uses at the same time;
  * its contents do not matter.  status: as for the attention kernels (a block that never sees its group's statistics
- * gives up after about a second and leaves STATUS 8 there), or NULL.  A cooperative launch of persistent blocks. */
+ * gives up after about a second and leaves STATUS 8 there), or NULL.  A cooperative launch of persistent blocks; up to 8192
+ * tokens a launch of clusters, and for few heads of these the single steps. */
 #define UNICA_B200_FUSED_SCRATCH_BYTES (2u << 20)
 int unica_b200_quantize_k_int8_fused(const void* k, unica_token_layout layout, int heads, int n_tokens, int tiles, void* scratch,
                                      size_t scratch_bytes, int8_t* codes, float* scales, float* mean, int* status, void* stream);

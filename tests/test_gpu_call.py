@@ -63,10 +63,11 @@ def test_short_operands_equal_the_separate_passes(tokens):
     unica.check_status()
 
 
-@pytest.mark.parametrize("heads", [55, 60, 112])
-@pytest.mark.parametrize("tokens", [1024, 1025, 4128, 8192])
-def test_short_operands_of_many_heads(tokens, heads):
-    """K alone and V alone, with and without enough heads for clusters of four blocks, which have room for 4096 tokens."""
+@pytest.mark.parametrize("heads", [8, 9, 55, 60, 112])
+@pytest.mark.parametrize("tokens", [1024, 1025, 2048, 2049, 4128, 8192])
+def test_short_operands_alone(tokens, heads):
+    """K alone and V alone: few heads, which go through the single steps above 2048 tokens, and with and without enough heads for
+    clusters of four blocks, which have room for 4096 tokens."""
     import unicaattention_b200 as unica
 
     x = (torch.randn(1, heads, tokens, 128, generator=torch.Generator("cuda").manual_seed(tokens), device="cuda") + 0.5).bfloat16()

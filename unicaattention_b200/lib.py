@@ -109,7 +109,9 @@ def stream() -> ctypes.c_void_p:
 # kernels an entry point launches when it succeeds (the statistics passes: partial sums, then their reduction)
 KERNELS_PER_CALL = {"unica_b200_channel_stats": 2, "unica_b200_channel_stats_rope": 2, "unica_b200_channel_stats_masked": 2,
                     "unica_b200_channel_stats_static": 2, "unica_b200_version": 0, "unica_b200_attention_workspace": 0}
-launches = 0  # kernels of this library launched by this process so far (benchmarks report differences of it)
+# Kernels of this library launched by this process so far (benchmarks report differences of it).  The one-launch quantizers of K or V
+# alone count as one, also for the few heads they take through the single steps.
+launches = 0
 
 
 def attention_workspace(call_bytes: bytes) -> int:
