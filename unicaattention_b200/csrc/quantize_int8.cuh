@@ -168,7 +168,7 @@ __device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__
 }
 
 // The same with each item converted as it is loaded.  The faster form for rotated tiles of 64 rows (40 heads x 32760 tokens: 218.8
-// -> 212.4 us; of 128 rows 203 -> 221), and for Q's tiles staged in shared memory, where nothing has to be under way (107.8 -> 104.5).
+// -> 212.4 us; of 128 rows 203 -> 221) and short ones (see quantize_int8 in quantize.cu), and for Q's tiles staged in shared memory, where nothing has to be under way (107.8 -> 104.5).
 template <int ROWS, int NT = THREADS>
 __device__ __forceinline__ void rows_int8_tile_once(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const float* mean, int head, int tile,
                                                     int n_tokens, int8_t* __restrict__ out, float* __restrict__ scale_out, const RopeTable& rope,
