@@ -84,7 +84,8 @@ struct __align__(128) Fp4Smem {
     // seen the first of two phases must not take a look for the second for an answer.)
     uint64_t q_full[2], k_full[F4_K_RING], v_full[F4_V_RING], s_full[F4_TILES][2], pv_done[F4_TILES][2], drain[1 + F4_TILES];
     uint32_t tmem_base;
-    int abort_flag, never;  // never: stays 0, for waits that nothing may cut short
+    int abort_flag;
+    int alone[2 + F4_TILES];  // zeros: a word for each warp that drains what it issued, which no other warp's wait may cut short
 };
 static_assert(sizeof(Fp4Smem) + 128 <= 227 * 1024, "the block's shared memory");
 
@@ -226,7 +227,7 @@ __device__ __forceinline__ void f4_scores_warp(Fp4Smem& sm, const Fp4Args& a, in
 #pragma unroll
     for (int i = 0; i < F4_TILES; ++i) f4_s_free_sync(i);
     commit_elected(&sm.drain[0]);  // whatever was issued must finish before tensor memory is freed
-    mbar_wait_line(&sm.drain[0], 0, &sm.never, nullptr, 0);
+    mbar_wait_line(&sm.drain[0], 0, &sm.alone[0], nullptr, 0);
     __syncwarp();
 }
 
@@ -301,11 +302,12 @@ __device__ __forceinline__ void f4_copy_warp(Fp4Smem& sm, const Fp4Args& a, int 
         if (t == 0 && n >= 1 && n + 1 < n_items) copy_q(n + 1);
         if (++t == k_tiles) t = 0, ++n;
     }
-    // After a wait that gave up, copies may still be in flight: the block's shared memory must not go away under them.
+    // After a wait that gave up, copies may still be in flight: the block's shared memory must not go away under them.  (Should
+    // the first of these waits give up too, the others have been in flight all the while.)
     if (__any_sync(0xffffffffu, *static_cast<volatile int*>(&sm.abort_flag))) {
-        for (int i = max(0, total - F4_V_RING); i < total; ++i) mbar_wait_line(&sm.v_full[slot<F4_V_RING>(i)], round_parity<F4_V_RING>(i), &sm.never, nullptr, 0);
-        for (int i = max(0, total - F4_K_RING); i < total; ++i) mbar_wait_line(&sm.k_full[slot<F4_K_RING>(i)], round_parity<F4_K_RING>(i), &sm.never, nullptr, 0);
-        for (int i = max(0, n_items - 2); i < n_items; ++i) mbar_wait_line(&sm.q_full[slot<2>(i)], round_parity<2>(i), &sm.never, nullptr, 0);
+        for (int i = max(0, total - F4_V_RING); i < total; ++i) mbar_wait_line(&sm.v_full[slot<F4_V_RING>(i)], round_parity<F4_V_RING>(i), &sm.alone[1], nullptr, 0);
+        for (int i = max(0, total - F4_K_RING); i < total; ++i) mbar_wait_line(&sm.k_full[slot<F4_K_RING>(i)], round_parity<F4_K_RING>(i), &sm.alone[1], nullptr, 0);
+        for (int i = max(0, n_items - 2); i < n_items; ++i) mbar_wait_line(&sm.q_full[slot<2>(i)], round_parity<2>(i), &sm.alone[1], nullptr, 0);
     }
     __syncwarp();
 }
@@ -329,7 +331,7 @@ __device__ __forceinline__ void f4_pv_warp(Fp4Smem& sm, const Fp4Args& a, int k_
         if (++t == k_tiles) t = 0;
     }
     commit_elected(&sm.drain[1 + i]);
-    mbar_wait_line(&sm.drain[1 + i], 0, &sm.never, nullptr, 0);
+    mbar_wait_line(&sm.drain[1 + i], 0, &sm.alone[2 + i], nullptr, 0);
     __syncwarp();
 }
 
@@ -519,7 +521,8 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
     const int k_tiles = (a.n_keys + KEY_TILE - 1) / KEY_TILE;
 
     if (threadIdx.x == 0) {
-        sm.abort_flag = sm.never = 0;
+        sm.abort_flag = 0;
+        for (int& word : sm.alone) word = 0;
         for (int s = 0; s < 2; ++s) mbar_init(&sm.q_full[s], 1);
         for (int s = 0; s < F4_K_RING; ++s) mbar_init(&sm.k_full[s], 1);
         for (int s = 0; s < F4_V_RING; ++s) mbar_init(&sm.v_full[s], 1);

@@ -85,7 +85,8 @@ struct __align__(128) AttSmem {
     float tok[V_RING][2 * KEY_TILE];
     uint64_t q_full[2], q_free[2], k_full[K_RING], v_full[V_RING], s_full[S_RING], acc_full[2], drain[2];
     uint32_t tmem_base;
-    int abort_flag, never;  // never: stays 0, for waits that nothing may cut short
+    int abort_flag;
+    int alone[2];  // zeros: a word for each warp that drains what it issued, which no other warp's wait may cut short
 };
 static_assert(sizeof(AttSmem) + 128 <= 227 * 1024, "the block's shared memory");
 
@@ -272,12 +273,13 @@ __device__ __forceinline__ void scores_warp(AttSmem& sm, const AttArgs& a, int k
         if (b < v_later && total + b >= v_later) copy_v();
     }
     commit_elected(&sm.drain[0]);  // whatever was issued must finish before tensor memory is freed
-    mbar_wait_line(&sm.drain[0], 0, &sm.never, nullptr, 0);
-    // After a wait that gave up, copies may still be in flight: the block's shared memory must not go away under them.
+    mbar_wait_line(&sm.drain[0], 0, &sm.alone[0], nullptr, 0);
+    // After a wait that gave up, copies may still be in flight: the block's shared memory must not go away under them.  (Should
+    // the first of these waits give up too, the others have been in flight all the while.)
     if (__any_sync(0xffffffffu, *static_cast<volatile int*>(&sm.abort_flag))) {
-        for (int i = max(0, total - V_RING); i < total; ++i) mbar_wait_line(&sm.v_full[slot<V_RING>(i)], round_parity<V_RING>(i), &sm.never, nullptr, 0);
-        for (int i = max(0, total - K_RING); i < total; ++i) mbar_wait_line(&sm.k_full[i % K_RING], (i / K_RING) & 1, &sm.never, nullptr, 0);
-        for (int i = max(0, n_items - 2); i < n_items; ++i) mbar_wait_line(&sm.q_full[slot<2>(i)], round_parity<2>(i), &sm.never, nullptr, 0);
+        for (int i = max(0, total - V_RING); i < total; ++i) mbar_wait_line(&sm.v_full[slot<V_RING>(i)], round_parity<V_RING>(i), &sm.alone[0], nullptr, 0);
+        for (int i = max(0, total - K_RING); i < total; ++i) mbar_wait_line(&sm.k_full[i % K_RING], (i / K_RING) & 1, &sm.alone[0], nullptr, 0);
+        for (int i = max(0, n_items - 2); i < n_items; ++i) mbar_wait_line(&sm.q_full[slot<2>(i)], round_parity<2>(i), &sm.alone[0], nullptr, 0);
     }
     __syncwarp();
 }
@@ -296,7 +298,7 @@ __device__ __forceinline__ void pv_warp(AttSmem& sm, const AttArgs& a, int k_til
                  &sm.acc_full[slot<2>(g)]);
     }
     commit_elected(&sm.drain[1]);
-    mbar_wait_line(&sm.drain[1], 0, &sm.never, nullptr, 0);
+    mbar_wait_line(&sm.drain[1], 0, &sm.alone[1], nullptr, 0);
     __syncwarp();
 }
 
@@ -646,7 +648,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_int8_kernel(const __
     const int k_tiles = (a.n_keys + KEY_TILE - 1) / KEY_TILE;
 
     if (threadIdx.x == 0) {
-        sm.abort_flag = sm.never = 0;
+        sm.abort_flag = 0;
+        for (int& word : sm.alone) word = 0;
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sm.q_full[s], 1), mbar_init(&sm.q_free[s], 5);  // the scores' instructions and the four flush warps
             mbar_init(&sm.acc_full[s], 1);

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
         if (ok) ++seen[1], write_out(last, turn - 1);
     }
     if (!ok && threadIdx.x == 0) {  // whatever was issued must finish before tensor memory is freed
-        int never = 0;
+        int never = 0;  // (one word for both: the second half has been in flight all the while)
         for (int half = 0; half < 2; ++half)
             if (sent[half] > seen[half]) mbar_wait(&sm.done[half], (sent[half] - 1) & 1, &never, nullptr, 0);
     }
