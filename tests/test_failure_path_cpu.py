@@ -19,3 +19,13 @@ def test_no_two_warps_drain_on_one_word(name, warps):
             words[role] = used
     assert len(words) == warps and all(len(used) == 1 for used in words.values()), words
     assert len(set.union(*words.values())) == warps and not any("abort_flag" in word for used in words.values() for word in used), words
+
+
+@pytest.mark.parametrize("name", ["attention_int8.cu", "attention_fp4.cu"])
+def test_rows_are_sent_only_if_no_warp_gave_up(name):
+    """The warps that store rows see their own waits only: another's, which went on with whatever lay in its buffers, is in the word
+    that all share."""
+    source = (CSRC / name).read_text()
+    before, _, _ = source.partition("send_staged_rows(")
+    last = before[before.rindex("ok = __all_sync("):].partition(";")[0]
+    assert "gave_up(sm.abort_flag)" in last, last

@@ -69,6 +69,14 @@ __device__ __forceinline__ void copy_elected(void* dst, const void* src, int byt
         : "memory");
 }
 
+// Has a wait of any warp of the block given up?  Asked before an item's rows are stored: the warps that store them see their own waits
+// only, and one that gave up goes on with whatever lies in its buffers.
+__device__ __forceinline__ bool gave_up(const int& abort_flag) {
+    int word;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(word) : "r"(smem_u32(&abort_flag)) : "memory");
+    return word != 0;
+}
+
 // Output rows out through shared memory: each lane of a warp has written its row (256 bytes, STAGED_PITCH apart) and one bulk copy
 // per row takes it to the caller's tensor.  bulk_store_read_wait() before the rows are written again.
 constexpr int STAGED_PITCH = HEAD_DIM * 2 + 16;  // bytes from one staged output row to the next: rows of a quarter-warp on different banks

@@ -470,7 +470,7 @@ __device__ __forceinline__ void f4_softmax(Fp4Smem& sm, const Fp4Args& a, int k_
 
         if (t + 1 == k_tiles) {  // the item is done: its rows out
             ok &= mbar_wait_line(&sm.pv_done[qt][w], turn & 1, &sm.abort_flag, a.status, STATUS_WAIT_PV);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = __all_sync(0xffffffffu, ok && !gave_up(sm.abort_flag));
             tc_fence_after();
             if (n > 0 && ((g - k_tiles) & 1) != w) f4_staged_sync(qt);  // the item before was stored by the other warpgroup
             bulk_store_read_wait();

@@ -617,7 +617,7 @@ __device__ __forceinline__ void flush_warps(AttSmem& sm, const AttArgs& a, int k
 
         const int head = a.items.head(item), q_tile = a.items.tile(item);
         ok &= mbar_wait_line(&sm.q_full[slot<2>(i)], round_parity<2>(i), &sm.abort_flag, a.status, STATUS_WAIT_TILE);  // V's channel scales came with Q8
-        ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, ok && !gave_up(sm.abort_flag));
         bulk_store_read_wait();  // the item before has left the staging rows
         if constexpr (OUTLIERS) {
             add_outliers(sm, a, k_tiles, head, q_tile, slot<2>(i), row, m, o);
