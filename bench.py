@@ -427,7 +427,7 @@ class Bench:
             # tokens (every K/V tile comes from HBM once and is re-read from L2, so traffic grows with the token count)
             per_token_bytes = {"per_channel": 552.7, "fast": 441.9}.get(args.mode)
             head["roofline"]["traffic"] = per_token_bytes * batch * heads * tokens / self.world if per_token_bytes else None
-            head["roofline"]["traffic_unit"] = "bytes per launch per GPU, derived: ncu dram bytes of a 40 x 8192 capture scaled by heads x tokens"
+            head["roofline"]["traffic_unit"] = "bytes per launch per GPU, derived: ncu dram bytes of a 40 x 8192 capture of an earlier state of the kernel scaled by heads x tokens"
             line = {"metric": metric_name(args.mode, batch, heads, tokens), "value": head["value"], "unit": "TOPS", "n_gpus": self.world,
                     "steps": args.steps, "warmup": args.warmup, "ms_per_step": head["ms_per_step"], "higher_is_better": True,
                     "scaling": "strong", "vs_baseline": None, "dtype": dtype_of(args.mode), "data": "synthetic",

@@ -302,8 +302,8 @@ FUSED_SCRATCH_BYTES = 2 << 20  # include/unica_b200.h UNICA_B200_FUSED_SCRATCH_B
 @on_their_device
 def quantize_k(k: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """K's mean over the tokens taken away and the rest in INT8 with a scale per 64 keys, in one launch that reads K from
-    HBM once (unica_b200_quantize_k_int8_fused): what rope_stats(k)[0] and quantize_int8(k, mean, 64) give, except that
-    the mean's terms are added in another (fixed) order.  Returns codes, scales, mean [batch, heads, 128]."""
+    HBM once (unica_b200_quantize_k_int8_fused): what rope_stats(k)[0] and quantize_int8(k, mean, 64) give; above 8192
+    tokens the mean's terms are added in another (fixed) order.  Returns codes, scales, mean [batch, heads, 128]."""
     _check_input(k, "k")
     k = readable(k)
     batch, heads, n, _ = k.shape

@@ -33,7 +33,7 @@ def stale() -> bool:
 
 def build(force: bool = False, verbose: bool = False, defines: tuple[str, ...] = (), output: Path | None = None) -> Path:
     """Compile every .cu of csrc/ into objects (in build/) and link the shared library.  Returns its path.
-    defines: extra -D flags (e.g. ("UNICA_TRACE",)) for a diagnostic build written to `output` instead of LIB."""
+    defines: extra -D flags for a diagnostic build written to `output` instead of LIB."""
     if defines or output:
         return _build(HERE / "build" / ("-".join(defines) or "alt"), output or HERE / ("libunica_b200-" + "-".join(defines) + ".so"),
                       [f"-D{d}" for d in defines], verbose)
