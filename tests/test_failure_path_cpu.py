@@ -29,3 +29,9 @@ def test_rows_are_sent_only_if_no_warp_gave_up(name):
     before, _, _ = source.partition("send_staged_rows(")
     last = before[before.rindex("ok = __all_sync("):].partition(";")[0]
     assert "gave_up(sm.abort_flag)" in last, last
+
+
+def test_the_smoothing_kernel_has_its_tensor_memory_before_the_next_kernel_comes():
+    """An attention block takes all tensor memory of its SM and then waits for the kernel before it."""
+    body = (CSRC / "quantize_fp4.cu").read_text().partition("smooth_bias_kernel(")[2]
+    assert body.index("tmem_alloc(") < body.index("__syncthreads();") < body.index("let_next_kernel_start();") < body.index("wait_for_previous_kernel();")

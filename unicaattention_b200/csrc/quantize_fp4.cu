@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
     const int head = blockIdx.y, b0 = blockIdx.z * BIAS_BLOCKS, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int k_tiles = (n_keys + KEY_TILE - 1) / KEY_TILE, pairs = (k_tiles + 1) / 2;
     volatile int* abort_flag = &sm.abort_flag;
-    let_next_kernel_start();
     if (threadIdx.x == 0) {
         sm.abort_flag = 0;
         mbar_init(&sm.done[0], 1);
@@ -118,6 +117,10 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(&sm.tmem_base, 2 * BIAS_BLOCKS);
+    __syncthreads();
+    // Only now: a block of the attention kernel takes all tensor memory of its SM and then waits for this kernel, which could wait
+    // for tensor memory in turn.
+    let_next_kernel_start();
     wait_for_previous_kernel();
     // the means of this pass's query blocks, rows past the last block zero
     for (int item = threadIdx.x; item < BIAS_BLOCKS * (HEAD_DIM / 4); item += BIAS_THREADS) {
