@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(HEAD_DIM) channel_stats_finish_kernel(const fl
     high[o] = hi;
 }
 
-// One block per tile.  ONCE: see rows_int8_tile_once.  Grid (tiles, heads).
-template <int ROWS, bool ONCE>
+// One block per tile.  ONCE: see rows_int8_tile_once; BY_ROW: see RowsItem.  Grid (tiles, heads).
+template <int ROWS, bool ONCE, bool BY_ROW>
 __global__ void __launch_bounds__(THREADS) quantize_rows_int8_kernel(const __nv_bfloat16* __restrict__ x, TokenLayout in,
                                                                       const float* __restrict__ mean, int n_tokens,
                                                                       int8_t* __restrict__ codes, float* __restrict__ scales,
@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(THREADS) quantize_rows_int8_kernel(const __nv_
     int8_t* out = codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM);
     float* scale = scales + size_t(head) * gridDim.x + tile;
     if (ONCE)
-        rows_int8_tile_once<ROWS>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
+        rows_int8_tile_once<ROWS, THREADS, BY_ROW>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
     else
-        rows_int8_tile<ROWS>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
+        rows_int8_tile<ROWS, THREADS, BY_ROW>(x, in, mu, head, tile, n_tokens, out, scale, rope, scratch);
 }
 
 template <bool PER_TOKEN>
@@ -240,7 +240,9 @@ static int quantize_int8(const void* x, unica_token_layout layout, const float* 
     // Tiles of 64 rows in one pass where they are rotated, or come out of L2 (40 heads x 8192 tokens 42.8 -> 40.4 us, x 16384 78.0 ->
     // 75.7; x 32760 141 -> 144, 4 x 118320 47.7 -> 52.3)
     const bool once = block_tokens == 64 && (rope.table || (n_tokens <= 32768 && static_cast<long long>(heads) * n_tokens <= 1 << 20));
-    auto kernel = block_tokens == 128 ? quantize_rows_int8_kernel<128, false> : once ? quantize_rows_int8_kernel<64, true> : quantize_rows_int8_kernel<64, false>;
+    auto kernel = rope.table ? (block_tokens == 128 ? quantize_rows_int8_kernel<128, false, true> : quantize_rows_int8_kernel<64, true, true>)
+                  : block_tokens == 128 ? quantize_rows_int8_kernel<128, false, false>
+                  : once ? quantize_rows_int8_kernel<64, true, false> : quantize_rows_int8_kernel<64, false, false>;
     kernel<<<dim3(tiles, heads), THREADS, 0, s>>>(xb, to_layout(layout), mean, n_tokens, codes, scales, rope);
     return unica_check_launch("quantize_int8");
 }

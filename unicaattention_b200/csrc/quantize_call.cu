@@ -6,10 +6,12 @@
 //   1. the blocks of a cluster take the statistics of an eighth of the head's 256-token blocks each,
 //   2. they read one another's partial results through distributed shared memory, all in the same order,
 //   3. and quantize an eighth of the head's tiles each; the tokens come out of L2 now.
-// What bounds it: latency (two dependent trips to memory and a cluster barrier each way) for few tokens; at 30 heads x 4128
-// tokens the instructions of the conversions, so the loads of a tile are issued while the one before is worked on, minima
-// and maxima are taken on bfloat16 pairs, and outliers are looked for by all warps (that size on a B200: INT8 88 -> 63 us,
-// with outliers 127 -> 101 us, NVFP4 93 -> 80 us).
+// What bounds it: latency.  For few tokens two dependent trips to memory and a cluster barrier each way; at 30 heads x 4128 tokens every
+// block alternates between loads and conversions, with a third of the chip's warps in flight (issue 37 % busy).  Hence as many blocks
+// per SM as their registers allow, four for INT8 (64 registers; the clusters of K and V of that size are then on the GPU together) and
+// three for NVFP4 and rotated rows, with nothing loaded ahead of a tile, which the other blocks make up for (a call of 30 x 4128 per
+// token 375.6 -> 367.9 us, with outliers 380.3 -> 362.4); minima and maxima are taken on bfloat16 pairs, and outliers are looked for
+// by all warps.
 //
 // Sums run in the order of channel_stats_kernel and its finish kernel (quantize.cu), minima and maxima are exact: the
 // operands are bit for bit those of the separate passes.
@@ -47,10 +49,10 @@ struct CallStats {
 template <int CLUSTER = CALL_CLUSTER>
 __device__ __forceinline__ int share(int count, int rank) { return count * rank / CLUSTER; }
 
-// Sum, min and max per channel of 256-token block `b` into part[3][128]: channel_stats_kernel's arithmetic.
-template <bool SUMS, bool RANGE, typename Skip>
+// Sum, min and max per channel of 256-token block `b` into out[3][128]: channel_stats_kernel's arithmetic.
+template <bool SUMS, bool RANGE, int LOADS, typename Skip>
 __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const RopeTable& rope, Skip skip, int head, int b,
-                                            int n_tokens, CallStats& sm, float (&part)[3][HEAD_DIM]) {
+                                            int n_tokens, CallStats& sm, float (&out)[3][HEAD_DIM]) {
     const int chunk = threadIdx.x % 16, lane = threadIdx.x / 16;
     float2 sum[4], low[4], high[4];
     // minima and maxima of values that are not rotated are taken on the bfloat16 pairs as they come (exact)
@@ -64,11 +66,11 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
     const int first = b * CALL_BLOCK + lane;
     const __nv_bfloat16* src = x + in.offset(head, 0) + chunk * 8;
 #pragma unroll
-    for (int part8 = 0; part8 < CALL_BLOCK / CALL_LANES; part8 += 8) {  // eight loads in flight
-        uint4 raw[8], turns[8];
+    for (int part = 0; part < CALL_BLOCK / CALL_LANES; part += LOADS) {  // so many loads in flight
+        uint4 raw[LOADS], turns[LOADS];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int token = first + (part8 + j) * CALL_LANES;
+        for (int j = 0; j < LOADS; ++j) {
+            const int token = first + (part + j) * CALL_LANES;
             raw[j] = turns[j] = make_uint4(0, 0, 0, 0);
             if (token < n_tokens) {
                 raw[j] = load_bf16x8(src + token * in.token, in.half);
@@ -76,8 +78,8 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
             }
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int token = first + (part8 + j) * CALL_LANES;
+        for (int j = 0; j < LOADS; ++j) {
+            const int token = first + (part + j) * CALL_LANES;
             if (token >= n_tokens || skip(token)) continue;
             float2 v[4];
             unpack8(raw[j], v);
@@ -111,18 +113,18 @@ __device__ __forceinline__ void block_stats(const __nv_bfloat16* __restrict__ x,
             if (SUMS) s += sm.lanes[0][l][threadIdx.x];
             if (RANGE) lo = fminf(lo, sm.lanes[1][l][threadIdx.x]), hi = fmaxf(hi, sm.lanes[2][l][threadIdx.x]);
         }
-        if (SUMS) part[0][threadIdx.x] = s;
-        if (RANGE) part[1][threadIdx.x] = lo, part[2][threadIdx.x] = hi;
+        if (SUMS) out[0][threadIdx.x] = s;
+        if (RANGE) out[1][threadIdx.x] = lo, out[2][threadIdx.x] = hi;
     }
     __syncthreads();
 }
 
 // The head's mean (SUMS), min and max (RANGE) into sm of every block of the cluster.  Every thread of the cluster calls it.
-template <bool SUMS, bool RANGE, int CLUSTER = CALL_CLUSTER, typename Skip>
+template <bool SUMS, bool RANGE, int CLUSTER = CALL_CLUSTER, int LOADS = 8, typename Skip>
 __device__ __forceinline__ void head_stats(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const RopeTable& rope, Skip skip, int head,
                                            int n_tokens, int rank, CallStats& sm) {
     const int blocks = (n_tokens + CALL_BLOCK - 1) / CALL_BLOCK, b0 = share<CLUSTER>(blocks, rank), b1 = share<CLUSTER>(blocks, rank + 1);
-    for (int b = b0; b < b1; ++b) block_stats<SUMS, RANGE>(x, in, rope, skip, head, b, n_tokens, sm, sm.part[b - b0]);
+    for (int b = b0; b < b1; ++b) block_stats<SUMS, RANGE, LOADS>(x, in, rope, skip, head, b, n_tokens, sm, sm.part[b - b0]);
     cg::this_cluster().sync();
     if (threadIdx.x < HEAD_DIM) {
         // all blocks' partial results asked for before the first is added up: a trip to another SM takes some hundred cycles
@@ -261,23 +263,10 @@ struct SkipKeys {
     __device__ __forceinline__ bool operator()(int token) const { return (is_outlier[token / 32] >> (token % 32)) & 1; }
 };
 
-// Tiles first .. last - 1 in order, each loaded while the one before is worked on.
-template <typename Raw, typename Load, typename Finish>
-__device__ __forceinline__ void each_tile(int first, int last, Load load, Finish finish) {
-    if (first >= last) return;
-    Raw raw, next;
-    load(raw, first);
-    for (int t = first; t < last; ++t) {
-        if (t + 1 < last) load(next, t + 1);
-        finish(raw, t);
-        raw = next;
-    }
-}
-
 // V_MODE: UNICA_B200_V_*; HALF, ROPE: the input is float16, Q and K are rotated (template parameters so that the other calls
 // carry none of it).  Clusters: heads of K, heads of V, then CLUSTER tiles of Q each.
 template <int V_MODE, bool HALF, bool ROPE, int CLUSTER>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 3 : 4) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
     let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ CallOutliers outliers;
@@ -289,15 +278,13 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         TokenLayout in = op.in;
         in.half = HALF;
         const int head = cluster;
-        head_stats<true, false, CLUSTER>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, false, CLUSTER, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
-        each_tile<RowsRaw<KEY_TILE>>(
-            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { rows_load<KEY_TILE>(raw, op.x, in, head, t, op.n_tokens); },
-            [&](const auto& raw, int t) {
-                const size_t tile = size_t(head) * op.tiles + t;
-                rows_int8_finish<KEY_TILE>(raw, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
-                                           static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
-            });
+        for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
+            const size_t tile = size_t(head) * op.tiles + t;
+            rows_int8_tile<KEY_TILE, CALL_THREADS, ROPE>(op.x, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
+                                                         static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
+        }
     } else if ((cluster -= clusters_k) < clusters_v) {
         const CallOperand& op = call.v;
         TokenLayout in = op.in;
@@ -305,12 +292,9 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         const int head = cluster;
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
-            each_tile<VRaw>(
-                share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_load(raw, op.x, in, skip, head, t, op.n_tokens); },
-                [&](const auto& raw, int t) {
-                    v_int8_finish<decltype(per_token)::value>(raw, sm.low, sm.high, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale,
-                                                              call.v_token, sm.v_tile[t & 1]);
-                });
+            for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t)
+                v_int8_tile<decltype(per_token)::value>(op.x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale, call.v_token,
+                                                        sm.v_tile[t & 1]);
         };
         if constexpr (V_MODE == UNICA_B200_V_TOKEN) {
             tiles(std::true_type{}, NoSkip{});
@@ -346,7 +330,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
             int8_t* codes = reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM);
             float* scale = static_cast<float*>(op.scales) + tile;
             if constexpr (ROPE)
-                rows_int8_tile<QUERY_TILE>(op.x, in, nullptr, head, t, op.n_tokens, codes, scale, rope, sm.scratch[0]);
+                rows_int8_tile<QUERY_TILE, CALL_THREADS, true>(op.x, in, nullptr, head, t, op.n_tokens, codes, scale, rope, sm.scratch[0]);
             else
                 rows_int8_tile_raw<QUERY_TILE>(op.x, in, head, t, op.n_tokens, codes, scale, sm.scratch[0]);
         }
@@ -357,11 +341,12 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
 // max |x - mean| of the block's values -> the outer scale of all: see nvfp4_outer_rows_kernel
 __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (1.0f / 2688.0f), 1e-30f); }
 
-// HALF: the inputs are float16 (1) or bfloat16 (0), or each what its layout says.  Clusters: heads of K, of V, of Q.  Rotated inputs keep twice the loads in flight: with three blocks per SM their registers
-// spilled (2 x 16 heads x 777 tokens: 49 us, with two 42 us).
+// HALF: the inputs are float16 (1) or bfloat16 (0), or each what its layout says.  Clusters: heads of K, of V, of Q.  Rotated inputs load their
+// angles too, and half as many tokens at a time in the statistics, so that three blocks fit an SM (2 x 16 heads x 777 tokens: with two blocks
+// and eight tokens 61.5 us a call, with three and four 56.1; with three and eight, spilling, 59.4).
 constexpr int EACH_ITS_OWN = 2;
 template <int HALF, bool ROPE, int CLUSTER>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     let_next_kernel_start();
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
@@ -372,7 +357,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         const CallOperand& op = call.k;
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
-        head_stats<true, true, CLUSTER>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, true, CLUSTER, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
             const float m = sm.mean[threadIdx.x];
@@ -383,7 +368,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
         for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {  // (no barrier in a tile: the warps run ahead of one another)
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<KEY_TILE, true>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
+            rows_fp4_tile<KEY_TILE, true, ROPE>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
                                           static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), rope);
         }
     } else if (kind == 1) {
@@ -391,13 +376,11 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
         head_stats<false, true, CLUSTER>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
-        each_tile<VRaw>(
-            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, op.x, in, head, t, op.n_tokens); },
-            [&](const auto& raw, int t) {
-                const size_t tile = size_t(head) * op.tiles + t;
-                v_fp4_finish(raw, sm.low, sm.high, t, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
-                             op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
-            });
+        for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
+            const size_t tile = size_t(head) * op.tiles + t;
+            v_fp4_tile(op.x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
+                       op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
+        }
     } else {
         // Q: a mean per group of `smooth` tokens, whole groups per block
         const CallOperand& op = call.q;
@@ -409,7 +392,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
             float s = 0.0f, lo = INFINITY, hi = -INFINITY;
             const int b1 = min((g + 1) * per, blocks);
             for (int b = g * per; b < b1; ++b) {
-                block_stats<true, true>(op.x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
+                block_stats<true, true, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
                 if (threadIdx.x < HEAD_DIM)
                     s += sm.part[0][0][threadIdx.x], lo = fminf(lo, sm.part[0][1][threadIdx.x]), hi = fmaxf(hi, sm.part[0][2][threadIdx.x]);
                 __syncthreads();
@@ -435,7 +418,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         __syncthreads();
         for (int t = t0; t < t1; ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<QUERY_TILE, false>(op.x, in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
+            rows_fp4_tile<QUERY_TILE, false, ROPE>(op.x, in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
                                              op.codes + tile * (QUERY_TILE * HEAD_DIM / 2), static_cast<uint8_t*>(op.scales) + tile * (QUERY_TILE * 8), rope);
         }
     }

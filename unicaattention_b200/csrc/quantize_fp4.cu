@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(FP4_THREADS) quantize_rows_fp4_kernel(const __
                                                                          uint8_t* __restrict__ codes, uint8_t* __restrict__ sf,
                                                                          RopeTable rope) {
     const int head = blockIdx.y, tile = blockIdx.x;
-    rows_fp4_tile<ROWS, SLOTS>(x, in, [&](int token) { return mean ? mean + (size_t(head) * groups + token / mean_tokens) * HEAD_DIM : nullptr; }, fp4_outer(outer[head]),
+    rows_fp4_tile<ROWS, SLOTS, true>(x, in, [&](int token) { return mean ? mean + (size_t(head) * groups + token / mean_tokens) * HEAD_DIM : nullptr; }, fp4_outer(outer[head]),
                                head, tile, n_tokens, codes + (size_t(head) * gridDim.x + tile) * (ROWS * HEAD_DIM / 2),
                                sf + (size_t(head) * gridDim.x + tile) * (ROWS * 8), rope);
 }

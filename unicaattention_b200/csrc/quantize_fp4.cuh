@@ -73,14 +73,13 @@ __device__ __forceinline__ void quantize_block16(float2 (&v)[8], const Fp4Outer&
 // mean_of(token): the 128 means that go with the token, or null.
 // codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][32 lanes][4 words]
 // [4] bytes, K [32 lanes][4 words][4] bytes (see the store below).
-// In two halves, so that a caller with several tiles can have the next one's loads under way while it works on one.
-template <int ROWS, bool SLOTS>
+template <int ROWS, bool SLOTS, bool BY_ROW>
 __device__ __forceinline__ void rows_fp4_load(RowsRaw<ROWS, FP4_THREADS>& raw, const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile,
                                               int n_tokens) {
     const __nv_bfloat16* first = x + in.offset(head, tile * ROWS);
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
-        const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;  // block of 16 channels
+        const auto [row, block] = RowsItem<ROWS, FP4_THREADS, BY_ROW>(it);  // block of 16 channels
         const int at = SLOTS ? slot_key(row) : row;
         raw.piece[it][0] = raw.piece[it][1] = make_uint4(0, 0, 0, 0);
         if (tile * ROWS + at < n_tokens) {
@@ -89,13 +88,13 @@ __device__ __forceinline__ void rows_fp4_load(RowsRaw<ROWS, FP4_THREADS>& raw, c
         }
     }
 }
-template <int ROWS, bool SLOTS, typename MeanOf>
+template <int ROWS, bool SLOTS, bool BY_ROW, typename MeanOf>
 __device__ __forceinline__ void rows_fp4_finish(const RowsRaw<ROWS, FP4_THREADS>& raw, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
                                                 int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
                                                 const RopeTable& rope) {
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
-        const int item = it * FP4_THREADS + threadIdx.x, row = item % ROWS, block = item / ROWS;
+        const auto [row, block] = RowsItem<ROWS, FP4_THREADS, BY_ROW>(it);
         const int token = SLOTS ? tile * ROWS + slot_key(row) : tile * ROWS + row;
         uint4 turns[2];  // the table's row, asked for under no condition: the compiler may then ask for several at once
         if (rope.table) {
@@ -129,13 +128,13 @@ __device__ __forceinline__ void rows_fp4_finish(const RowsRaw<ROWS, FP4_THREADS>
         tile_sf[word * 4 + block % 4] = uint8_t(byte);
     }
 }
-template <int ROWS, bool SLOTS, typename MeanOf>
+template <int ROWS, bool SLOTS, bool BY_ROW, typename MeanOf>
 __device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
                                               int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
                                               const RopeTable& rope) {
     RowsRaw<ROWS, FP4_THREADS> raw;
-    rows_fp4_load<ROWS, SLOTS>(raw, x, in, head, tile, n_tokens);
-    rows_fp4_finish<ROWS, SLOTS>(raw, in, mean_of, outer, head, tile, n_tokens, tile_codes, tile_sf, rope);
+    rows_fp4_load<ROWS, SLOTS, BY_ROW>(raw, x, in, head, tile, n_tokens);
+    rows_fp4_finish<ROWS, SLOTS, BY_ROW>(raw, in, mean_of, outer, head, tile, n_tokens, tile_codes, tile_sf, rope);
 }
 
 // V in NVFP4 along the keys, per channel: one tile of 64 keys (slot order) by a block of FP4_THREADS.  low/high: the channel's

@@ -84,18 +84,28 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float2 (&v)[4]) {
 // staged: the tile's rows already in shared memory as the streaming kernels lay them out (see staged_chunk; then x is not
 // read), or null.
 //
-// In two halves, so that a caller with several tiles can have the next one's loads under way while it works on one.
+// Which row and 16-channel chunk a thread's item is.  BY_ROW: eight threads to a row, so that a warp's load touches 8 lines; the faster way
+// for rotated rows, whose angles are read alike (2 x 16 heads x 777 tokens, NVFP4: 64.9 -> 61.5 us a call; 40 x 32760, INT8: 90 us of 800).
+// Otherwise a row per lane: 32 lines, but a warp reads the same means and stores 512 contiguous bytes (30 x 4128, INT8: 374.4 against 378).
+template <int ROWS, int NT, bool BY_ROW>
+struct RowsItem {
+    int row, chunk;
+    __device__ __forceinline__ explicit RowsItem(int it) {
+        const int item = it * NT + int(threadIdx.x);
+        row = BY_ROW ? item / 8 : item % ROWS, chunk = BY_ROW ? item % 8 : item / ROWS;
+    }
+};
 template <int ROWS, int NT = THREADS>
 struct RowsRaw {
     uint4 piece[ROWS * 8 / NT][2];  // (row, 16-channel chunk) items of a thread, as bfloat16; zeros past the last token
 };
-template <int ROWS, int NT = THREADS>
+template <int ROWS, int NT = THREADS, bool BY_ROW = false>
 __device__ __forceinline__ void rows_load(RowsRaw<ROWS, NT>& raw, const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile,
                                           int n_tokens, const __nv_bfloat16* staged = nullptr) {
     const __nv_bfloat16* first = staged ? staged : x + in.offset(head, tile * ROWS);
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / NT; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
         raw.piece[it][0] = raw.piece[it][1] = make_uint4(0, 0, 0, 0);
         if (tile * ROWS + row < n_tokens) {
             const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : first + row * in.token + chunk * 16;
@@ -104,7 +114,7 @@ __device__ __forceinline__ void rows_load(RowsRaw<ROWS, NT>& raw, const __nv_bfl
     }
 }
 // The tile's values (v: a thread's items, local: the largest |v| of them) to codes and scale.
-template <int ROWS, int NT>
+template <int ROWS, int NT, bool BY_ROW>
 __device__ __forceinline__ void rows_int8_store(const float2 (&v)[ROWS * 8 / NT][8], float local, int8_t* __restrict__ out, float* __restrict__ scale_out,
                                                 float* scratch) {
     const float scale = fmaxf(block_max<NT>(local, scratch) * (1.0f / 127.0f), 1e-12f);
@@ -114,7 +124,7 @@ __device__ __forceinline__ void rows_int8_store(const float2 (&v)[ROWS * 8 / NT]
     if (threadIdx.x == 0) *scale_out = scale;
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / NT; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
         float2 t[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) t[i] = quotient_code2(v[it][i], inv2, minus_scale2);
@@ -126,7 +136,7 @@ __device__ __forceinline__ void rows_int8_store(const float2 (&v)[ROWS * 8 / NT]
             make_uint4(low_bytes(t[0], t[1]), low_bytes(t[2], t[3]), low_bytes(t[4], t[5]), low_bytes(t[6], t[7]));
     }
 }
-template <int ROWS, int NT = THREADS>
+template <int ROWS, int NT = THREADS, bool BY_ROW = false>
 __device__ __forceinline__ void rows_int8_finish(const RowsRaw<ROWS, NT>& raw, const TokenLayout& in, const float* mean, int head, int tile, int n_tokens,
                                                  int8_t* __restrict__ out, float* __restrict__ scale_out, const RopeTable& rope, float* scratch) {
     constexpr int ITEMS = ROWS * 8 / NT;
@@ -135,9 +145,9 @@ __device__ __forceinline__ void rows_int8_finish(const RowsRaw<ROWS, NT>& raw, c
     float local = 0.0f;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
         unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(v[it][0]));
         unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(v[it][4]));
+        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
         if (token0 + row < n_tokens) {
             if (rope.table) {  // rotate first, then take the mean (of the rotated x) away
                 const __half* f = rope.row(in, head, token0 + row);
@@ -156,20 +166,20 @@ __device__ __forceinline__ void rows_int8_finish(const RowsRaw<ROWS, NT>& raw, c
 #pragma unroll
         for (int i = 0; i < 8; ++i) local = max3(local, fabsf(v[it][i].x), fabsf(v[it][i].y));
     }
-    rows_int8_store<ROWS, NT>(v, local, out, scale_out, scratch);
+    rows_int8_store<ROWS, NT, BY_ROW>(v, local, out, scale_out, scratch);
 }
-template <int ROWS, int NT = THREADS>
+template <int ROWS, int NT = THREADS, bool BY_ROW = false>
 __device__ __forceinline__ void rows_int8_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const float* mean, int head,
                                                int tile, int n_tokens, int8_t* __restrict__ out, float* __restrict__ scale_out,
                                                const RopeTable& rope, float* scratch, const __nv_bfloat16* staged = nullptr) {
     RowsRaw<ROWS, NT> raw;
-    rows_load<ROWS, NT>(raw, x, in, head, tile, n_tokens, staged);
-    rows_int8_finish<ROWS, NT>(raw, in, mean, head, tile, n_tokens, out, scale_out, rope, scratch);
+    rows_load<ROWS, NT, BY_ROW>(raw, x, in, head, tile, n_tokens, staged);
+    rows_int8_finish<ROWS, NT, BY_ROW>(raw, in, mean, head, tile, n_tokens, out, scale_out, rope, scratch);
 }
 
 // The same with each item converted as it is loaded.  The faster form for rotated tiles of 64 rows (40 heads x 32760 tokens: 218.8
 // -> 212.4 us; of 128 rows 203 -> 221) and short ones (see quantize_int8 in quantize.cu), and for Q's tiles staged in shared memory, where nothing has to be under way (107.8 -> 104.5).
-template <int ROWS, int NT = THREADS>
+template <int ROWS, int NT = THREADS, bool BY_ROW = false>
 __device__ __forceinline__ void rows_int8_tile_once(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, const float* mean, int head, int tile,
                                                     int n_tokens, int8_t* __restrict__ out, float* __restrict__ scale_out, const RopeTable& rope,
                                                     float* scratch, const __nv_bfloat16* staged = nullptr) {
@@ -179,7 +189,7 @@ __device__ __forceinline__ void rows_int8_tile_once(const __nv_bfloat16* __restr
     float local = 0.0f;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
         if (token0 + row < n_tokens) {
             const __nv_bfloat16* src = staged ? staged_chunk(staged, row, chunk) : x + in.offset(head, token0 + row) + chunk * 16;
             float2 a[4], b[4];
@@ -203,12 +213,12 @@ __device__ __forceinline__ void rows_int8_tile_once(const __nv_bfloat16* __restr
 #pragma unroll
         for (int i = 0; i < 8; ++i) local = max3(local, fabsf(v[it][i].x), fabsf(v[it][i].y));
     }
-    rows_int8_store<ROWS, NT>(v, local, out, scale_out, scratch);
+    rows_int8_store<ROWS, NT, BY_ROW>(v, local, out, scale_out, scratch);
 }
 
 // rows_int8_tile without a mean and without RoPE (Q): the tile stays in registers as it came, two elements to a register, and
 // its maximum is taken on the bfloat16 pairs (exact), which halves the registers and the instructions up to the scale.
-template <int ROWS, int NT = THREADS>
+template <int ROWS, int NT = THREADS, bool BY_ROW = false>
 __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile, int n_tokens,
                                                    int8_t* __restrict__ out, float* __restrict__ scale_out, float* scratch,
                                                    const __nv_bfloat16* staged = nullptr) {
@@ -230,7 +240,7 @@ __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restri
     if (threadIdx.x == 0) *scale_out = scale;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-        const int item = it * NT + threadIdx.x, row = item % ROWS, chunk = item / ROWS;
+        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
         float2 t[8];
         unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(t[0]));
         unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(t[4]));
