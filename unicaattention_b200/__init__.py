@@ -83,12 +83,13 @@ def token_layout(x: torch.Tensor) -> TokenLayout:
 
 def readable(x: torch.Tensor) -> torch.Tensor:
     """x itself if the kernels can read it in place (contiguous last dimension, 16-byte aligned tokens), else a
-    contiguous copy (unica/__init__.py:103-108)."""
+    contiguous copy (unica/__init__.py:103-108); also of a contiguous tensor that starts between two 16-byte boundaries, which
+    contiguous() would return as it is."""
     batch, head, token, channel = x.stride()
     if channel == 1 and not (batch | head | token) & 7 and not x.data_ptr() & 15:
         return x
     in_place = channel == 1 and x.data_ptr() % 16 == 0 and all(x.stride(i) % 8 == 0 or x.shape[i] == 1 for i in range(3))
-    return x if in_place else x.contiguous()
+    return x if in_place else x.clone(memory_format=torch.contiguous_format)
 
 
 def on_their_device(function):
