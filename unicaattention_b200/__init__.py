@@ -477,6 +477,15 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
     peer_out: with out, up to 7 device addresses of tensors laid out like out in other GPUs' memory, mapped into this
     process; the kernel stores every row there as well (see shard.SharedOutput, which also does the barriers this needs).
     Same checks and exceptions as the reference (unica/__init__.py:126-190)."""
+    if inputs is None and rope is None and out is None and not peer_out and heads_per_call is _heads_per_call:
+        # The usual call, of shapes, strides, types and settings that have been seen before: everything that follows from those is in
+        # its plan (18 -> 10 us of host time a call, as long as the GPU takes for the smallest ones).
+        plan = _PLANS.get((kernel, q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.get_device(), k.get_device(),
+                           v.get_device(), *tile.items()))
+        if plan is not None:
+            planned = plan.run(q, k, v)
+            if planned is not None:
+                return planned
     settings = _settings(kernel, tile)
     if out is not None:
         if out.dtype != q.dtype or out.shape != q.shape or out.device != q.device or readable(out) is not out:
@@ -509,7 +518,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         return out
     if inputs is None:
         try:
-            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out)):
+            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out), tile):
                 return out
             inputs = kernel_inputs(q, k, v, kernel, rope, **tile)
         except torch.cuda.OutOfMemoryError:
@@ -539,7 +548,34 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
 _WORKSPACE_BYTES: dict = {}  # (heads, queries, keys, kernel, V mode, outliers, SMOOTH_Q, rope?) -> bytes
 
 
-def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int) -> bool:
+class _Plan:
+    """What attention() works out of a call's shapes, strides, types and settings.  Holds no tensor; what can change from one call to the
+    next (addresses and their alignment, free memory, the stream) is looked at in every call."""
+
+    __slots__ = ("device", "index", "need", "size", "fixed", "out_stride")
+
+    def run(self, q, k, v):
+        """The call, or None: not by this plan (not enough memory as far as one knows, or a tensor to be copied first)."""
+        q_at, k_at, v_at = q.data_ptr(), k.data_ptr(), v.data_ptr()
+        device, need = self.device, self.need
+        if (q_at | k_at | v_at) & 15 or LOG_VRAM or need > vram_reserve(device) // SMALL_CALL_FRACTION or need > free_vram(device) // STALE_FRACTION:
+            return None
+        out = torch.empty_like(q)
+        if out.stride() != self.out_stride:
+            return None
+        try:
+            workspace = torch.empty(self.size, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:  # attention() goes by heads then
+            return None
+        lib.attention_call(lib.pack_call_head(q_at, k_at, v_at, out.data_ptr(), workspace.data_ptr(), self.size, 0, 0, 0, status_word(device).data_ptr(),
+                                              torch._C._cuda_getCurrentRawStream(self.index)) + self.fixed)
+        return out
+
+
+_PLANS: dict = {}  # see attention() for the key
+
+
+def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, tile: dict | None = None) -> bool:
     """The whole call through one entry point of the library: quantization and kernel with their operands in one workspace.
     Bit for bit kernel_inputs() and the kernel, without their dozen allocations and trips through ctypes.  False: not
     for this call (the outlier keys of a long V are found by torch)."""
@@ -573,6 +609,15 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
                                      n_peers, scale))
+    if rope is None and peers is None and tile is not None:
+        # (readable() has let these strides pass, if not as they came then in a copy whose strides are a later call's: a plan asks for no copies)
+        plan = _Plan()
+        plan.device, plan.index, plan.size, plan.out_stride = device, device.index, size, os_
+        plan.need = _call_bytes(batch, heads, n_queries, n_keys, settings["SMOOTH_Q"] if fast else 0)
+        plan.fixed = lib.pack_call_tail(*layouts, *sizes, 0, scale)
+        if len(_PLANS) > 4096:
+            _PLANS.clear()
+        _PLANS[(kernel, q.shape, k.shape, v.shape, qs, ks, vs, q.dtype, k.dtype, v.dtype, device.index, k.get_device(), v.get_device(), *tile.items())] = plan
     return True
 
 
@@ -608,18 +653,22 @@ def vram_reserve(device: torch.device) -> int:
     return max(2**30, tenth)
 
 
+def _call_bytes(batch: int, heads: int, n_queries: int, n_keys: int, smooth: int) -> int:
+    """Temporary memory of a call, see heads_per_call."""
+    per_head = max(1, 2 * batch * HEAD_DIM * (n_queries + 2 * n_keys))
+    if smooth:
+        per_head += batch * 4 * math.ceil(n_queries / smooth) * n_keys
+    return heads * per_head
+
+
 def heads_per_call(q: torch.Tensor, k: torch.Tensor, kernel: str, tile: dict) -> int:
     """How many heads one call takes without its temporary buffers reaching the reserve.  Per head: the quantized q, k,
     v and the output, at most 2 bytes per element of q, k, v (float16 inputs are read in place, like bfloat16); in the fast
     mode the smoothing table, one float per key and block of SMOOTH_Q queries (unica/__init__.py:208-232 counts the same
     things).  A small call runs whole."""
     batch, heads, n_queries, _ = q.shape
-    n_keys = k.shape[2]
-    elements = batch * HEAD_DIM * (n_queries + 2 * n_keys)
-    per_head = max(1, elements * 2)
     smooth = (TILE | tile).get("SMOOTH_Q", 0) if kernel == "attention_fp4" else 0
-    if smooth:
-        per_head += batch * 4 * math.ceil(n_queries / smooth) * n_keys
+    per_head = _call_bytes(batch, 1, n_queries, k.shape[2], smooth)
     free, reserve = free_vram(q.device), vram_reserve(q.device)
     if heads * per_head > free // STALE_FRACTION:  # a call this size must not trust an answer something else may have outdated
         free = free_vram(q.device, fresh=True)
@@ -654,6 +703,7 @@ def in_pieces(q, k, v, kernel: str, rope, tile: dict, out: torch.Tensor | None =
     return in_pieces(q, k, v, kernel, rope, tile, out, (), step)
 
 
+_heads_per_call = heads_per_call  # a caller may put a planner of its own in its place: attention() then asks that one for every call
 _SM_COUNTS: dict = {}
 
 

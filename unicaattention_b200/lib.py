@@ -67,7 +67,9 @@ SIGNATURES = {
 # struct unica_b200_call as bytes, in the header's order (packing forty numbers at once costs a microsecond, filling a
 # ctypes structure several): q, k, v, out, workspace, its size, rope, its batch stride, peer_out, status, stream; the four
 # layouts; heads, n_queries, n_keys, kernel, v_mode, n_outliers, smooth_q, n_peers; scale_log2
-pack_call = struct.Struct("@PPPPPNPqPPP" + "qqqii" * 4 + "iiiiiiiif4x").pack
+_HEAD, _TAIL = "PPPPPNPqPPP", "qqqii" * 4 + "iiiiiiiif4x"
+pack_call = struct.Struct("@" + _HEAD + _TAIL).pack
+pack_call_head, pack_call_tail = struct.Struct("@" + _HEAD).pack, struct.Struct("@" + _TAIL).pack  # the same in two (the head ends on 8 bytes)
 CALL_TOKENS = 8192  # keys up to which a call with V_OUTLIERS fits one entry point
 
 
