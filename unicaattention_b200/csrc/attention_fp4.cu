@@ -7,7 +7,8 @@
 //                               128 multiplies P by a row of ones: the running softmax denominator, rescaled with O
 //
 // Persistent blocks, one per SM, each taking pairs of query tiles (items) blockIdx.x, blockIdx.x + gridDim.x, ...; the two
-// tiles of an item (t = 0, 1) share every K and V tile.  Key tiles are counted across items (g), and every ring runs on from
+// tiles of an item (t = 0, 1) share every K and V tile.  Where pairs would leave SMs idle an item is one query tile (TILES 1: two
+// softmax warpgroups, with as many registers as they like).  Key tiles are counted across items (g), and every ring runs on from
 // one item to the next.  Five warpgroups:
 //
 //   softmax [t][w]  query tile t, key tiles g with g & 1 = w: a thread is a query row (a tensor-memory lane), all 64 scores of
@@ -48,10 +49,13 @@
 
 namespace unica {
 
-constexpr int F4_TILES = 2;  // query tiles of 128 rows per item (tensor memory holds two: 2 x 232 of 512 columns)
-constexpr int F4_SCORES_WARP = 0, F4_PV_WARP = 1, F4_COPY_WARP = F4_PV_WARP + F4_TILES, F4_SOFTMAX_WARP = 4, F4_WARPS = F4_SOFTMAX_WARP + 8 * F4_TILES, F4_THREADS = F4_WARPS * 32;
-constexpr int F4_LAUNCH_REGISTERS = 96, F4_SOFTMAX_REGISTERS = 112, F4_SERVICE_REGISTERS = 32;
-static_assert(128 * (2 * F4_TILES * F4_SOFTMAX_REGISTERS + F4_SERVICE_REGISTERS) <= F4_THREADS * F4_LAUNCH_REGISTERS, "the split must fit the launch");
+// TILES, below: query tiles of 128 rows per item, 2 (tensor memory holds two: 2 x 232 of 512 columns) or, where that leaves SMs idle, 1.
+constexpr int F4_SCORES_WARP = 0, F4_PV_WARP = 1, F4_COPY_WARP = 3, F4_SOFTMAX_WARP = 4;
+template <int TILES>
+constexpr int F4_THREADS = (F4_SOFTMAX_WARP + 8 * TILES) * 32;
+// with two query tiles the registers are dealt out: what a thread is launched with, and has after setmaxnreg
+constexpr int F4_LAUNCH_REGISTERS = 96, F4_SOFTMAX_REGISTERS = 112, F4_SERVICE_REGISTERS = 32, F4_SPLIT_REGISTERS = 128 * (4 * F4_SOFTMAX_REGISTERS + F4_SERVICE_REGISTERS);
+static_assert(F4_SPLIT_REGISTERS <= F4_THREADS<2> * F4_LAUNCH_REGISTERS, "the split must fit the launch");
 constexpr int F4_HALF_SLOTS = KEY_TILE / 2;  // one 16-byte piece of a row of P^: two scale blocks of 16 slots
 constexpr int F4_K_RING = 4, F4_V_RING = 8;  // K4 and V4 tiles in shared memory, see f4_copy_warp
 constexpr int Q4_BYTES = QUERY_TILE * HEAD_DIM / 2;  // 8192
@@ -62,32 +66,32 @@ constexpr int V4_TILE_ROWS = 144, V4_BYTES = 2 * V4_TILE_ROWS * 16;  // 4608
 constexpr int SFV_BYTES = 256 * 4;                   // 1024: two blocks of 32 lanes x 4 words
 constexpr int BIAS_BYTES = KEY_TILE * 4;             // 256
 constexpr int P4_BYTES = QUERY_TILE * KEY_TILE / 2;  // 4096
-constexpr int F4_TMEM_COLUMNS = 256 * F4_TILES;
 constexpr int F4_S = 0, F4_O = 64, F4_SFQ = 208, F4_SFK = 216, F4_SFP = 220, F4_SFV = 224;
 constexpr float P_LOG2_GAIN = 10.0f;  // P is taken times 2^10: its block scales (up to 1024 / 6) stay below e4m3's 448
 
+template <int TILES>
 struct __align__(128) Fp4Smem {
-    uint8_t q[2][F4_TILES][Q4_BYTES];         // two items
-    uint32_t sfq[2][F4_TILES][2][32][4];      // scale words as tcgen05.cp takes them: [K step] lane, word row / 32
+    uint8_t q[2][TILES][Q4_BYTES];            // two items
+    uint32_t sfq[2][TILES][2][32][4];         // scale words as tcgen05.cp takes them: [K step] lane, word row / 32
     uint8_t k[F4_K_RING][K4_BYTES];
     uint32_t sfk[F4_K_RING][32][4];           // lane, word 2 step + row / 32
     uint8_t v[F4_V_RING][V4_BYTES];
     uint32_t sfv[F4_V_RING][2][32][4];        // block 0: channel c = word c / 32 of lane c % 32; block 1: the ones rows
     float bias[F4_V_RING][KEY_TILE];
     float mask[2][KEY_TILE];                  // what is added to the scores where there is no smoothing term: zeros / -inf in the last tile's empty slots
-    uint8_t p[F4_TILES][2][P4_BYTES];
-    uint32_t sfp[F4_TILES][2][32][4];         // P's scale words: row r = word r / 32 of lane r % 32
-    float m[F4_TILES][2][QUERY_TILE];         // the running maximum after the last tile of either warpgroup
-    uint8_t staged[F4_TILES][4][32 * STAGED_PITCH];  // output rows on their way out
+    uint8_t p[TILES][2][P4_BYTES];
+    uint32_t sfp[TILES][2][32][4];            // P's scale words: row r = word r / 32 of lane r % 32
+    float m[TILES][2][QUERY_TILE];            // the running maximum after the last tile of either warpgroup
+    uint8_t staged[TILES][4][32 * STAGED_PITCH];     // output rows on their way out
     float log2_e4m3[128];                     // log2 of every non-negative e4m3 byte's value; +inf for the byte 0, so that 2^(x - that) = 0
     // s_full, pv_done: [query tile][g & 1].  (One score buffer, but a barrier for either warpgroup: a warpgroup that has not yet
     // seen the first of two phases must not take a look for the second for an answer.)
-    uint64_t q_full[2], k_full[F4_K_RING], v_full[F4_V_RING], s_full[F4_TILES][2], pv_done[F4_TILES][2], drain[1 + F4_TILES];
+    uint64_t q_full[2], k_full[F4_K_RING], v_full[F4_V_RING], s_full[TILES][2], pv_done[TILES][2], drain[1 + TILES];
     uint32_t tmem_base;
     int abort_flag;
-    int alone[2 + F4_TILES];  // zeros: a word for each warp that drains what it issued, which no other warp's wait may cut short
+    int alone[2 + TILES];  // zeros: a word for each warp that drains what it issued, which no other warp's wait may cut short
 };
-static_assert(sizeof(Fp4Smem) + 128 <= 227 * 1024, "the block's shared memory");
+static_assert(sizeof(Fp4Smem<2>) + 128 <= 227 * 1024, "the block's shared memory");
 
 // scores of query tile t taken: one softmax warpgroup -> the scores warp
 __device__ __forceinline__ void f4_s_free_arrive(int t) { asm volatile("bar.arrive %0, 160;" ::"r"(1 + t) : "memory"); }
@@ -136,7 +140,7 @@ struct Fp4Args {
     TokenLayout out_layout;
     PeerOutputs peers;
     int n_queries, n_keys;
-    Items items;  // pairs of query tiles
+    Items items;  // (pairs of) query tiles
     float scale_log2;
     uint32_t* p_words;
     int* status;
@@ -198,7 +202,8 @@ __device__ __forceinline__ void f4_issue_pv(uint32_t base, uint64_t p_desc, uint
 // S(g) of both query tiles as soon as K4(g) has landed and the softmax of tile g - 1 has taken the scores.  A wait that gave up
 // changes nothing here: instructions on whatever lies in the buffers do no harm (the result is not stored), and every hand-over
 // still finds its receiver.
-__device__ __forceinline__ void f4_scores_warp(Fp4Smem& sm, const Fp4Args& a, int k_tiles, uint32_t tmem) {
+template <int TILES>
+__device__ __forceinline__ void f4_scores_warp(Fp4Smem<TILES>& sm, const Fp4Args& a, int k_tiles, uint32_t tmem) {
     const int total = a.items.mine() * k_tiles;
     const uint64_t q_desc0 = smem_desc(smem_u32(sm.q[0][0]), QUERY_TILE * 16, 128), k_desc0 = smem_desc(smem_u32(sm.k[0]), KEY_TILE * 16, 128);
     const uint64_t sfq_desc0 = smem_desc(smem_u32(sm.sfq[0][0]), 16, 128), sfk_desc0 = smem_desc(smem_u32(sm.sfk[0]), 16, 128);
@@ -209,23 +214,23 @@ __device__ __forceinline__ void f4_scores_warp(Fp4Smem& sm, const Fp4Args& a, in
         mbar_wait_line(&sm.k_full[slot<F4_K_RING>(g)], round_parity<F4_K_RING>(g), &sm.abort_flag, a.status, STATUS_WAIT_TILE);
         const uint64_t k_desc = desc_at(k_desc0, slot<F4_K_RING>(g) * (K4_BYTES / 16)), sfk_desc = desc_at(sfk_desc0, slot<F4_K_RING>(g) * (SFK_BYTES / 16));
 #pragma unroll
-        for (int i = 0; i < F4_TILES; ++i) {
+        for (int i = 0; i < TILES; ++i) {
             if (g > 0) f4_s_free_sync(i);
             __syncwarp();
             tc_fence_after();
             const uint32_t base = tmem + 256 * i;
             if (t == 0) {  // Q's scale bytes, for the whole item
-                const uint64_t sfq_desc = desc_at(sfq_desc0, (slot<2>(n) * F4_TILES + i) * (SFQ_BYTES / 16));
+                const uint64_t sfq_desc = desc_at(sfq_desc0, (slot<2>(n) * TILES + i) * (SFQ_BYTES / 16));
                 cp_elected(base + F4_SFQ, sfq_desc);
                 cp_elected(base + F4_SFQ + 4, desc_at(sfq_desc, SFQ_BYTES / 32));
             }
-            f4_issue_scores(base, desc_at(q_desc0, (slot<2>(n) * F4_TILES + i) * (Q4_BYTES / 16)), k_desc, sfk_desc, &sm.s_full[i][slot<2>(g)]);
+            f4_issue_scores(base, desc_at(q_desc0, (slot<2>(n) * TILES + i) * (Q4_BYTES / 16)), k_desc, sfk_desc, &sm.s_full[i][slot<2>(g)]);
         }
         f4_copies_sync();
         if (++t == k_tiles) t = 0, ++n;
     }
 #pragma unroll
-    for (int i = 0; i < F4_TILES; ++i) f4_s_free_sync(i);
+    for (int i = 0; i < TILES; ++i) f4_s_free_sync(i);
     commit_elected(&sm.drain[0]);  // whatever was issued must finish before tensor memory is freed
     mbar_wait_line(&sm.drain[0], 0, &sm.alone[0], nullptr, 0);
     __syncwarp();
@@ -238,17 +243,18 @@ __device__ __forceinline__ void f4_scores_warp(Fp4Smem& sm, const Fp4Args& a, in
 //             g - 3, waited for P.V(g - 5)
 //   Q4 of the item after the next, at an item's first key tile: every score of the item before has been taken
 static_assert(F4_K_RING == 4 && F4_V_RING == 8, "see above");
-__device__ __forceinline__ void f4_copy_warp(Fp4Smem& sm, const Fp4Args& a, int k_tiles) {
+template <int TILES>
+__device__ __forceinline__ void f4_copy_warp(Fp4Smem<TILES>& sm, const Fp4Args& a, int k_tiles) {
     const int n_items = a.items.mine(), total = n_items * k_tiles;
     auto item_of = [&](int n) { return int(blockIdx.x) + n * int(gridDim.x); };
     auto copy_q = [&](int n) {
         const int item = item_of(n);
-        const size_t first = size_t(a.items.head(item)) * a.items.allocated + F4_TILES * a.items.tile(item);
+        const size_t first = size_t(a.items.head(item)) * a.items.allocated + TILES * a.items.tile(item);
         if (elect_one()) {
             uint64_t* full = &sm.q_full[slot<2>(n)];
-            mbar_expect_tx(full, F4_TILES * (Q4_BYTES + SFQ_BYTES));
-            bulk_load(sm.q[slot<2>(n)], a.q4 + first * Q4_BYTES, F4_TILES * Q4_BYTES, full);
-            bulk_load(sm.sfq[slot<2>(n)], a.sfq + first * (SFQ_BYTES / 4), F4_TILES * SFQ_BYTES, full);
+            mbar_expect_tx(full, TILES * (Q4_BYTES + SFQ_BYTES));
+            bulk_load(sm.q[slot<2>(n)], a.q4 + first * Q4_BYTES, TILES * Q4_BYTES, full);
+            bulk_load(sm.sfq[slot<2>(n)], a.sfq + first * (SFQ_BYTES / 4), TILES * SFQ_BYTES, full);
         }
         __syncwarp();
     };
@@ -258,7 +264,7 @@ __device__ __forceinline__ void f4_copy_warp(Fp4Smem& sm, const Fp4Args& a, int 
     const float* bias_row = nullptr;
     auto bias_of = [&](int n) {
         const int item = item_of(n);
-        return a.bias + (size_t(a.items.head(item)) * a.q_blocks + (F4_TILES * QUERY_TILE * a.items.tile(item)) / a.smooth_q) * (size_t(k_tiles) * KEY_TILE);
+        return a.bias + (size_t(a.items.head(item)) * a.q_blocks + (TILES * QUERY_TILE * a.items.tile(item)) / a.smooth_q) * (size_t(k_tiles) * KEY_TILE);
     };
     if (a.bias) bias_row = bias_of(0);
     auto copy_k = [&]() {
@@ -314,7 +320,8 @@ __device__ __forceinline__ void f4_copy_warp(Fp4Smem& sm, const Fp4Args& a, int 
 
 // P.V(g) of query tile i as soon as P4(g) is delivered and V4(g) is there (and, at an item's first key tile, the O of the item
 // before has been read).
-__device__ __forceinline__ void f4_pv_warp(Fp4Smem& sm, const Fp4Args& a, int k_tiles, uint32_t tmem, int i) {
+template <int TILES>
+__device__ __forceinline__ void f4_pv_warp(Fp4Smem<TILES>& sm, const Fp4Args& a, int k_tiles, uint32_t tmem, int i) {
     const int total = a.items.mine() * k_tiles;
     const uint32_t base = tmem + 256 * i;
     const uint64_t p_desc0 = smem_desc(smem_u32(sm.p[i][0]), QUERY_TILE * 16, 128), v_desc0 = smem_desc(smem_u32(sm.v[0]), V4_TILE_ROWS * 16, 128);
@@ -338,8 +345,8 @@ __device__ __forceinline__ void f4_pv_warp(Fp4Smem& sm, const Fp4Args& a, int k_
 // ---------------------------------------------------------------------------------------------------------------------
 // softmax: query tile `qt`, key tiles g = w, w + 2, ..; thread = query row
 
-template <bool CODES>
-__device__ __forceinline__ void f4_softmax(Fp4Smem& sm, const Fp4Args& a, int k_tiles, uint32_t tmem, int qt, int w, int quarter, int lane) {
+template <int TILES, bool CODES>
+__device__ __forceinline__ void f4_softmax(Fp4Smem<TILES>& sm, const Fp4Args& a, int k_tiles, uint32_t tmem, int qt, int w, int quarter, int lane) {
     const int row = quarter * 32 + lane, n_items = a.items.mine(), total = n_items * k_tiles;
     const uint32_t my = tmem + (uint32_t(quarter * 32) << 16) + qt * 256;
     const bool smoothed = a.bias != nullptr;
@@ -423,7 +430,7 @@ __device__ __forceinline__ void f4_softmax(Fp4Smem& sm, const Fp4Args& a, int k_
                 codes[2 * b + half] = e2m1x8(r);
             }
         }
-        auto first_row = [&]() { return (F4_TILES * a.items.tile(item_of(n)) + qt) * QUERY_TILE + quarter * 32; };  // of this warp
+        auto first_row = [&]() { return (TILES * a.items.tile(item_of(n)) + qt) * QUERY_TILE + quarter * 32; };  // of this warp
         if (CODES && first_row() + lane < a.n_queries) {  // diagnostics: this row's P^ of the tile, 8 words of codes and the 4 scale bytes
             uint32_t* dst = a.p_words + ((size_t(a.items.head(item_of(n))) * a.n_queries + first_row() + lane) * k_tiles + t) * 9;
 #pragma unroll
@@ -513,10 +520,10 @@ __device__ __forceinline__ void f4_softmax(Fp4Smem& sm, const Fp4Args& a, int k_
     bulk_store_read_wait();
 }
 
-template <bool CODES>
-__global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __grid_constant__ Fp4Args a) {
+template <int TILES, bool CODES>
+__global__ void __launch_bounds__(F4_THREADS<TILES>, 1) attention_fp4_kernel(const __grid_constant__ Fp4Args a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    Fp4Smem& sm = *reinterpret_cast<Fp4Smem*>(smem_raw);
+    Fp4Smem<TILES>& sm = *reinterpret_cast<Fp4Smem<TILES>*>(smem_raw);
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x / 32), 0), lane = threadIdx.x % 32;  // (the shuffle tells the compiler that it is uniform)
     const int k_tiles = (a.n_keys + KEY_TILE - 1) / KEY_TILE;
 
@@ -526,9 +533,9 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
         for (int s = 0; s < 2; ++s) mbar_init(&sm.q_full[s], 1);
         for (int s = 0; s < F4_K_RING; ++s) mbar_init(&sm.k_full[s], 1);
         for (int s = 0; s < F4_V_RING; ++s) mbar_init(&sm.v_full[s], 1);
-        for (int i = 0; i < F4_TILES; ++i) 
+        for (int i = 0; i < TILES; ++i)
             for (int w = 0; w < 2; ++w) mbar_init(&sm.s_full[i][w], 1), mbar_init(&sm.pv_done[i][w], 1);
-        for (int i = 0; i < 1 + F4_TILES; ++i) mbar_init(&sm.drain[i], 1);
+        for (int i = 0; i < 1 + TILES; ++i) mbar_init(&sm.drain[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x >= 128 && threadIdx.x < 256) {
@@ -542,7 +549,7 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
         sm.mask[0][at] = 0.0f;
         sm.mask[1][at] = key < a.n_keys ? 0.0f : -INFINITY;
     }
-    if (warp == 0) tmem_alloc(&sm.tmem_base, F4_TMEM_COLUMNS);
+    if (warp == 0) tmem_alloc(&sm.tmem_base, 256 * TILES);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -550,16 +557,16 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
     wait_for_previous_kernel();
 
     if (warp >= F4_SOFTMAX_WARP) {
-        set_registers<F4_SOFTMAX_REGISTERS, F4_LAUNCH_REGISTERS>();
+        if constexpr (TILES == 2) set_registers<F4_SOFTMAX_REGISTERS, F4_LAUNCH_REGISTERS>();
         const int group = (warp - F4_SOFTMAX_WARP) / 4;
-        f4_softmax<CODES>(own_view(sm), a, k_tiles, tmem, group >> 1, group & 1, warp % 4, lane);
+        f4_softmax<TILES, CODES>(own_view(sm), a, k_tiles, tmem, group >> 1, group & 1, warp % 4, lane);
     } else {
-        set_registers<F4_SERVICE_REGISTERS, F4_LAUNCH_REGISTERS>();
+        if constexpr (TILES == 2) set_registers<F4_SERVICE_REGISTERS, F4_LAUNCH_REGISTERS>();
         if (warp == F4_SCORES_WARP)
             f4_scores_warp(own_view(sm), a, k_tiles, tmem);
         else if (warp == F4_COPY_WARP)
             f4_copy_warp(own_view(sm), a, k_tiles);
-        else
+        else if (warp < F4_PV_WARP + TILES)
             f4_pv_warp(own_view(sm), a, k_tiles, tmem, warp - F4_PV_WARP);
         __syncwarp();
     }
@@ -568,13 +575,28 @@ __global__ void __launch_bounds__(F4_THREADS, 1) attention_fp4_kernel(const __gr
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(sm.tmem_base, F4_TMEM_COLUMNS);
+        tmem_dealloc(sm.tmem_base, 256 * TILES);
     }
 }
 
 }  // namespace unica
 
 using namespace unica;
+
+static constexpr int F4_MAX_DEVICES = 64;
+
+// SMs of the current device; asked for once per device.
+static int sm_count(int* sms) {
+    static std::atomic<int> known[F4_MAX_DEVICES];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
+    *sms = device < F4_MAX_DEVICES ? known[device].load(std::memory_order_relaxed) : 0;
+    if (*sms == 0) {
+        if (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
+        if (device < F4_MAX_DEVICES) known[device].store(*sms, std::memory_order_relaxed);
+    }
+    return UNICA_B200_OK;
+}
 
 int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4, const void* sfv,
                          const float* qk_outer, const float* k_outer, const float* v_outer, const float* bias, int q_blocks, int smooth_q, void* out,
@@ -594,32 +616,37 @@ int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, c
     args.qk_outer = qk_outer, args.k_outer = k_outer, args.v_outer = v_outer, args.bias = bias, args.q_blocks = q_blocks, args.smooth_q = smooth_q > 0 ? smooth_q : 1;
     args.out = static_cast<__nv_bfloat16*>(out), args.out_layout = to_layout(out_layout), args.peers = peers;
     args.n_queries = n_queries, args.n_keys = n_keys, args.scale_log2 = scale_log2, args.p_words = p_words, args.status = status;
-    const long long pairs = (n_queries + 2 * QUERY_TILE - 1) / (2 * QUERY_TILE), count = pairs * heads;  // Q4 holds an even number of tiles
-    if (count > INT_MAX / 2) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: more than 2^30 pairs of query tiles");
-    args.items.tiles = int(pairs), args.items.allocated = int(2 * pairs), args.items.count = int(count);
-    const size_t smem = sizeof(Fp4Smem) + 128;
-    auto launch = [&](auto kernel, int instance) -> int {
+    const long long pairs = (n_queries + 2 * QUERY_TILE - 1) / (2 * QUERY_TILE), tiles = (n_queries + QUERY_TILE - 1) / QUERY_TILE;  // Q4 holds an even number of tiles
+    if (pairs * heads > INT_MAX / 2) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: more than 2^30 pairs of query tiles");
+    int sms = 0;  // persistent blocks, one per SM
+    if (int e = sm_count(&sms)) return e;
+    auto launch = [&](auto kernel, int threads, int smem, int instance) -> int {
         // Set up once per kernel instance and device, as in attention_int8.cu.
-        constexpr int MAX_DEVICES = 64;
-        static std::atomic<int> blocks_of[2][MAX_DEVICES];  // persistent blocks (one per SM), 0: not set up
+        static std::atomic<bool> ready[3][F4_MAX_DEVICES];
         int device = 0;
         if (cudaGetDevice(&device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
-        int blocks = device < MAX_DEVICES ? blocks_of[instance][device].load(std::memory_order_acquire) : 0;
-        if (blocks == 0) {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
+        if (device >= F4_MAX_DEVICES || !ready[instance][device].load(std::memory_order_acquire)) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
                 cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
                 return unica_check_launch("attention_fp4 (shared memory size)");
             cudaFuncAttributes attributes;
             if (cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess) return unica_check_launch("attention_fp4 (attributes)");
-            if (attributes.numRegs * F4_THREADS < 128 * (2 * F4_TILES * F4_SOFTMAX_REGISTERS + F4_SERVICE_REGISTERS))
+            if (threads == F4_THREADS<2> && attributes.numRegs * threads < F4_SPLIT_REGISTERS)
                 return unica_fail(UNICA_B200_ERR_KERNEL, "attention_fp4: this build holds fewer registers per block than its setmaxnreg split needs");
-            if (cudaDeviceGetAttribute(&blocks, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
-            if (device < MAX_DEVICES) blocks_of[instance][device].store(blocks, std::memory_order_release);
+            if (device < F4_MAX_DEVICES) ready[instance][device].store(true, std::memory_order_release);
         }
-        launch_after(kernel, dim3(args.items.count < blocks ? args.items.count : blocks), F4_THREADS, smem, static_cast<cudaStream_t>(stream), overlapped, args);
+        launch_after(kernel, dim3(args.items.count < sms ? args.items.count : sms), threads, size_t(smem), static_cast<cudaStream_t>(stream), overlapped, args);
         return unica_check_launch("attention_fp4");
     };
-    return p_words ? launch(attention_fp4_kernel<true>, 1) : launch(attention_fp4_kernel<false>, 0);
+    // One query tile per block where that takes less time: a block takes two thirds of the time of a pair's for a key tile (1 head x 8192 tokens
+    // 126.0 -> 82.4 us, 4 x 1024 24.4 -> 17.9, 18 x 1024 25.1 -> 19.2; 16 x 1000 queries, 77 keys 9.6 -> 9.0), so it depends on the rounds that
+    // the blocks of either kind go.  Their results are the same.
+    const auto rounds = [&](long long items) { return (items + sms - 1) / sms; };
+    const bool single = !p_words && 2 * rounds(tiles * heads) < 3 * rounds(pairs * heads);
+    args.items.tiles = int(single ? tiles : pairs), args.items.allocated = int(2 * pairs), args.items.count = args.items.tiles * heads;
+    return single    ? launch(attention_fp4_kernel<1, false>, F4_THREADS<1>, int(sizeof(Fp4Smem<1>)) + 128, 2)
+           : p_words ? launch(attention_fp4_kernel<2, true>, F4_THREADS<2>, int(sizeof(Fp4Smem<2>)) + 128, 1)
+                     : launch(attention_fp4_kernel<2, false>, F4_THREADS<2>, int(sizeof(Fp4Smem<2>)) + 128, 0);
 }
 
 extern "C" int unica_b200_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4,
