@@ -13,7 +13,8 @@ int unica_check_launch(const char* what);  // cudaGetLastError after a launch ->
 int unica_check_device();                  // the current device must be compute capability 10.0 (cached per device)
 
 // Launches a kernel that begins with wait_for_previous_kernel(), overlapped with the end of the one before it in the stream
-// (which must be one of this library's that starts only when ITS predecessor is complete, or waits for it).
+// (one of this library's that starts only when ITS predecessor is complete, or waits for it, before it lets this one in; or, where the
+// kernel lets nobody in before its wait, any).
 template <typename... Params, typename... Args>
 cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool overlapped, Args&&... args) {
     cudaLaunchConfig_t config = {};
