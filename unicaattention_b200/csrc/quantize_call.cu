@@ -459,10 +459,10 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
         return UNICA_B200_OK;
     }
     const long long q_tiles = call.q.x ? static_cast<long long>(call.heads) * call.q.tiles : 0, kv_heads = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0);
-    // as in quantize_call_fp4: 32 heads x 777 50.6 -> 43.3 us a call, 40 x 1024 70.5 -> 62; the tiles of Q fill gaps, and where only
-    // they make a second wave (24 x 1000) four blocks per head were 2 us slower
+    // as in quantize_call_fp4, with four blocks per SM (36 x 1024 53.3 -> 52.3 us a call, 60 x 2048 222 -> 219.7; 32 x 777, rotated, 47.1 -> 49.5 with the
+    // line at four blocks); the tiles of Q fill gaps, and where only they make a second wave (24 x 1000) four blocks per head were 2 us slower
     const int keys = call.k.n_tokens > call.v.n_tokens ? call.k.n_tokens : call.v.n_tokens;  // (a call may have one of the two alone)
-    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= 4 * CALL_BLOCK && kv_heads * CALL_CLUSTER > 3 * 148;
+    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= (call.rope.table ? 4 : 8) * CALL_BLOCK && kv_heads * CALL_CLUSTER > 148 * (call.rope.table ? 3 : 4);
     const int cluster = four ? 4 : CALL_CLUSTER;
     if (keys > cluster * CALL_PARTS * CALL_BLOCK) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: more tokens than a cluster's blocks have room for");
     const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
@@ -486,11 +486,13 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
 
 int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
-    // Four blocks per head where a head's statistics are four 256-token blocks at most, if eight blocks per head are more than
-    // the chip takes at once: half of the eight have nothing to do in the first step, and a second wave costs its latency again
-    // (2 x 16 heads x 777 tokens, rotated: 41.7 -> 38 us, and 75.6 -> 68.1 for the call; 40 x 1024 not rotated 37 -> 30).
+    // Four blocks per head where a head's statistics are eight 256-token blocks at most, if eight blocks per head are more than
+    // the chip takes at once: some of the eight have little to do in the first step, and a second wave costs its latency again
+    // (2 x 16 heads x 777 tokens, rotated: 41.7 -> 38 us, 40 x 1024 not rotated 37 -> 30; calls of 20 x 2048 119.2 -> 113.3, 40 x 2048
+    // 185 -> 177.3, 16 x 777, rotated, which eight blocks per head do fit, 45.2 against 48.1).  Longer heads are better with eight (20 x 4128,
+    // rotated, 296.8 against 304.5; not rotated the same).
     const int longest = call.q.n_tokens > call.k.n_tokens ? call.q.n_tokens : call.k.n_tokens;
-    const bool four = longest <= 4 * CALL_BLOCK && 3 * call.heads * CALL_CLUSTER > 148 * (call.rope.table ? 2 : 3);
+    const bool four = longest <= (call.rope.table ? 4 : 8) * CALL_BLOCK && 3 * call.heads * CALL_CLUSTER > 148 * 3;
     auto launch = [&](auto half, auto rope) {
         constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
         const bool mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
