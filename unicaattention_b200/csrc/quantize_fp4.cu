@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(BIAS_THREADS, 1) smooth_bias_kernel(const __nv
         }
         __syncwarp();
     };
-    // one warp watches the barrier, everybody learns the outcome
+    // one warp watches the barrier, without naps (the block waits for it: 40 heads x 32760 keys 428 -> 420 us), everybody learns the outcome
     auto wait_done = [&](int half, int turn) {
-        return __syncthreads_and(warp != 0 || mbar_wait(&sm.done[half], turn & 1, abort_flag, status, STATUS_WAIT_SCORES)) != 0;
+        return __syncthreads_and(warp != 0 || mbar_wait<0>(&sm.done[half], turn & 1, abort_flag, status, STATUS_WAIT_SCORES)) != 0;
     };
     // warp w: the 32 keys of lane quarter w % 4, query blocks 16 (w / 4) .. + 15 of this pass
     auto write_out = [&](int pair, int turn) {
