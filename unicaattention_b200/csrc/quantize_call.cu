@@ -462,7 +462,9 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
     // as in quantize_call_fp4, with four blocks per SM (36 x 1024 53.3 -> 52.3 us a call, 60 x 2048 222 -> 219.7; 32 x 777, rotated, 47.1 -> 49.5 with the
     // line at four blocks); the tiles of Q fill gaps, and where only they make a second wave (24 x 1000) four blocks per head were 2 us slower
     const int keys = call.k.n_tokens > call.v.n_tokens ? call.k.n_tokens : call.v.n_tokens;  // (a call may have one of the two alone)
-    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= (call.rope.table ? 4 : 8) * CALL_BLOCK && kv_heads * CALL_CLUSTER > 148 * (call.rope.table ? 3 : 4);
+    // (Up to 256 keys one block has all statistics and four have a tile each: 16 x 200 19.2 -> 18.4, rotated 22.1 -> 18.8; up to 512 always: 4 x 512 17.0 -> 18.5.)
+    const bool crowded = kv_heads * CALL_CLUSTER > 148 * (call.rope.table ? 3 : 4);
+    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= (!crowded ? 1 : call.rope.table ? 4 : 8) * CALL_BLOCK;
     const int cluster = four ? 4 : CALL_CLUSTER;
     if (keys > cluster * CALL_PARTS * CALL_BLOCK) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: more tokens than a cluster's blocks have room for");
     const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
@@ -492,7 +494,9 @@ int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     // 185 -> 177.3, 16 x 777, rotated, which eight blocks per head do fit, 45.2 against 48.1).  Longer heads are better with eight (20 x 4128,
     // rotated, 296.8 against 304.5; not rotated the same).
     const int longest = call.q.n_tokens > call.k.n_tokens ? call.q.n_tokens : call.k.n_tokens;
-    const bool four = longest <= (call.rope.table ? 4 : 8) * CALL_BLOCK && 3 * call.heads * CALL_CLUSTER > 148 * 3;
+    // And up to 512 tokens in any case (4 x 256 21.8 -> 20.4, 12 x 500 32.5 -> 30.9, rotated 12 x 200 32.7 -> 30.8; 4 x 512 the same).
+    const bool crowded = 3 * call.heads * CALL_CLUSTER > 148 * 3;
+    const bool four = longest <= (!crowded ? 2 : call.rope.table ? 4 : 8) * CALL_BLOCK;
     auto launch = [&](auto half, auto rope) {
         constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
         const bool mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
