@@ -58,3 +58,17 @@ def test_what_a_plan_looks_at_in_every_call(monkeypatch):
             unica.attention(*bad)
     with pytest.raises(ValueError):
         unica.attention(q, k, v, NOPE=1)
+
+
+def test_a_changed_default(monkeypatch):
+    import unicaattention_b200 as unica
+
+    q, k, v = (t.cuda() for t in qkv(1, 4, 260, 77, seed=9))
+    per_channel, per_token = unica.attention(q, k, v), unica.attention(q, k, v, V_TOKEN=1)
+    assert not torch.equal(per_channel, per_token)
+    with monkeypatch.context() as patch:
+        patch.setitem(unica.TILE, "V_TOKEN", 1)
+        for _ in range(2):
+            assert torch.equal(unica.attention(q, k, v), per_token)
+            assert torch.equal(unica.attention(q, k, v, V_TOKEN=0), per_channel)
+    assert torch.equal(unica.attention(q, k, v), per_channel)

@@ -480,8 +480,10 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
     if inputs is None and rope is None and out is None and not peer_out and heads_per_call is _heads_per_call:
         # The usual call, of shapes, strides, types and settings that have been seen before: everything that follows from those is in
         # its plan (18 -> 10 us of host time a call, as long as the GPU takes for the smallest ones).
-        plan = _PLANS.get((kernel, q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.get_device(), k.get_device(),
-                           v.get_device(), *tile.items()))
+        try:
+            plan = _PLANS.get(_plan_key(kernel, q, k, v, TILE | tile))
+        except Exception:  # arguments that have no key: the checks below say what they always have
+            plan = None
         if plan is not None:
             planned = plan.run(q, k, v)
             if planned is not None:
@@ -572,7 +574,14 @@ class _Plan:
         return out
 
 
-_PLANS: dict = {}  # see attention() for the key
+_PLANS: dict = {}  # see _plan_key
+
+
+def _plan_key(kernel: str, q, k, v, settings: dict) -> tuple:
+    """What a plan follows from.  settings: the caller's and TILE's as it is in this call; by their types too, since what is equal need not be taken
+    alike (SMOOTH_Q=512.0 is refused)."""
+    return (kernel, q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.get_device(), k.get_device(), v.get_device(),
+            *settings, *settings.values(), *map(type, settings.values()))
 
 
 def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, tile: dict | None = None) -> bool:
@@ -609,7 +618,7 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
                                      n_peers, scale))
-    if rope is None and peers is None and tile is not None:
+    if rope is None and peers is None and tile is not None and all(isinstance(x, int) for x in settings.values()):
         # (readable() has let these strides pass, if not as they came then in a copy whose strides are a later call's: a plan asks for no copies)
         plan = _Plan()
         plan.device, plan.index, plan.size, plan.out_stride = device, device.index, size, os_
@@ -617,7 +626,7 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
         plan.fixed = lib.pack_call_tail(*layouts, *sizes, 0, scale)
         if len(_PLANS) > 4096:
             _PLANS.clear()
-        _PLANS[(kernel, q.shape, k.shape, v.shape, qs, ks, vs, q.dtype, k.dtype, v.dtype, device.index, k.get_device(), v.get_device(), *tile.items())] = plan
+        _PLANS[_plan_key(kernel, q, k, v, settings)] = plan
     return True
 
 
