@@ -72,3 +72,22 @@ def test_a_changed_default(monkeypatch):
             assert torch.equal(unica.attention(q, k, v), per_token)
             assert torch.equal(unica.attention(q, k, v, V_TOKEN=0), per_channel)
     assert torch.equal(unica.attention(q, k, v), per_channel)
+
+
+def test_only_plain_calls_leave_a_plan():
+    """A call with out= in another layout, or on tensors that are copied first, takes no plan: it must not leave one that plain calls cannot use either."""
+    import unicaattention_b200 as unica
+
+    q, k, v = (t.cuda() for t in qkv(1, 4, 260, 77, seed=10))
+    want = without_plans(unica, q, k, v)
+    (plan,) = unica._PLANS.values()
+    out = torch.empty(1, 260, 4, 128, dtype=q.dtype, device="cuda").transpose(1, 2)
+    assert torch.equal(unica.attention(q, k, v, out=out), want) and list(unica._PLANS.values()) == [plan]
+    assert plan.run(q, k, v) is not None
+    unica._PLANS.clear()
+    unica.attention(q, k, v, out=out)
+    odd = torch.cat([q.flatten(), q.flatten()[:8]])[1 : 1 + q.numel()].view(q.shape)  # two bytes off a 16-byte boundary
+    assert torch.equal(unica.attention(odd, k, v), without_plans(unica, odd.clone(), k, v))
+    unica._PLANS.clear()
+    unica.attention(odd, k, v)
+    assert not unica._PLANS

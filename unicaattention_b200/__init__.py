@@ -512,7 +512,9 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         rope_table(rope, batch, n_queries, n_keys)
     if inputs is None and heads_per_call(q, k, kernel, tile) < heads:
         return in_pieces(q, k, v, kernel, rope, tile, out, peer_out)
+    given = (q, k, v) if out is None else None
     q, k, v = readable(q), readable(k), readable(v)
+    plain = given is not None and q is given[0] and k is given[1] and v is given[2]
     if out is None:
         out = torch.empty_like(q)
     peers = (ctypes.c_void_p * len(peer_out))(*peer_out) if peer_out else None
@@ -520,7 +522,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         return out
     if inputs is None:
         try:
-            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out), tile):
+            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out), plain):
                 return out
             inputs = kernel_inputs(q, k, v, kernel, rope, **tile)
         except torch.cuda.OutOfMemoryError:
@@ -584,10 +586,11 @@ def _plan_key(kernel: str, q, k, v, settings: dict) -> tuple:
             *settings, *settings.values(), *map(type, settings.values()))
 
 
-def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, tile: dict | None = None) -> bool:
+def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, plain: bool = False) -> bool:
     """The whole call through one entry point of the library: quantization and kernel with their operands in one workspace.
     Bit for bit kernel_inputs() and the kernel, without their dozen allocations and trips through ctypes.  False: not
-    for this call (the outlier keys of a long V are found by torch)."""
+    for this call (the outlier keys of a long V are found by torch).
+    plain: the caller gave no out and tensors that are read in place, so a plan of this call serves the next one like it."""
     batch, heads, n_queries, _ = q.shape
     n_keys = k.shape[2]
     fast, smooth, outliers = kernel == "attention_fp4", settings["SMOOTH_Q"], 0
@@ -618,15 +621,14 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
                                      n_peers, scale))
-    if rope is None and peers is None and tile is not None and all(isinstance(x, int) for x in settings.values()):
-        # (readable() has let these strides pass, if not as they came then in a copy whose strides are a later call's: a plan asks for no copies)
+    if plain and rope is None and all(isinstance(x, int) for x in settings.values()) and (key := _plan_key(kernel, q, k, v, settings)) not in _PLANS:
         plan = _Plan()
         plan.device, plan.index, plan.size, plan.out_stride = device, device.index, size, os_
         plan.need = _call_bytes(batch, heads, n_queries, n_keys, settings["SMOOTH_Q"] if fast else 0)
         plan.fixed = lib.pack_call_tail(*layouts, *sizes, 0, scale)
         if len(_PLANS) > 4096:
             _PLANS.clear()
-        _PLANS[_plan_key(kernel, q, k, v, settings)] = plan
+        _PLANS[key] = plan
     return True
 
 
