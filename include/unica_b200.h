@@ -307,6 +307,11 @@ typedef struct {
 int unica_b200_attention_workspace(const unica_b200_call* call, size_t* bytes);
 int unica_b200_attention_call(const unica_b200_call* call, int* launches);
 
+/* Query rows that one of the fast kernel's persistent blocks takes at a time, for a call of `heads` (batch * heads) on a device with `sms`
+ * SMs: 256 (two tiles sharing every key tile), or 128 where that takes less time (two thirds of the time per key tile).  0 for arguments that
+ * are not positive.  Makes no CUDA call. */
+int unica_b200_fast_item_rows(int heads, int n_queries, int sms);
+
 /* V in INT8 per channel without each head's n_outliers (1..8) keys of largest max |v| (ties: the lower key), which are written
  * as zeros: what quantize_v(outliers=..) makes of n_tokens <= 8192 (unica/__init__.py:384-399, 420-432), in one launch.
  * keys [heads][n_outliers] (-1: the head has fewer keys), rows float [heads][n_outliers][128]: V over the scale. */

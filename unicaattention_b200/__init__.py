@@ -171,20 +171,21 @@ def block_stats(x: torch.Tensor, rope: torch.Tensor | None = None) -> torch.Tens
 
 def wave_layout(heads: int, n_queries: int, n_keys: int, v_token: int, device) -> dict:
     """The reference picks between a 4-warp and an 8-warp block per call to fill its last wave (unica/__init__.py:281-285).
-    Here every kernel has one block shape, persistent and one per SM, each taking tiles in turn (accurate: 128 queries, 16
-    warps; fast: two such tiles, 20 warps), so there is nothing to pick: always {}.  What the last round costs is what
-    wave_plan() reports."""
+    Here blocks are persistent and one per SM, each taking tiles in turn (accurate: 128 queries, 16 warps; fast: two such tiles, 20
+    warps, or one, 12 warps, which the launch picks by itself), so there is nothing to pick: always {}.  What the last round
+    costs is what wave_plan() reports."""
     return {}
 
 
 def wave_plan(heads: int, n_queries: int, kernel: str = DEFAULT_KERNEL, device=None) -> dict:
     """How a call's items (query tiles, or pairs of them) fall on the SMs' persistent blocks: blocks (items, all of equal
-    length: every query tile meets every key), blocks per wave (one per SM), waves, and the share of the SM time of those waves that does work.  batch * heads for `heads`."""
-    rows = 256 if kernel == "attention_fp4" else 128
-    blocks = heads * math.ceil(n_queries / rows)
+    length: every query tile meets every key), blocks per wave (one per SM), waves, and the share of the SM time of those waves that does work;
+    rows: queries per item, which the fast kernel picks per call (items of 128 take two thirds of the time of items of 256).  batch * heads for `heads`."""
     per_wave = sm_count(torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device))
+    rows = lib.library().unica_b200_fast_item_rows(heads, n_queries, per_wave) if kernel == "attention_fp4" else 128
+    blocks = heads * math.ceil(n_queries / rows)
     waves = math.ceil(blocks / per_wave)
-    return {"blocks": blocks, "per_wave": per_wave, "waves": waves, "efficiency": blocks / (waves * per_wave)}
+    return {"blocks": blocks, "per_wave": per_wave, "waves": waves, "efficiency": blocks / (waves * per_wave), "rows": rows}
 
 
 def source(kernel: str, tile: dict) -> str:

@@ -585,6 +585,15 @@ using namespace unica;
 
 static constexpr int F4_MAX_DEVICES = 64;
 
+// One query tile per block where that takes less time: a block takes two thirds of the time of a pair's for a key tile (1 head x 8192 tokens
+// 126.0 -> 82.4 us, 4 x 1024 24.4 -> 17.9, 18 x 1024 25.1 -> 19.2; 16 x 1000 queries, 77 keys 9.6 -> 9.0), so it depends on the rounds that
+// the blocks of either kind go.  Their results are the same.
+extern "C" int unica_b200_fast_item_rows(int heads, int n_queries, int sms) {
+    if (heads <= 0 || n_queries <= 0 || sms <= 0) return 0;
+    const auto rounds = [&](int rows) { return ((n_queries + rows - 1LL) / rows * heads + sms - 1) / sms; };
+    return 2 * rounds(QUERY_TILE) < 3 * rounds(2 * QUERY_TILE) ? QUERY_TILE : 2 * QUERY_TILE;
+}
+
 // SMs of the current device; asked for once per device.
 static int sm_count(int* sms) {
     static std::atomic<int> known[F4_MAX_DEVICES];
@@ -638,11 +647,7 @@ int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, c
         launch_after(kernel, dim3(args.items.count < sms ? args.items.count : sms), threads, size_t(smem), static_cast<cudaStream_t>(stream), overlapped, args);
         return unica_check_launch("attention_fp4");
     };
-    // One query tile per block where that takes less time: a block takes two thirds of the time of a pair's for a key tile (1 head x 8192 tokens
-    // 126.0 -> 82.4 us, 4 x 1024 24.4 -> 17.9, 18 x 1024 25.1 -> 19.2; 16 x 1000 queries, 77 keys 9.6 -> 9.0), so it depends on the rounds that
-    // the blocks of either kind go.  Their results are the same.
-    const auto rounds = [&](long long items) { return (items + sms - 1) / sms; };
-    const bool single = !p_words && 2 * rounds(tiles * heads) < 3 * rounds(pairs * heads);
+    const bool single = !p_words && unica_b200_fast_item_rows(heads, n_queries, sms) == QUERY_TILE;
     args.items.tiles = int(single ? tiles : pairs), args.items.allocated = int(2 * pairs), args.items.count = args.items.tiles * heads;
     return single    ? launch(attention_fp4_kernel<1, false>, F4_THREADS<1>, int(sizeof(Fp4Smem<1>)) + 128, 2)
            : p_words ? launch(attention_fp4_kernel<2, true>, F4_THREADS<2>, int(sizeof(Fp4Smem<2>)) + 128, 1)

@@ -62,7 +62,13 @@ def attention_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
         # the largest group: about an eighth of the heads, picked so that its blocks fill their last wave of SMs well
         kernel = settings.get("kernel", unica.DEFAULT_KERNEL)
         candidates = range(max(1, -(-heads // 10)), max(1, -(-heads // 6)) + 1)
-        largest = max(candidates, key=lambda g: (round(unica.wave_plan(batch * g, q.shape[2], kernel, device)["efficiency"], 2), g))
+        whole = 256 if kernel == "attention_fp4" else 128
+
+        def worth(g: int) -> float:
+            plan = unica.wave_plan(batch * g, q.shape[2], kernel, device)
+            return round(plan["efficiency"] * (1 if plan["rows"] == whole else 0.75), 2)  # (items of half the rows take two thirds of the time)
+
+        largest = max(candidates, key=lambda g: (worth(g), g))
         sizes = group_sizes(heads, largest)
     else:
         sizes = [min(heads_per_group, heads - f) for f in range(0, heads, heads_per_group)]

@@ -63,6 +63,7 @@ SIGNATURES = {
     "unica_b200_quantize_v_int8_outliers": [_P, TokenLayout, _I, _I, _I, _P, _P, _P, _P, _P],
     "unica_b200_attention_workspace": [_P, _P],
     "unica_b200_attention_call": [_P, _P],
+    "unica_b200_fast_item_rows": [_I, _I, _I],
 }
 # struct unica_b200_call as bytes, in the header's order (packing forty numbers at once costs a microsecond, filling a
 # ctypes structure several): q, k, v, out, workspace, its size, rope, its batch stride, peer_out, status, stream; the four
