@@ -139,11 +139,16 @@ __device__ __forceinline__ float4 load_result4(const float* p) {
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
     return v;
 }
-// The same for a const __restrict__ pointer: loads through it cannot be moved above this, which stands behind the wait.
+// The same for a const __restrict__ pointer, or for an index that an address is made with: loads cannot be moved above this, which stands
+// behind the wait.
 template <typename T>
 __device__ __forceinline__ T* behind_wait(T* p) {
     asm volatile("" : "+l"(p) : : "memory");
     return p;
+}
+__device__ __forceinline__ int behind_wait(int i) {
+    asm volatile("" : "+r"(i) : : "memory");
+    return i;
 }
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 

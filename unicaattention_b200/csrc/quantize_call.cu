@@ -265,8 +265,10 @@ struct SkipKeys {
 
 // The kernel is launched to overlap the end of the kernel before it in the stream, whatever that is: its blocks are set up while that one's
 // results are being written back (a loop of 4 heads x 1024 tokens 24.7 -> 22.7 us a call, 2 x 8 x 1000 queries with 77 keys 22.6 -> 20.4).
-// Nothing is read or written before the wait, and the call's next kernel is let in only after it: its blocks take tensor memory, which a
-// kernel before the call may not have taken yet.
+// Nothing is read or written before the wait: the addresses of all that is read follow from a head or a pointer that comes out of behind_wait
+// (in INT8 from the head: with q's, k's and v's pointers, as in NVFP4, calls of 1 head x 8192 tokens per channel took 106.6 us, not 103.4).  And the call's next
+// kernel is let in only after it, for two reasons: its blocks take tensor memory, which a kernel before the call may not have taken yet; and
+// smooth_bias_few_kernel reads K before a wait of its own, which is as early as K is sure to be there.
 __device__ __forceinline__ void begin_call() {
     wait_for_previous_kernel();
     let_next_kernel_start();
@@ -283,11 +285,10 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     const int rank = int(blockIdx.x) % CLUSTER, clusters_k = call.k.x ? call.heads : 0, clusters_v = call.v.x ? call.heads : 0;
     int cluster = int(blockIdx.x) / CLUSTER;
     if (cluster < clusters_k) {
-        CallOperand op = call.k;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.k;
         TokenLayout in = op.in;
         in.half = HALF;
-        const int head = cluster;
+        const int head = behind_wait(cluster);
         head_stats<true, false, CLUSTER, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
         for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
@@ -296,48 +297,48 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
                                                          static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
         }
     } else if ((cluster -= clusters_k) < clusters_v) {
-        CallOperand op = call.v;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.v;
         TokenLayout in = op.in;
         in.half = HALF;
-        const int head = cluster;
+        constexpr bool OUTLIERS = V_MODE == UNICA_B200_V_OUTLIERS;  // (of the two, what costs them less: 1 x 1024 33.7 us a call with the head, 33.0 with the pointer)
+        const __nv_bfloat16* x = OUTLIERS ? behind_wait(op.x) : op.x;
+        const int head = OUTLIERS ? cluster : behind_wait(cluster);
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
             for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t)
-                v_int8_tile<decltype(per_token)::value>(op.x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale, call.v_token,
+                v_int8_tile<decltype(per_token)::value>(x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale, call.v_token,
                                                         sm.v_tile[t & 1]);
         };
         if constexpr (V_MODE == UNICA_B200_V_TOKEN) {
             tiles(std::true_type{}, NoSkip{});
         } else if constexpr (V_MODE == UNICA_B200_V_OUTLIERS) {
-            find_outliers(op.x, in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
+            find_outliers(x, in, head, op.n_tokens, call.n_outliers, rank, sm.candidates, outliers);
             const SkipKeys skip{outliers.is_outlier};
-            head_stats<false, true, CLUSTER>(op.x, in, none, skip, head, op.n_tokens, rank, sm);
+            head_stats<false, true, CLUSTER>(x, in, none, skip, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, skip);
             if (rank == 0) {  // the outliers' rows over the channel scales
                 for (int i = threadIdx.x; i < call.n_outliers * HEAD_DIM; i += CALL_THREADS) {
                     const int o = i / HEAD_DIM, c = i % HEAD_DIM, key = outliers.keys[o];
                     const float s = fmaxf(fmaxf(sm.high[c], -sm.low[c]) * (1.0f / 127.0f), 1e-12f);
-                    float x = 0.0f;
+                    float value = 0.0f;
                     if (key >= 0) {
-                        const __nv_bfloat16* src = op.x + in.offset(head, key) + c;
-                        x = HALF ? __bfloat162float(__float2bfloat16_rn(__half2float(*reinterpret_cast<const __half*>(src)))) : __bfloat162float(*src);
+                        const __nv_bfloat16* src = x + in.offset(head, key) + c;
+                        value = HALF ? __bfloat162float(__float2bfloat16_rn(__half2float(*reinterpret_cast<const __half*>(src)))) : __bfloat162float(*src);
                     }
-                    call.outlier_rows[(size_t(head) * call.n_outliers) * HEAD_DIM + i] = __fdiv_rn(x, s);
+                    call.outlier_rows[(size_t(head) * call.n_outliers) * HEAD_DIM + i] = __fdiv_rn(value, s);
                     if (c == 0) call.outlier_keys[size_t(head) * call.n_outliers + o] = key;
                 }
             }
         } else {
-            head_stats<false, true, CLUSTER>(op.x, in, none, NoSkip{}, head, op.n_tokens, rank, sm);
+            head_stats<false, true, CLUSTER>(x, in, none, NoSkip{}, head, op.n_tokens, rank, sm);
             tiles(std::false_type{}, NoSkip{});
         }
     } else {
         cluster -= clusters_v;
-        CallOperand op = call.q;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.q;
         TokenLayout in = op.in;
         in.half = HALF;
-        const int tile = cluster * CLUSTER + rank, head = tile / op.tiles, t = tile % op.tiles;
+        const int tile = behind_wait(cluster * CLUSTER + rank), head = tile / op.tiles, t = tile % op.tiles;
         if (head < call.heads) {
             int8_t* codes = reinterpret_cast<int8_t*>(op.codes) + size_t(tile) * (QUERY_TILE * HEAD_DIM);
             float* scale = static_cast<float*>(op.scales) + tile;
@@ -366,11 +367,11 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     const int rank = int(blockIdx.x) % CLUSTER;
     const int kind = int(blockIdx.x) / CLUSTER / call.heads, head = int(blockIdx.x) / CLUSTER % call.heads;
     if (kind == 0) {
-        CallOperand op = call.k;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.k;
+        const __nv_bfloat16* x = behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
-        head_stats<true, true, CLUSTER, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, true, CLUSTER, ROPE ? 4 : 8>(x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
             const float m = sm.mean[threadIdx.x];
@@ -381,24 +382,24 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         if (rank == 0 && threadIdx.x == 0) op.outer[head] = outer.value;
         for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {  // (no barrier in a tile: the warps run ahead of one another)
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<KEY_TILE, true, ROPE>(op.x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
+            rows_fp4_tile<KEY_TILE, true, ROPE>(x, in, [&](int) { return sm.mean; }, outer, head, t, op.n_tokens, op.codes + tile * (KEY_TILE * HEAD_DIM / 2),
                                           static_cast<uint8_t*>(op.scales) + tile * (KEY_TILE * 8), rope);
         }
     } else if (kind == 1) {
-        CallOperand op = call.v;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.v;
+        const __nv_bfloat16* x = behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
-        head_stats<false, true, CLUSTER>(op.x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<false, true, CLUSTER>(x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
         for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            v_fp4_tile(op.x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
+            v_fp4_tile(x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
                        op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
         }
     } else {
         // Q: a mean per group of `smooth` tokens, whole groups per block
-        CallOperand op = call.q;
-        op.x = behind_wait(op.x);
+        const CallOperand& op = call.q;
+        const __nv_bfloat16* x = behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
         const int groups = (op.n_tokens + call.smooth - 1) / call.smooth, per = call.smooth / CALL_BLOCK, blocks = (op.n_tokens + CALL_BLOCK - 1) / CALL_BLOCK;
@@ -407,7 +408,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
             float s = 0.0f, lo = INFINITY, hi = -INFINITY;
             const int b1 = min((g + 1) * per, blocks);
             for (int b = g * per; b < b1; ++b) {
-                block_stats<true, true, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
+                block_stats<true, true, ROPE ? 4 : 8>(x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
                 if (threadIdx.x < HEAD_DIM)
                     s += sm.part[0][0][threadIdx.x], lo = fminf(lo, sm.part[0][1][threadIdx.x]), hi = fmaxf(hi, sm.part[0][2][threadIdx.x]);
                 __syncthreads();
@@ -433,7 +434,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         __syncthreads();
         for (int t = t0; t < t1; ++t) {
             const size_t tile = size_t(head) * op.tiles + t;
-            rows_fp4_tile<QUERY_TILE, false, ROPE>(op.x, in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
+            rows_fp4_tile<QUERY_TILE, false, ROPE>(x, in, [&](int token) { return q_means[token / call.smooth - g0]; }, outer, head, t, op.n_tokens,
                                              op.codes + tile * (QUERY_TILE * HEAD_DIM / 2), static_cast<uint8_t*>(op.scales) + tile * (QUERY_TILE * 8), rope);
         }
     }
