@@ -97,7 +97,7 @@ def on_their_device(function):
 
     @functools.wraps(function)
     def run(q, *args, **kwargs):
-        if q.is_cuda and q.device.index == torch.cuda.current_device():  # already so: the usual case, and entering it again costs 3 us
+        if q.is_cuda and q.get_device() == torch._C._cuda_getDevice():  # already so: the usual case, and entering it again costs 3 us
             return function(q, *args, **kwargs)
         with torch.cuda.device(q.device):
             return function(q, *args, **kwargs)
@@ -482,7 +482,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         # The usual call, of shapes, strides, types and settings that have been seen before: everything that follows from those is in
         # its plan (18 -> 10 us of host time a call, as long as the GPU takes for the smallest ones).
         try:
-            plan = _PLANS.get(_plan_key(kernel, q, k, v, TILE | tile))
+            plan = _PLANS.get(_plan_key(kernel, q, k, v, tile))
         except Exception:  # arguments that have no key: the checks below say what they always have
             plan = None
         if plan is not None:
@@ -523,7 +523,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
         return out
     if inputs is None:
         try:
-            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out), plain):
+            if _attention_call(q, k, v, out, kernel, settings, rope, peers, len(peer_out), tile if plain else None):
                 return out
             inputs = kernel_inputs(q, k, v, kernel, rope, **tile)
         except torch.cuda.OutOfMemoryError:
@@ -580,18 +580,18 @@ class _Plan:
 _PLANS: dict = {}  # see _plan_key
 
 
-def _plan_key(kernel: str, q, k, v, settings: dict) -> tuple:
-    """What a plan follows from.  settings: the caller's and TILE's as it is in this call; by their types too, since what is equal need not be taken
-    alike (SMOOTH_Q=512.0 is refused)."""
+def _plan_key(kernel: str, q, k, v, tile: dict) -> tuple:
+    """What a plan follows from: the settings by their types too, since what is equal need not be taken alike (SMOOTH_Q=512.0 is refused), and
+    the defaults as they are now."""
     return (kernel, q.shape, k.shape, v.shape, q.stride(), k.stride(), v.stride(), q.dtype, k.dtype, v.dtype, q.get_device(), k.get_device(), v.get_device(),
-            *settings, *settings.values(), *map(type, settings.values()))
+            *tile.items(), *map(type, tile.values()), *TILE.values())
 
 
-def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, plain: bool = False) -> bool:
+def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_peers: int, plain: dict | None = None) -> bool:
     """The whole call through one entry point of the library: quantization and kernel with their operands in one workspace.
     Bit for bit kernel_inputs() and the kernel, without their dozen allocations and trips through ctypes.  False: not
     for this call (the outlier keys of a long V are found by torch).
-    plain: the caller gave no out and tensors that are read in place, so a plan of this call serves the next one like it."""
+    plain: the caller's settings, where there was no out and tensors that are read in place: a plan of this call then serves the next one like it."""
     batch, heads, n_queries, _ = q.shape
     n_keys = k.shape[2]
     fast, smooth, outliers = kernel == "attention_fp4", settings["SMOOTH_Q"], 0
@@ -622,7 +622,7 @@ def _attention_call(q, k, v, out, kernel: str, settings: dict, rope, peers, n_pe
     workspace = torch.empty(size, dtype=torch.uint8, device=device)
     lib.attention_call(lib.pack_call(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), workspace.data_ptr(), size, *where, *layouts, *sizes,
                                      n_peers, scale))
-    if plain and rope is None and all(isinstance(x, int) for x in settings.values()) and (key := _plan_key(kernel, q, k, v, settings)) not in _PLANS:
+    if plain is not None and rope is None and all(isinstance(x, int) for x in settings.values()) and (key := _plan_key(kernel, q, k, v, plain)) not in _PLANS:
         plan = _Plan()
         plan.device, plan.index, plan.size, plan.out_stride = device, device.index, size, os_
         plan.need = _call_bytes(batch, heads, n_queries, n_keys, settings["SMOOTH_Q"] if fast else 0)
