@@ -594,19 +594,6 @@ extern "C" int unica_b200_fast_item_rows(int heads, int n_queries, int sms) {
     return 2 * rounds(QUERY_TILE) < 3 * rounds(2 * QUERY_TILE) ? QUERY_TILE : 2 * QUERY_TILE;
 }
 
-// SMs of the current device; asked for once per device.
-static int sm_count(int* sms) {
-    static std::atomic<int> known[F4_MAX_DEVICES];
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
-    *sms = device < F4_MAX_DEVICES ? known[device].load(std::memory_order_relaxed) : 0;
-    if (*sms == 0) {
-        if (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("attention_fp4 (device)");
-        if (device < F4_MAX_DEVICES) known[device].store(*sms, std::memory_order_relaxed);
-    }
-    return UNICA_B200_OK;
-}
-
 int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, const void* sfk, const uint8_t* v4, const void* sfv,
                          const float* qk_outer, const float* k_outer, const float* v_outer, const float* bias, int q_blocks, int smooth_q, void* out,
                          void* const* peer_out, int n_peers, unica_token_layout out_layout, int heads, int n_queries, int n_keys,
@@ -628,7 +615,7 @@ int unica_attention_fp4(const uint8_t* q4, const void* sfq, const uint8_t* k4, c
     const long long pairs = (n_queries + 2 * QUERY_TILE - 1) / (2 * QUERY_TILE), tiles = (n_queries + QUERY_TILE - 1) / QUERY_TILE;  // Q4 holds an even number of tiles
     if (pairs * heads > INT_MAX / 2) return unica_fail(UNICA_B200_ERR_ARGUMENT, "attention_fp4: more than 2^30 pairs of query tiles");
     int sms = 0;  // persistent blocks, one per SM
-    if (int e = sm_count(&sms)) return e;
+    if (int e = unica_sm_count(&sms)) return e;
     auto launch = [&](auto kernel, int threads, int smem, int instance) -> int {
         // Set up once per kernel instance and device, as in attention_int8.cu.
         static std::atomic<bool> ready[3][F4_MAX_DEVICES];

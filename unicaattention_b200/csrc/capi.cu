@@ -38,5 +38,18 @@ int unica_check_device() {
     return UNICA_B200_OK;
 }
 
+int unica_sm_count(int* sms) {
+    constexpr int MAX_DEVICES = 64;
+    static std::atomic<int> known[MAX_DEVICES];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return unica_fail(UNICA_B200_ERR_CUDA, "cannot query the current CUDA device");
+    *sms = device < MAX_DEVICES ? known[device].load(std::memory_order_relaxed) : 0;
+    if (*sms == 0) {
+        if (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return unica_check_launch("sm_count");
+        if (device < MAX_DEVICES) known[device].store(*sms, std::memory_order_relaxed);
+    }
+    return UNICA_B200_OK;
+}
+
 extern "C" const char* unica_b200_last_error(void) { return g_error; }
 extern "C" int unica_b200_version(void) { return 1; }

@@ -11,6 +11,7 @@
 int unica_fail(int code, const char* message);
 int unica_check_launch(const char* what);  // cudaGetLastError after a launch -> 0 or UNICA_B200_ERR_CUDA
 int unica_check_device();                  // the current device must be compute capability 10.0 (cached per device)
+int unica_sm_count(int* sms);              // of the current device (cached per device)
 
 // Launches a kernel that begins with wait_for_previous_kernel(), overlapped with the end of the one before it in the stream
 // (one of this library's that starts only when ITS predecessor is complete, or waits for it, before it lets this one in; or, where the

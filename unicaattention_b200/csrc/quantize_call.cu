@@ -1,22 +1,24 @@
 // The quantization of a short call (up to CALL_TOKENS tokens) in ONE launch: Q, K and V of all heads, statistics included.
 //
 // The separate passes need three to eight launches for this, each a few microseconds on the device and as many on the host:
-// for 4 heads x 1024 tokens that was most of the call.  Here the grid is made of clusters of eight blocks (four for many short heads), each of which is
+// for 4 heads x 1024 tokens that was most of the call.  Here the grid is made of clusters of eight blocks (four for short heads, see the host code), each of which is
 // given a head's K, a head's V or (NVFP4) a head's Q, and in INT8 eight tiles of Q, which need no statistics:
 //   1. the blocks of a cluster take the statistics of an eighth of the head's 256-token blocks each,
 //   2. they read one another's partial results through distributed shared memory, all in the same order,
 //   3. and quantize an eighth of the head's tiles each; the tokens come out of L2 now.
 // What bounds it: latency.  For few tokens two dependent trips to memory and a cluster barrier each way; at 30 heads x 4128 tokens every
-// block alternates between loads and conversions, with a third of the chip's warps in flight (issue 37 % busy).  Hence as many blocks
-// per SM as their registers allow, four for INT8 (64 registers; the clusters of K and V of that size are then on the GPU together) and
-// three for NVFP4 and rotated rows, with nothing loaded ahead of a tile, which the other blocks make up for (a call of 30 x 4128 per
-// token 375.6 -> 367.9 us, with outliers 380.3 -> 362.4); minima and maxima are taken on bfloat16 pairs, and outliers are looked for
-// by all warps.
+// block alternates between loads and conversions, with a third of the chip's warps in flight (issue 37 % busy).  So where there are blocks
+// enough, four share an SM in INT8 (64 registers, some 110 bytes of them spilled in bfloat16; the clusters of K and V of that size are then on the GPU together) and
+// three in NVFP4 and rotated (80 registers; rotated rows spill 130 to 180 bytes), with nothing loaded ahead of a tile, which the other blocks make
+// up for: a call of 30 x 4128 per token 376.8 -> 370.3 us, with outliers 381.7 -> 363.0.  Where there are not (AHEAD, see quantize_call_int8 and
+// quantize_call_fp4), a block has more registers, the next tile under way while it works on one, and rotated twice the tokens in flight in the
+// statistics.  Minima and maxima are taken on bfloat16 pairs, and outliers are looked for by all warps.
 //
 // Sums run in the order of channel_stats_kernel and its finish kernel (quantize.cu), minima and maxima are exact: the
 // operands are bit for bit those of the separate passes.
 #include <cooperative_groups.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "quantize_call.h"
@@ -263,6 +265,27 @@ struct SkipKeys {
     __device__ __forceinline__ bool operator()(int token) const { return (is_outlier[token / 32] >> (token % 32)) & 1; }
 };
 
+// Tiles first .. last - 1 in order; AHEAD: each loaded while the one before is worked on.
+template <bool AHEAD, typename Raw, typename Load, typename Finish>
+__device__ __forceinline__ void each_tile(int first, int last, Load load, Finish finish) {
+    if constexpr (AHEAD) {
+        if (first >= last) return;
+        Raw raw, next;
+        load(raw, first);
+        for (int t = first; t < last; ++t) {
+            if (t + 1 < last) load(next, t + 1);
+            finish(raw, t);
+            raw = next;
+        }
+    } else {
+        for (int t = first; t < last; ++t) {
+            Raw raw;
+            load(raw, t);
+            finish(raw, t);
+        }
+    }
+}
+
 // The kernel is launched to overlap the end of the kernel before it in the stream, whatever that is: its blocks are set up while that one's
 // results are being written back (a loop of 4 heads x 1024 tokens 24.7 -> 22.7 us a call, 2 x 8 x 1000 queries with 77 keys 22.6 -> 20.4).
 // Nothing is read or written before the wait: the addresses of all that is read follow from a head or a pointer that comes out of behind_wait
@@ -283,9 +306,9 @@ static bool capturing(cudaStream_t stream) {
 }
 
 // V_MODE: UNICA_B200_V_*; HALF, ROPE: the input is float16, Q and K are rotated (template parameters so that the other calls
-// carry none of it).  Clusters: heads of K, heads of V, then CLUSTER tiles of Q each.
-template <int V_MODE, bool HALF, bool ROPE, int CLUSTER>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE ? 3 : 4) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
+// carry none of it); AHEAD: see each_tile.  Clusters: heads of K, heads of V, then CLUSTER tiles of Q each.
+template <int V_MODE, bool HALF, bool ROPE, int CLUSTER, bool AHEAD>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE || AHEAD ? 3 : 4) quantize_call_int8_kernel(const __grid_constant__ CallQuantize call) {
     begin_call();
     __shared__ CallStats sm;
     __shared__ CallOutliers outliers;
@@ -299,11 +322,14 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         const int head = behind_wait(cluster);
         head_stats<true, false, CLUSTER, ROPE ? 4 : 8>(op.x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         if (rank == 0 && threadIdx.x < HEAD_DIM) op.mean[size_t(head) * HEAD_DIM + threadIdx.x] = sm.mean[threadIdx.x];
-        for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
-            const size_t tile = size_t(head) * op.tiles + t;
-            rows_int8_tile<KEY_TILE, CALL_THREADS, ROPE>(op.x, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
-                                                         static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
-        }
+        each_tile<AHEAD, RowsRaw<KEY_TILE>>(
+            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1),
+            [&](auto& raw, int t) { rows_load<KEY_TILE, CALL_THREADS, ROPE>(raw, op.x, in, head, t, op.n_tokens); },
+            [&](const auto& raw, int t) {
+                const size_t tile = size_t(head) * op.tiles + t;
+                rows_int8_finish<KEY_TILE, CALL_THREADS, ROPE>(raw, in, sm.mean, head, t, op.n_tokens, reinterpret_cast<int8_t*>(op.codes) + tile * (KEY_TILE * HEAD_DIM),
+                                                               static_cast<float*>(op.scales) + tile, rope, sm.scratch[t & 1]);
+            });
     } else if ((cluster -= clusters_k) < clusters_v) {
         const CallOperand& op = call.v;
         TokenLayout in = op.in;
@@ -313,9 +339,12 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         const int head = OUTLIERS ? cluster : behind_wait(cluster);
         float* scale = static_cast<float*>(op.scales);
         auto tiles = [&](auto per_token, auto skip) {
-            for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t)
-                v_int8_tile<decltype(per_token)::value>(x, in, sm.low, sm.high, skip, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale, call.v_token,
-                                                        sm.v_tile[t & 1]);
+            each_tile<AHEAD, VRaw>(
+                share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_load(raw, x, in, skip, head, t, op.n_tokens); },
+                [&](const auto& raw, int t) {
+                    v_int8_finish<decltype(per_token)::value>(raw, sm.low, sm.high, head, t, op.tiles, op.n_tokens, reinterpret_cast<int8_t*>(op.codes), scale,
+                                                              call.v_token, sm.v_tile[t & 1]);
+                });
         };
         if constexpr (V_MODE == UNICA_B200_V_TOKEN) {
             tiles(std::true_type{}, NoSkip{});
@@ -363,23 +392,24 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
 __device__ __forceinline__ float outer_scale(float amax) { return fmaxf(amax * (1.0f / 2688.0f), 1e-30f); }
 
 // HALF: the inputs are float16 (1) or bfloat16 (0), or each what its layout says.  Clusters: heads of K, of V, of Q.  Rotated inputs load their
-// angles too, and half as many tokens at a time in the statistics, so that three blocks fit an SM (2 x 16 heads x 777 tokens: with two blocks
-// and eight tokens 61.5 us a call, with three and four 56.1; with three and eight, spilling, 59.4).
+// angles too, and without AHEAD half as many tokens at a time in the statistics, so that three blocks fit an SM (2 x 16 heads x 777 tokens: with two blocks
+// and eight tokens 61.5 us a call, with three and four 56.1; with three and eight, which spills more, 59.4).
 constexpr int EACH_ITS_OWN = 2;
-template <int HALF, bool ROPE, int CLUSTER>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
+template <int HALF, bool ROPE, int CLUSTER, bool AHEAD>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, ROPE && AHEAD ? 2 : 3) quantize_call_fp4_kernel(const __grid_constant__ CallQuantize call) {
     begin_call();
     __shared__ CallStats sm;
     __shared__ float q_means[CALL_GROUPS][HEAD_DIM], q_amax;
     const RopeTable rope = ROPE ? call.rope : RopeTable{nullptr, 0};
     const int rank = int(blockIdx.x) % CLUSTER;
-    const int kind = int(blockIdx.x) / CLUSTER / call.heads, head = int(blockIdx.x) / CLUSTER % call.heads;
+    const int kind = int(blockIdx.x) / CLUSTER / call.heads, any_head = int(blockIdx.x) / CLUSTER % call.heads;
+    const int head = AHEAD ? behind_wait(any_head) : any_head;  // (of the two, what costs less: 40 x 128 28.9 us a call with the pointers, 29.9 with the head; 4 x 8192 182.1 and 179.4)
     if (kind == 0) {
         const CallOperand& op = call.k;
-        const __nv_bfloat16* x = behind_wait(op.x);
+        const __nv_bfloat16* x = AHEAD ? op.x : behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
-        head_stats<true, true, CLUSTER, ROPE ? 4 : 8>(x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
+        head_stats<true, true, CLUSTER, ROPE && !AHEAD ? 4 : 8>(x, in, rope, NoSkip{}, head, op.n_tokens, rank, sm);
         float amax = 0.0f;
         if (threadIdx.x < HEAD_DIM) {
             const float m = sm.mean[threadIdx.x];
@@ -395,19 +425,21 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
         }
     } else if (kind == 1) {
         const CallOperand& op = call.v;
-        const __nv_bfloat16* x = behind_wait(op.x);
+        const __nv_bfloat16* x = AHEAD ? op.x : behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
         head_stats<false, true, CLUSTER>(x, in, RopeTable{nullptr, 0}, NoSkip{}, head, op.n_tokens, rank, sm);
-        for (int t = share<CLUSTER>(op.tiles, rank); t < share<CLUSTER>(op.tiles, rank + 1); ++t) {
-            const size_t tile = size_t(head) * op.tiles + t;
-            v_fp4_tile(x, in, sm.low, sm.high, head, t, op.n_tokens, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
-                       op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
-        }
+        each_tile<AHEAD, VRaw>(
+            share<CLUSTER>(op.tiles, rank), share<CLUSTER>(op.tiles, rank + 1), [&](auto& raw, int t) { v_fp4_load(raw, x, in, head, t, op.n_tokens); },
+            [&](const auto& raw, int t) {
+                const size_t tile = size_t(head) * op.tiles + t;
+                v_fp4_finish(raw, sm.low, sm.high, t, op.codes + tile * (V4_ROWS * 32), static_cast<uint8_t*>(op.scales) + tile * (V4_SF_WORDS * 4),
+                             op.outer + size_t(head) * HEAD_DIM, sm.v4_tile[t & 1]);
+            });
     } else {
         // Q: a mean per group of `smooth` tokens, whole groups per block
         const CallOperand& op = call.q;
-        const __nv_bfloat16* x = behind_wait(op.x);
+        const __nv_bfloat16* x = AHEAD ? op.x : behind_wait(op.x);
         TokenLayout in = op.in;
         if (HALF != EACH_ITS_OWN) in.half = HALF;
         const int groups = (op.n_tokens + call.smooth - 1) / call.smooth, per = call.smooth / CALL_BLOCK, blocks = (op.n_tokens + CALL_BLOCK - 1) / CALL_BLOCK;
@@ -416,7 +448,7 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
             float s = 0.0f, lo = INFINITY, hi = -INFINITY;
             const int b1 = min((g + 1) * per, blocks);
             for (int b = g * per; b < b1; ++b) {
-                block_stats<true, true, ROPE ? 4 : 8>(x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
+                block_stats<true, true, ROPE && !AHEAD ? 4 : 8>(x, in, rope, NoSkip{}, head, b, op.n_tokens, sm, sm.part[0]);
                 if (threadIdx.x < HEAD_DIM)
                     s += sm.part[0][0][threadIdx.x], lo = fminf(lo, sm.part[0][1][threadIdx.x]), hi = fmaxf(hi, sm.part[0][2][threadIdx.x]);
                 __syncthreads();
@@ -449,6 +481,26 @@ __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(CALL_THREADS, 
     cg::this_cluster().sync();
 }
 
+// Clusters of a kernel that the device takes at once, as the runtime has it (asked once per device): fewer than the SMs would hold of single blocks, since a
+// cluster lies within one group of SMs (48 of eight blocks, three to an SM, where 148 SMs make 55).
+template <auto KERNEL, int CLUSTER>
+int clusters_at_once() {
+    constexpr int MAX_DEVICES = 64;
+    static std::atomic<int> known[MAX_DEVICES];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    int count = device < MAX_DEVICES ? known[device].load(std::memory_order_relaxed) : 0;
+    if (count == 0) {
+        cudaLaunchConfig_t config = {};
+        cudaLaunchAttribute shape = {};
+        shape.id = cudaLaunchAttributeClusterDimension, shape.val.clusterDim.x = CLUSTER, shape.val.clusterDim.y = shape.val.clusterDim.z = 1;
+        config.gridDim = dim3(1024 * CLUSTER), config.blockDim = dim3(CALL_THREADS), config.attrs = &shape, config.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&count, KERNEL, &config) != cudaSuccess) return cudaGetLastError(), 0;
+        if (device < MAX_DEVICES) known[device].store(count, std::memory_order_relaxed);
+    }
+    return count;
+}
+
 int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launches) {
     if (int e = unica_check_device()) return e;
     const CallOperand* operands[] = {&call.q, &call.k, &call.v};
@@ -468,30 +520,45 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
         return UNICA_B200_OK;
     }
     const long long q_tiles = call.q.x ? static_cast<long long>(call.heads) * call.q.tiles : 0, kv_heads = (call.k.x ? call.heads : 0) + (call.v.x ? call.heads : 0);
-    // as in quantize_call_fp4, with four blocks per SM (36 x 1024 53.3 -> 52.3 us a call, 60 x 2048 222 -> 219.7; 32 x 777, rotated, 47.1 -> 49.5 with the
-    // line at four blocks); the tiles of Q fill gaps, and where only they make a second wave (24 x 1000) four blocks per head were 2 us slower
+    int sms = 0;
+    if (int e = unica_sm_count(&sms)) return e;
     const int keys = call.k.n_tokens > call.v.n_tokens ? call.k.n_tokens : call.v.n_tokens;  // (a call may have one of the two alone)
+    const bool rotated = call.rope.table, outliers = call.v_mode == UNICA_B200_V_OUTLIERS;
+    // as in quantize_call_fp4, with four blocks per SM (60 x 2048 222 -> 219.7 us a call; 32 x 777, rotated, 47.1 -> 49.5 with the
+    // line at four blocks); the tiles of Q fill gaps, and where only they make a second wave (24 x 1000) four blocks per head were 2 us slower
     // (Up to 256 keys one block has all statistics and four have a tile each: 16 x 200 19.2 -> 18.4, rotated 22.1 -> 18.8; up to 512 always: 4 x 512 17.0 -> 18.5.)
-    const bool crowded = kv_heads * CALL_CLUSTER > 148 * (call.rope.table ? 3 : 4);
-    const bool four = kv_heads > 0 && call.v_mode != UNICA_B200_V_OUTLIERS && keys <= (!crowded ? 1 : call.rope.table ? 4 : 8) * CALL_BLOCK;
+    const bool crowded = kv_heads * CALL_CLUSTER > sms * (rotated ? 3 : 4);
+    const bool four = kv_heads > 0 && !outliers && keys <= (!crowded ? 1 : rotated ? 4 : 8) * CALL_BLOCK;
     const int cluster = four ? 4 : CALL_CLUSTER;
     if (keys > cluster * CALL_PARTS * CALL_BLOCK) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: more tokens than a cluster's blocks have room for");
     const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
     if (clusters > (1 << 27)) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: too many heads and tiles");
     const dim3 grid(unsigned(clusters) * cluster);
-    auto launch = [&](auto half, auto rope) {
-        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
-        auto kernel = call.v_mode == UNICA_B200_V_OUTLIERS ? quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, HALF, ROPE, CALL_CLUSTER>
-                      : call.v_mode == UNICA_B200_V_TOKEN ? (four ? quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, 4>
-                                                                  : quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, CALL_CLUSTER>)
-                                                          : (four ? quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, 4>
-                                                                  : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, CALL_CLUSTER>);
+    // Loads ahead of a tile, with three blocks per SM, or four blocks per SM without.  Ahead where a block has several tiles and at most one other block
+    // beside it (1 x 8192 per token 123.5 -> 121.3 us a call, 4 x 4128 73.6 -> 71.3; 24 x 1024 44.9 against 46.5).  With outliers, whose V takes longest, what matters is that Q's tiles do
+    // not get in between: three blocks per SM where that has room for K and V but not for Q beside them (20 x 777 42.7 -> 40.3, 16 x 4128 217 -> 212; 8 x 2048 53.1
+    // against 54.0, 28 x 2048 130.6 against 139.8).
+    const int room = outliers ? clusters_at_once<quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, false, false, CALL_CLUSTER, true>, CALL_CLUSTER>() : 0;
+    const bool ahead = !rotated && (outliers ? kv_heads <= room && clusters > room : keys > cluster * KEY_TILE && kv_heads * cluster <= 2 * sms);
+    auto launch = [&](auto half, auto rope, auto ahead) {
+        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value, AHEAD = decltype(ahead)::value;
+        auto kernel = call.v_mode == UNICA_B200_V_OUTLIERS ? quantize_call_int8_kernel<UNICA_B200_V_OUTLIERS, HALF, ROPE, CALL_CLUSTER, AHEAD>
+                      : call.v_mode == UNICA_B200_V_TOKEN ? (four ? quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, 4, AHEAD>
+                                                                  : quantize_call_int8_kernel<UNICA_B200_V_TOKEN, HALF, ROPE, CALL_CLUSTER, AHEAD>)
+                                                          : (four ? quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, 4, AHEAD>
+                                                                  : quantize_call_int8_kernel<UNICA_B200_V_CHANNEL, HALF, ROPE, CALL_CLUSTER, AHEAD>);
         launch_after(kernel, grid, CALL_THREADS, 0, stream, !capturing(stream), call);
     };
     const bool half = first->in.half;
     if (launches) ++*launches;
-    call.rope.table ? (half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))
-                    : (half ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{}));
+    const std::true_type yes{};
+    const std::false_type no{};
+    if (rotated)
+        half ? launch(yes, yes, no) : launch(no, yes, no);
+    else if (ahead)
+        half ? launch(yes, no, yes) : launch(no, no, yes);
+    else
+        half ? launch(yes, no, no) : launch(no, no, no);
     return unica_check_launch("quantize_call_int8");
 }
 
@@ -502,20 +569,33 @@ int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     // (2 x 16 heads x 777 tokens, rotated: 41.7 -> 38 us, 40 x 1024 not rotated 37 -> 30; calls of 20 x 2048 119.2 -> 113.3, 40 x 2048
     // 185 -> 177.3, 16 x 777, rotated, which eight blocks per head do fit, 45.2 against 48.1).  Longer heads are better with eight (20 x 4128,
     // rotated, 296.8 against 304.5; not rotated the same).
+    int sms = 0;
+    if (int e = unica_sm_count(&sms)) return e;
     const int longest = call.q.n_tokens > call.k.n_tokens ? call.q.n_tokens : call.k.n_tokens;
+    const bool rotated = call.rope.table, mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
+    const long long clusters = 3LL * call.heads;
     // And up to 512 tokens in any case (4 x 256 21.8 -> 20.4, 12 x 500 32.5 -> 30.9, rotated 12 x 200 32.7 -> 30.8; 4 x 512 the same).
-    const bool crowded = 3 * call.heads * CALL_CLUSTER > 148 * 3;
-    const bool four = longest <= (!crowded ? 2 : call.rope.table ? 4 : 8) * CALL_BLOCK;
-    auto launch = [&](auto half, auto rope) {
-        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value;
-        const bool mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
-        const int cluster = four && !mixed ? 4 : CALL_CLUSTER;
-        auto kernel = mixed ? quantize_call_fp4_kernel<EACH_ITS_OWN, ROPE, CALL_CLUSTER>
-                      : four ? quantize_call_fp4_kernel<HALF, ROPE, 4> : quantize_call_fp4_kernel<HALF, ROPE, CALL_CLUSTER>;
-        launch_after(kernel, dim3(3u * call.heads * cluster), CALL_THREADS, 0, stream, true, call);
+    const bool crowded = clusters * CALL_CLUSTER > 3 * sms;
+    const bool four = !mixed && longest <= (!crowded ? 2 : rotated ? 4 : 8) * CALL_BLOCK;
+    // Rotated: with eight tokens at a time and V's loads ahead of a tile, which takes two blocks per SM, where that holds all of them at once (1 x 8192 137 -> 130 us a call, 10 x 1024
+    // 47.3 -> 42.8, 23 x 777 52.4 -> 48.2; 12 x 1024 48.1 against 51.4).  Not rotated: V's loads ahead cost no room, and pay
+    // with more than eight tiles to a block (12 x 8192 469.5 -> 465).
+    bool ahead = longest > 8 * KEY_TILE * CALL_CLUSTER;
+    if (rotated && four) {
+        ahead = clusters <= clusters_at_once<quantize_call_fp4_kernel<false, true, 4, true>, 4>();
+    } else if (rotated) {
+        ahead = clusters <= clusters_at_once<quantize_call_fp4_kernel<false, true, CALL_CLUSTER, true>, CALL_CLUSTER>();
+    }
+    auto launch = [&](auto half, auto rope, auto ahead) {
+        constexpr bool HALF = decltype(half)::value, ROPE = decltype(rope)::value, AHEAD = decltype(ahead)::value;
+        auto kernel = mixed ? quantize_call_fp4_kernel<EACH_ITS_OWN, ROPE, CALL_CLUSTER, AHEAD>
+                      : four ? quantize_call_fp4_kernel<HALF, ROPE, 4, AHEAD> : quantize_call_fp4_kernel<HALF, ROPE, CALL_CLUSTER, AHEAD>;
+        launch_after(kernel, dim3(unsigned(clusters) * (four ? 4 : CALL_CLUSTER)), CALL_THREADS, 0, stream, true, call);
     };
-    call.rope.table ? (call.q.in.half ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{}))
-                    : (call.q.in.half ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{}));
+    auto launch_half = [&](auto half, auto rope) { ahead ? launch(half, rope, std::true_type{}) : launch(half, rope, std::false_type{}); };
+    const std::true_type yes{};
+    const std::false_type no{};
+    rotated ? (call.q.in.half ? launch_half(yes, yes) : launch_half(no, yes)) : (call.q.in.half ? launch_half(yes, no) : launch_half(no, no));
     return unica_check_launch("quantize_call_fp4");
 }
 
