@@ -524,11 +524,13 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
     if (int e = unica_sm_count(&sms)) return e;
     const int keys = call.k.n_tokens > call.v.n_tokens ? call.k.n_tokens : call.v.n_tokens;  // (a call may have one of the two alone)
     const bool rotated = call.rope.table, outliers = call.v_mode == UNICA_B200_V_OUTLIERS;
-    // as in quantize_call_fp4, with four blocks per SM (60 x 2048 222 -> 219.7 us a call; 32 x 777, rotated, 47.1 -> 49.5 with the
-    // line at four blocks); the tiles of Q fill gaps, and where only they make a second wave (24 x 1000) four blocks per head were 2 us slower
-    // (Up to 256 keys one block has all statistics and four have a tile each: 16 x 200 19.2 -> 18.4, rotated 22.1 -> 18.8; up to 512 always: 4 x 512 17.0 -> 18.5.)
-    const bool crowded = kv_heads * CALL_CLUSTER > sms * (rotated ? 3 : 4);
-    const bool four = kv_heads > 0 && !outliers && keys <= (!crowded ? 1 : rotated ? 4 : 8) * CALL_BLOCK;
+    // Four blocks per head, as in quantize_call_fp4, where eight would crowd the SMs.  How much they may depends on what a second wave costs and on what the four then
+    // have to do: up to 512 keys 3.7 to an SM (36 x 300 25.7 -> 22.1 us a call; 32 x 300 23.2 against 24.4), up to 1024 3.2 (36 x 777 47.9 -> 42.9, 32 x 600 36.1 -> 33.3;
+    // 28 x 1024 42.9 against 43.9), up to 2048 4 (60 x 2048 222 -> 219.7; 34 x 1500 77.2 against 81.8); rotated, up to 1024, 3 (32 x 777 47.1 against 49.5 with 4).  Up to 256
+    // always, since one block has all statistics then and four have a tile each (16 x 200 19.2 -> 18.4, rotated 22.1 -> 18.8; 4 x 512 17.0 against 18.5).
+    const double per_sm = double(kv_heads * CALL_CLUSTER) / sms;  // blocks for K and V, with eight to a head
+    const double most = rotated ? 3 : keys <= 2 * CALL_BLOCK ? 3.7 : keys <= 4 * CALL_BLOCK ? 3.2 : 4;
+    const bool four = kv_heads > 0 && !outliers && (keys <= CALL_BLOCK || (keys <= (rotated ? 4 : 8) * CALL_BLOCK && per_sm > most));
     const int cluster = four ? 4 : CALL_CLUSTER;
     if (keys > cluster * CALL_PARTS * CALL_BLOCK) return unica_fail(UNICA_B200_ERR_ARGUMENT, "quantize_call: more tokens than a cluster's blocks have room for");
     const long long clusters = kv_heads + (q_tiles + cluster - 1) / cluster;
@@ -564,25 +566,25 @@ int quantize_call_int8(const CallQuantize& call, cudaStream_t stream, int* launc
 
 int quantize_call_fp4(const CallQuantize& call, cudaStream_t stream) {
     if (int e = unica_check_device()) return e;
-    // Four blocks per head where a head's statistics are eight 256-token blocks at most, if eight blocks per head are more than
+    // Four blocks per head where a head's statistics are eight 256-token blocks at most (rotated: four), if eight blocks per head are more than
     // the chip takes at once: some of the eight have little to do in the first step, and a second wave costs its latency again
     // (2 x 16 heads x 777 tokens, rotated: 41.7 -> 38 us, 40 x 1024 not rotated 37 -> 30; calls of 20 x 2048 119.2 -> 113.3, 40 x 2048
-    // 185 -> 177.3, 16 x 777, rotated, which eight blocks per head do fit, 45.2 against 48.1).  Longer heads are better with eight (20 x 4128,
-    // rotated, 296.8 against 304.5; not rotated the same).
-    int sms = 0;
-    if (int e = unica_sm_count(&sms)) return e;
+    // 185 -> 177.3, 18 x 777, rotated, 53.7 -> 44.1; 16 x 777, rotated, which eight blocks per head do fit, 44.3 against 45.0).  Longer heads are better with eight
+    // (20 x 4128, rotated, 296.8 against 304.5; not rotated the same).
     const int longest = call.q.n_tokens > call.k.n_tokens ? call.q.n_tokens : call.k.n_tokens;
     const bool rotated = call.rope.table, mixed = call.k.in.half != call.q.in.half || call.v.in.half != call.q.in.half;
     const long long clusters = 3LL * call.heads;
     // And up to 512 tokens in any case (4 x 256 21.8 -> 20.4, 12 x 500 32.5 -> 30.9, rotated 12 x 200 32.7 -> 30.8; 4 x 512 the same).
-    const bool crowded = clusters * CALL_CLUSTER > 3 * sms;
+    const bool crowded = clusters > clusters_at_once<quantize_call_fp4_kernel<false, true, CALL_CLUSTER, false>, CALL_CLUSTER>();  // (three blocks per SM, rotated or not)
     const bool four = !mixed && longest <= (!crowded ? 2 : rotated ? 4 : 8) * CALL_BLOCK;
     // Rotated: with eight tokens at a time and V's loads ahead of a tile, which takes two blocks per SM, where that holds all of them at once (1 x 8192 137 -> 130 us a call, 10 x 1024
-    // 47.3 -> 42.8, 23 x 777 52.4 -> 48.2; 12 x 1024 48.1 against 51.4).  Not rotated: V's loads ahead cost no room, and pay
+    // 47.3 -> 42.8, 23 x 777 52.4 -> 48.2; 12 x 1024 48.1 against 51.4).  Up to 512 tokens also where it takes two rounds and three blocks per SM would take
+    // more than one and a tenth (40 x 500 54.9 -> 50.5, 47 x 300 47.3 -> 43.1; 36 x 300 41.8 against 42.3, 44 x 1024 94.4 against 99.2).  Not rotated: V's loads ahead cost no room, and pay
     // with more than eight tiles to a block (12 x 8192 469.5 -> 465).
     bool ahead = longest > 8 * KEY_TILE * CALL_CLUSTER;
     if (rotated && four) {
-        ahead = clusters <= clusters_at_once<quantize_call_fp4_kernel<false, true, 4, true>, 4>();
+        const int two = clusters_at_once<quantize_call_fp4_kernel<false, true, 4, true>, 4>(), three = clusters_at_once<quantize_call_fp4_kernel<false, true, 4, false>, 4>();
+        ahead = clusters <= two || (longest <= 2 * CALL_BLOCK && clusters <= 2 * two && 10 * clusters > 11 * three);
     } else if (rotated) {
         ahead = clusters <= clusters_at_once<quantize_call_fp4_kernel<false, true, CALL_CLUSTER, true>, CALL_CLUSTER>();
     }
