@@ -73,9 +73,11 @@ __device__ __forceinline__ void quantize_block16(float2 (&v)[8], const Fp4Outer&
 // mean_of(token): the 128 means that go with the token, or null.
 // codes: the tile's [4 chunks of 32 channels][ROWS][16] bytes; sf: Q [2 halves of 64 channels][32 lanes][4 words]
 // [4] bytes, K [32 lanes][4 words][4] bytes (see the store below).
-template <int ROWS, bool SLOTS, bool BY_ROW>
-__device__ __forceinline__ void rows_fp4_load(RowsRaw<ROWS, FP4_THREADS>& raw, const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile,
-                                              int n_tokens) {
+template <int ROWS, bool SLOTS, bool BY_ROW, typename MeanOf>
+__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
+                                              int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
+                                              const RopeTable& rope) {
+    RowsRaw<ROWS, FP4_THREADS> raw;
     const __nv_bfloat16* first = x + in.offset(head, tile * ROWS);
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
@@ -87,11 +89,6 @@ __device__ __forceinline__ void rows_fp4_load(RowsRaw<ROWS, FP4_THREADS>& raw, c
             raw.piece[it][0] = load_bf16x8(src, in.half), raw.piece[it][1] = load_bf16x8(src + 8, in.half);
         }
     }
-}
-template <int ROWS, bool SLOTS, bool BY_ROW, typename MeanOf>
-__device__ __forceinline__ void rows_fp4_finish(const RowsRaw<ROWS, FP4_THREADS>& raw, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
-                                                int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
-                                                const RopeTable& rope) {
 #pragma unroll
     for (int it = 0; it < ROWS * 8 / FP4_THREADS; ++it) {
         const auto [row, block] = RowsItem<ROWS, FP4_THREADS, BY_ROW>(it);
@@ -127,14 +124,6 @@ __device__ __forceinline__ void rows_fp4_finish(const RowsRaw<ROWS, FP4_THREADS>
         const int word = ROWS == 64 ? (row % 32) * 4 + 2 * (block / 4) + row / 32 : (block / 4) * ROWS + (row % 32) * 4 + row / 32;
         tile_sf[word * 4 + block % 4] = uint8_t(byte);
     }
-}
-template <int ROWS, bool SLOTS, bool BY_ROW, typename MeanOf>
-__device__ __forceinline__ void rows_fp4_tile(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, MeanOf mean_of, const Fp4Outer& outer, int head,
-                                              int tile, int n_tokens, uint8_t* __restrict__ tile_codes, uint8_t* __restrict__ tile_sf,
-                                              const RopeTable& rope) {
-    RowsRaw<ROWS, FP4_THREADS> raw;
-    rows_fp4_load<ROWS, SLOTS, BY_ROW>(raw, x, in, head, tile, n_tokens);
-    rows_fp4_finish<ROWS, SLOTS, BY_ROW>(raw, in, mean_of, outer, head, tile, n_tokens, tile_codes, tile_sf, rope);
 }
 
 // V in NVFP4 along the keys, per channel: one tile of 64 keys (slot order) by a block of FP4_THREADS.  low/high: the channel's

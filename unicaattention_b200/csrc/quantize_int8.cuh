@@ -8,17 +8,6 @@ namespace unica {
 
 constexpr int THREADS = 256;
 
-__device__ __forceinline__ void load8(float (&v)[8], const __nv_bfloat16* src, bool half) {
-    const uint4 raw = load_bf16x8(src, half);
-    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 f = __bfloat1622float2(pairs[i]);
-        v[2 * i] = f.x;
-        v[2 * i + 1] = f.y;
-    }
-}
-
 template <int NT = THREADS>
 __device__ __forceinline__ float block_max(float x, float* scratch) {
 #pragma unroll
@@ -85,7 +74,8 @@ __device__ __forceinline__ void unpack8(const uint4 raw, float2 (&v)[4]) {
 // read), or null.
 //
 // Which row and 16-channel chunk a thread's item is.  BY_ROW: eight threads to a row, so that a warp's load touches 8 lines; the faster way
-// for rotated rows, whose angles are read alike (2 x 16 heads x 777 tokens, NVFP4: 64.9 -> 61.5 us a call; 40 x 32760, INT8: 90 us of 800).
+// for rotated rows, whose angles are read alike (2 x 16 heads x 777 tokens, NVFP4: 64.9 -> 61.5 us a call; 40 x 32760, INT8: 90 us of 800),
+// and for all NVFP4 rows that come from HBM (40 x 32760, Q 163 -> 133 us, K 145 -> 130, rotated 220 -> 161 and 154; 8 x 12000 Q 17.9 -> 15.2).
 // Otherwise a row per lane: 32 lines, but a warp reads the same means and stores 512 contiguous bytes (30 x 4128, INT8: 374.4 against 378).
 template <int ROWS, int NT, bool BY_ROW>
 struct RowsItem {
@@ -218,7 +208,7 @@ __device__ __forceinline__ void rows_int8_tile_once(const __nv_bfloat16* __restr
 
 // rows_int8_tile without a mean and without RoPE (Q): the tile stays in registers as it came, two elements to a register, and
 // its maximum is taken on the bfloat16 pairs (exact), which halves the registers and the instructions up to the scale.
-template <int ROWS, int NT = THREADS, bool BY_ROW = false>
+template <int ROWS, int NT = THREADS>
 __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restrict__ x, const TokenLayout& in, int head, int tile, int n_tokens,
                                                    int8_t* __restrict__ out, float* __restrict__ scale_out, float* scratch,
                                                    const __nv_bfloat16* staged = nullptr) {
@@ -240,7 +230,7 @@ __device__ __forceinline__ void rows_int8_tile_raw(const __nv_bfloat16* __restri
     if (threadIdx.x == 0) *scale_out = scale;
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-        const auto [row, chunk] = RowsItem<ROWS, NT, BY_ROW>(it);
+        const auto [row, chunk] = RowsItem<ROWS, NT, false>(it);
         float2 t[8];
         unpack8(raw.piece[it][0], reinterpret_cast<float2(&)[4]>(t[0]));
         unpack8(raw.piece[it][1], reinterpret_cast<float2(&)[4]>(t[4]));
@@ -266,7 +256,8 @@ struct VTileSmem {
     float key_scale[KEY_TILE], key_inv[KEY_TILE];
 };
 // low, high: this head's [128] (global or shared memory); skip(token): the key is written as zeros; tiles: key tiles per head;
-// v_scale [heads][128] or null (the caller writes it); sm: free again after a __syncthreads().  In two halves, like the rows.
+// v_scale [heads][128] or null (the caller writes it); sm: free again after a __syncthreads().  In two halves, like the rows, so that a caller can
+// have the next tile's loads under way while it works on one.
 struct VRaw {
     uint4 piece[KEY_TILE * 16 / THREADS];
 };
