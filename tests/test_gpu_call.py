@@ -83,7 +83,8 @@ def test_short_operands_alone(tokens, heads):
 @pytest.mark.parametrize("preset", PRESETS)
 @pytest.mark.parametrize("keys", [255, 1024, 1025])
 def test_many_short_heads_equal_the_same_heads_alone(keys, preset, rotated):
-    """Enough heads for the one-launch quantizers to take clusters of four blocks (up to 1024 tokens), against one head at a time."""
+    """Enough heads for the one-launch quantizers to take clusters of four blocks (up to 2048 tokens, rotated 1024), against one head at a time, which
+    takes clusters of eight above 256 keys (NVFP4: 512 tokens); test_gpu_call_lines.py has the lines themselves."""
     import unicaattention_b200 as unica
 
     q, k, v = (x.cuda() for x in qkv(1, 48, keys, keys, seed=keys, channel_scale=True))

@@ -38,3 +38,16 @@ def test_heads_of_one_tile():
         one = [t[b : b + 1, h : h + 1] for t in (q, k, v)]
         assert torch.equal(unica.attention(*one, **unica.PRESETS["fast"]), whole[b : b + 1, h : h + 1])
     unica.check_status()
+
+
+@pytest.mark.parametrize("keys", [1, 64, 65, 190, 256, 300, 513])
+def test_blocks_of_several_one_tile_items(keys):
+    """Four items for most blocks, at key counts around the rings' lengths: from the third on the two query slots are taken again."""
+    import unicaattention_b200 as unica
+
+    q, k, v = (randn_bf16((1, 500, n, 128), i).cuda() for i, n in enumerate((100, keys, keys)))
+    whole = unica.attention(q, k, v, **unica.PRESETS["fast"])
+    for head in (0, 147, 148, 295, 296, 320, 443, 444, 499):  # a block's first, second, third and fourth item
+        one = [t[:, head : head + 1] for t in (q, k, v)]
+        assert torch.equal(unica.attention(*one, **unica.PRESETS["fast"]), whole[:, head : head + 1]), head
+    unica.check_status()
