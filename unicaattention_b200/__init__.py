@@ -480,7 +480,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel: str = D
     Same checks and exceptions as the reference (unica/__init__.py:126-190)."""
     if inputs is None and rope is None and out is None and not peer_out and heads_per_call is _heads_per_call:
         # The usual call, of shapes, strides, types and settings that have been seen before: everything that follows from those is in
-        # its plan (18 -> 10 us of host time a call, as long as the GPU takes for the smallest ones).
+        # its plan (18.9 -> 15.0 us of host time a call, launches included).
         try:
             plan = _PLANS.get(_plan_key(kernel, q, k, v, tile))
         except Exception:  # arguments that have no key: the checks below say what they always have

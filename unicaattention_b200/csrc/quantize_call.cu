@@ -7,8 +7,8 @@
 //   2. they read one another's partial results through distributed shared memory, all in the same order,
 //   3. and quantize an eighth of the head's tiles each; the tokens come out of L2 now.
 // What bounds it: latency.  For few tokens two dependent trips to memory and a cluster barrier each way; at 30 heads x 4128 tokens every
-// block alternates between loads and conversions, with a third of the chip's warps in flight (issue 37 % busy).  So where there are blocks
-// enough, four share an SM in INT8 (64 registers, some 110 bytes of them spilled in bfloat16; the clusters of K and V of that size are then on the GPU together) and
+// block alternates between loads and conversions: with three blocks per SM a third of the chip's warps were in flight and issue 37 % busy, with four it
+// is 47 and 43 %.  So where there are blocks enough, four share an SM in INT8 (64 registers, some 110 bytes of them spilled in bfloat16; the clusters of K and V of that size are then on the GPU together) and
 // three in NVFP4 and rotated (80 registers; rotated rows spill 130 to 180 bytes), with nothing loaded ahead of a tile, which the other blocks make
 // up for: a call of 30 x 4128 per token 376.8 -> 370.3 us, with outliers 381.7 -> 363.0.  Where there are not (AHEAD, see quantize_call_int8 and
 // quantize_call_fp4), a block has more registers, the next tile under way while it works on one, and rotated twice the tokens in flight in the
