@@ -18,7 +18,7 @@ def test_inputs_just_written(preset, shape):
     base = [t.cuda() for t in qkv(*shape, seed=12)]
     given = [t.clone() for t in base]
     factor = torch.linspace(0.5, 2.0, calls, device="cuda").bfloat16()
-    ballast = torch.zeros(64 << 20, device="cuda")  # a kernel long enough for everything behind it to be queued
+    ballast = torch.zeros(64 << 20, device="cuda")  # 0.1 ms: the first calls or so are queued behind it (for all of them see below)
 
     def write(i):
         for x, t in zip(given, base):
